@@ -186,11 +186,42 @@ int device_error_status(gca3d_context *ctx, int word, const char *where);
 
 // colour -> intensity in FP64 then rounded, without contraction, as
 // color3::to_intensity (src/geometry/type.hpp:45-51)
-__device__ __forceinline__ float intensity_of(float r, float g, float b)
+static __device__ __noinline__ float intensity_f64(float r, float g, float b)
 {
     double s = __dadd_rn(__dmul_rn(0.2126, (double)r), __dmul_rn(0.7152, (double)g));
     s = __dadd_rn(s, __dmul_rn(0.0722, (double)b));
     return (float)s;
+}
+
+// the same value from FP32 pairs: an SM issues two FP64 operations per clock, so the nine
+// of intensity_f64 cost a warp 144 cycles of its SM's FP64 pipe and bound every kernel that
+// writes points; this takes about 35 FP32 instructions.  Each product is an exact pair (FMA
+// residual, the weight split in two floats), the sum a pair (hi, lo) within 2^-44 of the
+// magnitudes' sum m of both the real value and the FP64 one.  When hi + lo rounds to hi
+// from either end of an interval of m 2^-43 around it, FP64 rounds there too; otherwise
+// (two in 10^6 random colours), and where a pair could lose bits to the exponent range, the FP64
+// operations decide.
+__device__ __forceinline__ float intensity_of(float r, float g, float b)
+{
+    constexpr float h0 = (float)0.2126, l0 = (float)(0.2126 - (double)h0);
+    constexpr float h1 = (float)0.7152, l1 = (float)(0.7152 - (double)h1);
+    constexpr float h2 = (float)0.0722, l2 = (float)(0.0722 - (double)h2);
+    const float p0 = __fmul_rn(r, h0), p1 = __fmul_rn(g, h1), p2 = __fmul_rn(b, h2);
+    const float e0 = __fmaf_rn(r, l0, __fmaf_rn(r, h0, -p0)), e1 = __fmaf_rn(g, l1, __fmaf_rn(g, h1, -p1)),
+                e2 = __fmaf_rn(b, l2, __fmaf_rn(b, h2, -p2));
+    const float s = __fadd_rn(p0, p1), sb = __fsub_rn(s, p0);
+    const float t = __fadd_rn(__fsub_rn(p0, __fsub_rn(s, sb)), __fsub_rn(p1, sb));
+    const float s2 = __fadd_rn(s, p2), sc = __fsub_rn(s2, s);
+    const float t2 = __fadd_rn(__fsub_rn(s, __fsub_rn(s2, sc)), __fsub_rn(p2, sc));
+    const float low = __fadd_rn(__fadd_rn(t, t2), __fadd_rn(__fadd_rn(e0, e1), e2));
+    const float hi = __fadd_rn(s2, low), lo = __fsub_rn(low, __fsub_rn(hi, s2));
+    const float m = __fadd_rn(__fadd_rn(fabsf(p0), fabsf(p1)), fabsf(p2));
+    const float d = __fmul_rn(m, 1.1368683772161603e-13f); // 2^-43
+    if (m > 1e-15f && m < 1e15f && __fadd_rn(hi, __fadd_rn(lo, d)) == hi && __fadd_rn(hi, __fsub_rn(lo, d)) == hi)
+        return hi;
+    if (r == 0.0f && g == 0.0f && b == 0.0f)
+        return s2; // black, with the sign that FP64 gives
+    return intensity_f64(r, g, b);
 }
 
 // float <-> order-preserving int (for atomicMin/atomicMax on floats)

@@ -53,6 +53,27 @@ def test_upload_download_roundtrip(ctx, golden, orc):
     np.testing.assert_array_equal(d["rgb"], rgb)
 
 
+def test_intensity_equals_fp64(ctx):
+    """the intensity of every point is the FP64 weighted sum rounded to float, bit for bit:
+    random, 8-bit, grey, negative, tiny, huge and non-finite colours"""
+    rng = np.random.default_rng(4)
+    f = np.float32
+    parts = [rng.random((200_000, 3)), rng.integers(0, 256, (50_000, 3)) * f(1 / 255),
+             np.repeat(rng.integers(0, 256, (256, 1)) * f(1 / 255), 3, 1),
+             rng.normal(size=(50_000, 3)) * 10.0 ** rng.integers(-44, 38, (50_000, 1)),
+             np.array(np.meshgrid(*[[0.0, -0.0, 1.0, 1e-45, 3e38, np.inf, -np.inf, np.nan]] * 3)).reshape(3, -1).T]
+    rgb = np.concatenate([p.astype(f) for p in parts])
+    cloud = ctx.cloud_from(np.zeros_like(rgb), rgb)
+    pos = np.empty((len(rgb), 4), f)
+    ctx.check(ctx.L.gca3d_copy(ctx.h, pos.ctypes.data, cloud.device_views()[0], pos.nbytes))
+    with np.errstate(all="ignore"):
+        c = rgb.astype(np.float64)
+        want = ((0.2126 * c[:, 0] + 0.7152 * c[:, 1]) + 0.0722 * c[:, 2]).astype(f)
+    nan = np.isnan(want)
+    np.testing.assert_array_equal(np.isnan(pos[:, 3]), nan)
+    np.testing.assert_array_equal(pos[~nan, 3].view(np.uint32), want[~nan].view(np.uint32))
+
+
 def test_upload_from_pinned_and_device_memory(ctx, N, golden):
     """Pinned host buffers and device buffers are read in place by the packing
     kernel; pageable ones go through a staging copy.  All three give the same cloud
