@@ -512,6 +512,24 @@ def test_frame_tmin_zero_nan_quirk(ctx, N, orc, frames):
     np.testing.assert_array_equal(d["xyz"], ox)
 
 
+@pytest.mark.parametrize("w,h", [(1, 1), (33, 5), (65, 9), (129, 3), (2048, 2)])
+@pytest.mark.parametrize("mode,radius,sd", [(0, 0, 1.0), (1, 0, 1.0), (2, 0, 30.0), (2, 1, 5.0), (2, 3, 99.0),
+                                            (2, 4, 30.0), (2, 5, 300.0), (2, 6, 30.0), (2, 7, 101.0)])
+def test_frame_tiles_and_weight_tables_vs_oracle(ctx, N, orc, w, h, mode, radius, sd):
+    """ragged tiles, every filter radius, and depth sigmas whose weights end inside the
+    range table (5, 30, 99), at its end (101) and beyond it (300)"""
+    rng = np.random.default_rng(w * 1000 + h)
+    depth = (1500 + 40 * rng.normal(size=(h, w)) + 2000 * (rng.random((h, w)) < 0.3)).astype(np.uint16)
+    depth[rng.random((h, w)) < 0.1] = 0
+    depth[rng.random((h, w)) < 0.05] = 65535
+    bgr = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+    d = frame_gpu(ctx, N, depth, bgr, mode, radius=radius, sd=sd)
+    ox, oc = orc.make_point_cloud(depth, bgr, (525.0, 525.0, 319.5, 239.5), mode=mode, radius=radius,
+                                  sigma_space=3.0, sigma_depth=sd, tmin=0.2, tmax=10.0)
+    np.testing.assert_array_equal(d["xyz"], ox)
+    np.testing.assert_array_equal(d["rgb"], oc)
+
+
 # --------------------------------------------------------------------------- #
 # radius outlier removal, gather by index, AoS view
 # --------------------------------------------------------------------------- #
