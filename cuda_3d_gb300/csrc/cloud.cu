@@ -384,7 +384,7 @@ int gca3d_create(int device, void *stream, gca3d_context **out)
         ctx->own_stream = true;
     }
     if (cudaMalloc(&ctx->d_err, 2 * sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&ctx->h_pinned, 64 * sizeof(int)) != cudaSuccess)
+        cudaMallocHost(&ctx->h_pinned, kPinnedBytes) != cudaSuccess)
     {
         gca3d_destroy(ctx);
         return GCA3D_ERR_OUT_OF_MEMORY;

@@ -18,6 +18,8 @@ namespace gca3d
 // ---------------------------------------------------------------------------
 constexpr int kMaxSegments = 4096;       // pairs / clouds in one batched stage
 constexpr int kBlock = 256;              // threads per block for streaming kernels
+constexpr int kPinnedBytes = 96 << 10;   // the context's pinned read-back buffer
+constexpr int kPinnedBulk = 256;         // its part after the single words
 constexpr int kWaitLimitDefault = 1 << 22; // polls before a cross-block wait gives up (about 0.3 s)
 
 // device error word bits
@@ -118,7 +120,7 @@ struct gca3d_context
     // consumed by the host), [1] polls after which a cross-block wait gives up
     // (gca3d_set_wait_limit; kernels read it when they start)
     int *d_err = nullptr;
-    int *h_pinned = nullptr; // pinned scratch for small read-backs (64 ints)
+    int *h_pinned = nullptr; // pinned read-backs: 64 ints, and from kPinnedBulk bytes on larger ones
     int upload_mode = 0;     // GCA3D_UPLOAD_IN_PLACE or GCA3D_UPLOAD_COPY_ENGINE
     int64_t launches = 0;
     std::string last_error;

@@ -28,12 +28,18 @@ __device__ __forceinline__ int isel(bool s, int a, int b)
 // pivot's row / column exchange is a conditional swap (bsel) against each candidate
 // row, so the matrix stays in registers (the solve is one thread's dependent FP64
 // chain on the ICP critical path; in local memory it cost several times more).
-__device__ inline int solve6_device(const double *S /* 21 upper + 6 rhs */, double x[6])
+//
+// Split in two, because a system may be factored before its right-hand side is known.
+// solve6_factor: P A P^T = L D L^T (L in the strict lower triangle of A, the pivots in D);
+// returns 1 when A is singular or not finite (then A, D and perm are not usable if finite
+// is false).  solve6_substitute_warp: x = -A^-1 rhs.
+constexpr double kSolveTiny = 2.2250738585072014e-308;
+__device__ __forceinline__ int solve6_factor(const double *S /* 21 upper */, double A[6][6], double D[6], int perm[6],
+                                             bool &finite)
 {
-    constexpr double kTiny = 2.2250738585072014e-308;
-    double A[6][6], b[6], D[6];
-    int perm[6];
+    constexpr double kTiny = kSolveTiny;
     int status = 0;
+    finite = true;
     {
         int u = 0;
 #pragma unroll
@@ -48,22 +54,14 @@ __device__ inline int solve6_device(const double *S /* 21 upper + 6 rhs */, doub
 #pragma unroll
     for (int i = 0; i < 6; ++i)
     {
-        b[i] = -S[21 + i];
         perm[i] = i;
-        if (!isfinite(b[i]))
-            status = 1;
 #pragma unroll
         for (int j = 0; j < 6; ++j)
             if (!isfinite(A[i][j]))
-                status = 1;
+                finite = false;
     }
-    if (status)
-    {
-#pragma unroll
-        for (int i = 0; i < 6; ++i)
-            x[i] = 0.0;
+    if (!finite)
         return 1;
-    }
 #pragma unroll
     for (int k = 0; k < 6; ++k)
     {
@@ -127,46 +125,52 @@ __device__ inline int solve6_device(const double *S /* 21 upper + 6 rhs */, doub
                 }
         }
     }
-    double y[6], z[6];
+    return status;
+}
+
+// by one warp (all 32 lanes call it; A, D, perm and rhs in memory that all lanes read):
+// lane i holds row i of the forward substitution and of the division by the pivots, since
+// a warp's FP64 instruction costs 64 cycles however many of its lanes are active; every
+// entry is summed in the order of a serial substitution.  Every lane returns x.
+__device__ __forceinline__ void solve6_substitute_warp(const double (*A)[6], const double *D, const int *perm,
+                                                       const double *rhs, double x[6])
+{
+    constexpr double kTiny = kSolveTiny;
+    const unsigned full = 0xffffffffu;
+    const int i = min((int)(threadIdx.x & 31), 5);
+    double y = -rhs[perm[i]];
 #pragma unroll
-    for (int i = 0; i < 6; ++i)
+    for (int j = 0; j < 5; ++j)
     {
-        double s = 0.0;
-#pragma unroll
-        for (int q = 0; q < 6; ++q)
-            s = bsel(perm[i] == q, b[q], s);
-#pragma unroll
-        for (int j = 0; j < i; ++j)
-            s -= A[i][j] * y[j];
-        y[i] = s;
+        const double yj = __shfl_sync(full, y, j);
+        if (i > j)
+            y -= A[i][j] * yj;
     }
+    y = fabs(D[i]) > kTiny ? y / D[i] : 0.0;
+    double z[6];
 #pragma unroll
-    for (int i = 0; i < 6; ++i)
-        y[i] = fabs(D[i]) > kTiny ? y[i] / D[i] : 0.0;
-#pragma unroll
-    for (int i = 5; i >= 0; --i)
+    for (int q = 5; q >= 0; --q)
     {
-        double s = y[i];
+        double s = __shfl_sync(full, y, q);
 #pragma unroll
-        for (int j = i + 1; j < 6; ++j)
-            s -= A[j][i] * z[j];
-        z[i] = s;
+        for (int j = q + 1; j < 6; ++j)
+            s -= A[j][q] * z[j];
+        z[q] = s;
     }
 #pragma unroll
     for (int q = 0; q < 6; ++q)
     {
         double v = 0.0;
 #pragma unroll
-        for (int i = 0; i < 6; ++i)
-            v = bsel(perm[i] == q, z[i], v);
+        for (int k = 0; k < 6; ++k)
+            v = bsel(perm[k] == q, z[k], v);
         x[q] = v;
     }
-    return status;
 }
 
 // ---------------------------------------------------------------------------
-// Warp-parallel restatements of solve6_device and pose_from_x_device for the
-// per-iteration finalize.  FP64 issues at a small fraction of the FP32 rate on
+// Warp-parallel restatements of the solve and of pose_from_x_device, for the per-iteration
+// finalize.  FP64 issues at a small fraction of the FP32 rate on
 // this part, so a single thread's dependent FP64 chain costs tens of
 // microseconds; spread over the lanes of a warp, the chain is the depth of the
 // computation instead of its length.
@@ -241,7 +245,7 @@ __device__ __forceinline__ void exp_coeffs_small(double t2, double &A, double &B
     C = fma(c, -t2, 1.0 / 6.0);
 }
 
-// solve6_device over one warp (same symmetric pivots, factorisation and
+// the solve over one warp (same symmetric pivots, factorisation and
 // substitutions; the backward substitution sums in the opposite order, and the
 // reciprocals of the pivots are rcp_nr's).  Lane
 // tri_lane(i, j) < 21 holds A[i][j] of the lower triangle, lanes 21..26 the
@@ -492,42 +496,44 @@ __device__ inline void pose_from_x_device(const double x[6], int map, double T[1
     T[15] = 1.0;
 }
 
-// dU/dx_m of the pose map as 3x4 row-major blocks (the adjoint of a step).
+// dU/dx_m of the pose map as a 3x4 row-major block (the adjoint of a step), m given per
+// lane; every array index is static, so nothing goes to local memory.
 // Euler ZYX: U = Rz(x2) Ry(x1) Rx(x0), t = x3..5.  SE(3) exponential:
 // R = I + A K + B K^2, t = (I + B K + C K^2) v with K = [w]x, differentiated
 // through A, B, C as functions of theta^2 (series below theta = 1e-2).
-__device__ inline void mat3_mul(const double *A, const double *B, double *C)
+__device__ __forceinline__ void mat3_mul(const double *A, const double *B, double *C)
 {
+#pragma unroll
     for (int i = 0; i < 3; ++i)
+#pragma unroll
         for (int j = 0; j < 3; ++j)
             C[3 * i + j] = A[3 * i] * B[j] + A[3 * i + 1] * B[3 + j] + A[3 * i + 2] * B[6 + j];
 }
 
-__device__ inline void pose_jacobian_device(const double x[6], int map, double dU[6][12])
+__device__ inline void pose_derivative_device(const double x[6], int map, int m, double d[12])
 {
-    for (int m = 0; m < 6; ++m)
-        for (int k = 0; k < 12; ++k)
-            dU[m][k] = 0.0;
     if (map == GCA3D_UPDATE_EULER_ZYX)
     {
         double sa, ca, sb, cb, sc, cc;
         sincos(x[0], &sa, &ca);
         sincos(x[1], &sb, &cb);
         sincos(x[2], &sc, &cc);
-        const double Rx[9] = {1, 0, 0, 0, ca, -sa, 0, sa, ca}, dRx[9] = {0, 0, 0, 0, -sa, -ca, 0, ca, -sa};
-        const double Ry[9] = {cb, 0, sb, 0, 1, 0, -sb, 0, cb}, dRy[9] = {-sb, 0, cb, 0, 0, 0, -cb, 0, -sb};
-        const double Rz[9] = {cc, -sc, 0, sc, cc, 0, 0, 0, 1}, dRz[9] = {-sc, -cc, 0, cc, -sc, 0, 0, 0, 0};
-        for (int m = 0; m < 3; ++m)
-        {
-            double M1[9], M2[9];
-            mat3_mul(m == 2 ? dRz : Rz, m == 1 ? dRy : Ry, M1);
-            mat3_mul(M1, m == 0 ? dRx : Rx, M2);
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j)
-                    dU[m][4 * i + j] = M2[3 * i + j];
-        }
+        // the factor of axis m replaced by its derivative (c, s -> -s, c; the unit entry -> 0)
+        const bool d0 = m == 0, d1 = m == 1, d2 = m == 2;
+        const double Rx[9] = {d0 ? 0.0 : 1.0, 0, 0, 0, d0 ? -sa : ca, d0 ? -ca : -sa, 0, d0 ? ca : sa, d0 ? -sa : ca};
+        const double Ry[9] = {d1 ? -sb : cb, 0, d1 ? cb : sb, 0, d1 ? 0.0 : 1.0, 0, d1 ? -cb : -sb, 0, d1 ? -sb : cb};
+        const double Rz[9] = {d2 ? -sc : cc, d2 ? -cc : -sc, 0, d2 ? cc : sc, d2 ? -sc : cc, 0, 0, 0, d2 ? 0.0 : 1.0};
+        double M1[9], M2[9];
+        mat3_mul(Rz, Ry, M1);
+        mat3_mul(M1, Rx, M2);
+#pragma unroll
         for (int i = 0; i < 3; ++i)
-            dU[3 + i][4 * i + 3] = 1.0;
+        {
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                d[4 * i + j] = m < 3 ? M2[3 * i + j] : 0.0;
+            d[4 * i + 3] = m == 3 + i ? 1.0 : 0.0;
+        }
         return;
     }
     const double w[3] = {x[0], x[1], x[2]}, v[3] = {x[3], x[4], x[5]};
@@ -557,31 +563,29 @@ __device__ inline void pose_jacobian_device(const double x[6], int map, double d
     const double K[9] = {0, -w[2], w[1], w[2], 0, -w[0], -w[1], w[0], 0};
     double K2[9];
     mat3_mul(K, K, K2);
-    for (int m = 0; m < 3; ++m)
+    const int a = m % 3;
+    const double wa = a == 0 ? w[0] : (a == 1 ? w[1] : w[2]);
+    const double g0 = a == 0 ? 1.0 : 0.0, g1 = a == 1 ? 1.0 : 0.0, g2 = a == 2 ? 1.0 : 0.0;
+    const double G[9] = {0, -g2, g1, g2, 0, -g0, -g1, g0, 0}; // [e_a]x
+    double GK[9], KG[9], dV[9];
+    mat3_mul(G, K, GK);
+    mat3_mul(K, G, KG);
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
     {
-        double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}; // [e_m]x
-        if (m == 0)
-            G[5] = -1, G[7] = 1;
-        else if (m == 1)
-            G[2] = 1, G[6] = -1;
-        else
-            G[1] = -1, G[3] = 1;
-        double GK[9], KG[9];
-        mat3_mul(G, K, GK);
-        mat3_mul(K, G, KG);
-        double dV[9];
-        for (int k = 0; k < 9; ++k)
-        {
-            const double sym = GK[k] + KG[k];
-            dU[m][4 * (k / 3) + k % 3] = 2.0 * w[m] * Ad * K[k] + A * G[k] + 2.0 * w[m] * Bd * K2[k] + B * sym;
-            dV[k] = 2.0 * w[m] * Bd * K[k] + B * G[k] + 2.0 * w[m] * Cd * K2[k] + C * sym;
-        }
-        for (int i = 0; i < 3; ++i)
-            dU[m][4 * i + 3] = dV[3 * i] * v[0] + dV[3 * i + 1] * v[1] + dV[3 * i + 2] * v[2];
+        const double sym = GK[k] + KG[k];
+        const double r = 2.0 * wa * Ad * K[k] + A * G[k] + 2.0 * wa * Bd * K2[k] + B * sym;
+        d[4 * (k / 3) + k % 3] = m < 3 ? r : 0.0;
+        dV[k] = 2.0 * wa * Bd * K[k] + B * G[k] + 2.0 * wa * Cd * K2[k] + C * sym;
     }
-    for (int m = 0; m < 3; ++m)
-        for (int i = 0; i < 3; ++i)
-            dU[3 + m][4 * i + 3] = (i == m ? 1.0 : 0.0) + B * K[3 * i + m] + C * K2[3 * i + m];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+    {
+        const double t = dV[3 * i] * v[0] + dV[3 * i + 1] * v[1] + dV[3 * i + 2] * v[2];
+        const double Ka = a == 0 ? K[3 * i] : (a == 1 ? K[3 * i + 1] : K[3 * i + 2]);
+        const double K2a = a == 0 ? K2[3 * i] : (a == 1 ? K2[3 * i + 1] : K2[3 * i + 2]);
+        d[4 * i + 3] = m < 3 ? t : (i == a ? 1.0 : 0.0) + B * Ka + C * K2a;
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -113,6 +113,27 @@ def test_vjp_matches_fp64_adjoint(ctx, N, orc, c2, K, umap):
         assert np.abs(r["dxi0"]).max() <= 1e-3 * np.abs(G).max()
 
 
+@pytest.mark.parametrize("n", [255, 64 * 256, 64 * 256 + 1])
+@pytest.mark.parametrize("K,umap", [(1, 1), (3, 0)])
+def test_vjp_block_counts_vs_fp64(ctx, N, orc, c2, n, K, umap):
+    """one point block, a whole tile of block partials (64) and one more: points and
+    colours against the FP64 adjoint, rows without a correspondence exactly zero"""
+    pr = c2["pr"]
+    src = ctx.cloud_from(pr.src_xyz[:n], pr.src_rgb[:n])
+    G, gE = _loss_seed(n + K)
+    r = N.color_icp_vjp(ctx, src, c2["tgt"], c2["xi0"], K=K, max_corr=MAX_CORR, update_map=umap, dT=G, dE=gE,
+                        want_corr=True)
+    assert r["status"] == N.OK
+    a = _oracle_args(c2)
+    a = (a[0][:n], a[1][:n]) + a[2:]
+    _, dX, dC, st = orc.icp_unrolled_vjp_f64(*a, c2["xi0"], r["corr"], G, gE, K=K, max_corr=MAX_CORR, update_map=umap)
+    assert st == 0
+    for g, ref in ((r["dxyz"], dX), (r["drgb"], dC)):
+        assert np.linalg.norm(g - ref) <= GRAD_RTOL * np.linalg.norm(ref)
+    none = (r["corr"] < 0).all(0)
+    assert none.any() and not r["dxyz"][none].any() and not r["drgb"][none].any()
+
+
 @pytest.mark.parametrize("K,rtol", [(2, 2e-3), (3, 1e-2)])
 def test_vjp_pose_gradient_far_from_convergence(ctx, N, orc, c2, K, rtol):
     """The pose block of the gradient where it is not negligible.  With the
