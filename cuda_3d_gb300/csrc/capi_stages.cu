@@ -10,11 +10,6 @@ using namespace gca3d;
 namespace
 {
 
-__global__ void k_set_count(const int32_t *src, int32_t *dst)
-{
-    *dst = *src;
-}
-
 int upload_segsrc(gca3d_context *ctx, gca3d_cloud *const *clouds, int P, SegSrc **out)
 {
     std::vector<SegSrc> h(P);
@@ -35,7 +30,7 @@ int upload_segsrc(gca3d_context *ctx, gca3d_cloud *const *clouds, int P, SegSrc 
 namespace gca3d
 {
 // a single-segment batch view of a cloud (no copy)
-int cloud_batch(gca3d_context *ctx, gca3d_cloud *c, Batch &b)
+int cloud_batch(gca3d_context *ctx, gca3d_cloud *c, Batch &b, bool by_grid)
 {
     b.pos = c->pos;
     b.col = c->col;
@@ -47,6 +42,11 @@ int cloud_batch(gca3d_context *ctx, gca3d_cloud *c, Batch &b)
     b.seg_off = ctx->arena.get<int32_t>(2);
     if (!b.seg_off)
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "cloud_batch: scratch");
+    if (by_grid)
+    {
+        b.d_count = c->d_count;
+        return GCA3D_OK;
+    }
     return single_seg_offsets(ctx, c->d_count, b.seg_off);
 }
 
@@ -67,10 +67,8 @@ int gca3d_voxel_downsample(gca3d_context *ctx, gca3d_cloud *in, float voxel, gca
     if (out->capacity < in->capacity)
         return fail(ctx, GCA3D_ERR_CAPACITY, "voxel_downsample: output capacity below input capacity");
     ctx->arena.reset();
-    SegSrc *d_src = nullptr;
-    int st = upload_segsrc(ctx, &in, 1, &d_src);
-    if (st)
-        return st;
+    SegSrc *d_src = ctx->arena.get<SegSrc>(1);
+    const SegSrc one{in->pos, in->col, nullptr, in->d_count};
     Batch b;
     b.pos = out->pos;
     b.col = out->col;
@@ -78,13 +76,12 @@ int gca3d_voxel_downsample(gca3d_context *ctx, gca3d_cloud *in, float voxel, gca
     b.cap = in->capacity;
     b.max_seg_cap = in->capacity;
     b.seg_off = ctx->arena.get<int32_t>(2);
-    if (!b.seg_off)
+    if (!b.seg_off || !d_src)
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "voxel_downsample: scratch");
-    st = voxel_stage(ctx, d_src, 1, in->capacity, in->capacity, voxel, b);
+    const int st = voxel_stage(ctx, d_src, 1, in->capacity, in->capacity, voxel, b, false, nullptr, nullptr, &one,
+                               out->d_count);
     if (st)
         return st;
-    k_set_count<<<1, 1, 0, ctx->stream>>>(b.seg_off + 1, out->d_count);
-    GCA_CHECK_LAUNCH(ctx);
     out->has_normals = out->has_grad = false;
     return consume_device_error(ctx, "voxel_downsample");
 }
@@ -98,7 +95,7 @@ int gca3d_estimate_normals(gca3d_context *ctx, gca3d_cloud *c, float radius, int
         return st;
     ctx->arena.reset();
     Batch b;
-    if ((st = cloud_batch(ctx, c, b)))
+    if ((st = cloud_batch(ctx, c, b, true)))
         return st;
     Grid g;
     if ((st = grid_build(ctx, b, radius, kOriginPadF64, nullptr, g)))
@@ -121,7 +118,7 @@ int gca3d_color_gradient(gca3d_context *ctx, gca3d_cloud *c, float radius)
         return st;
     ctx->arena.reset();
     Batch b;
-    if ((st = cloud_batch(ctx, c, b)))
+    if ((st = cloud_batch(ctx, c, b, true)))
         return st;
     Grid g;
     if ((st = grid_build(ctx, b, radius, kOriginPadF32, nullptr, g)))
@@ -139,7 +136,7 @@ int gca3d_nn_search(gca3d_context *ctx, gca3d_cloud *query, gca3d_cloud *ref, fl
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "nn_search: bad arguments");
     ctx->arena.reset();
     Batch b;
-    int st = cloud_batch(ctx, ref, b);
+    int st = cloud_batch(ctx, ref, b, true);
     if (st)
         return st;
     Grid g;
@@ -158,7 +155,7 @@ int gca3d_radius_search(gca3d_context *ctx, gca3d_cloud *query, gca3d_cloud *ref
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "radius_search: bad arguments");
     ctx->arena.reset();
     Batch b;
-    int st = cloud_batch(ctx, ref, b);
+    int st = cloud_batch(ctx, ref, b, true);
     if (st)
         return st;
     Grid g;

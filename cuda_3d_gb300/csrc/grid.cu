@@ -12,6 +12,7 @@
 // then ascending original index) are the reference's, so radius lists come out in
 // the reference's order for the same grid origin.  Memory is O(points), not
 // O(bounding-box volume).
+#include "cluster_sort.cuh"
 #include "grid_query.cuh"
 #include "stages.cuh"
 
@@ -20,85 +21,98 @@
 namespace gca3d
 {
 
-__global__ void k_grid_layout(const int *ord, int P, float cell, int mode, float3 given, float3 *origin,
-                              KeyLayout *lay, int *d_err)
+__device__ __forceinline__ float3 grid_origin(const float mn[3], float cell, int mode, float3 given)
 {
-    __shared__ uint32_t s_max[3];
-    if (threadIdx.x < 3)
-        s_max[threadIdx.x] = 1;
-    __syncthreads();
-    for (int s = threadIdx.x; s < P; s += blockDim.x)
-    {
-        float mn[3], mx[3], o[3];
-        for (int a = 0; a < 3; ++a)
-        {
-            mn[a] = ordered_to_float(ord[6 * s + a]);
-            mx[a] = ordered_to_float(ord[6 * s + 3 + a]);
-        }
-        const float g[3] = {given.x, given.y, given.z};
-        for (int a = 0; a < 3; ++a)
-        {
-            if (mode == kOriginGiven)
-                o[a] = g[a];
-            else if (mode == kOriginPadF64)
-                o[a] = (float)__dsub_rn((double)mn[a], __dmul_rn(1.5, (double)cell));
-            else
-                o[a] = __fsub_rn(mn[a], __fmul_rn(1.5f, cell));
-        }
-        origin[s] = make_float3(o[0], o[1], o[2]);
-        if (!(mx[0] >= mn[0]))
-            continue; // empty segment
-        for (int a = 0; a < 3; ++a)
-        {
-            int lo = cell_of(mn[a], o[a], cell);
-            int hi = cell_of(mx[a], o[a], cell);
-            if (lo < 0 || hi >= (1 << 21))
-            {
-                atomicOr(d_err, kErrKeyBits);
-                hi = (1 << 21) - 1;
-            }
-            atomicMax(&s_max[a], (uint32_t)max(hi, 1));
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        KeyLayout L;
-        L.bseg = bitlen_u32((uint32_t)(P - 1));
-        L.bx = bitlen_u32(s_max[0]);
-        L.by = bitlen_u32(s_max[1]);
-        L.bz = bitlen_u32(s_max[2]);
-        L.total_bits = L.bseg + L.bx + L.by + L.bz;
-        L.morton = 0;
-        if (L.total_bits > 64)
-            atomicOr(d_err, kErrKeyBits);
-        *lay = L;
-    }
+    float o[3];
+    const float g[3] = {given.x, given.y, given.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        o[a] = mode == kOriginGiven
+                   ? g[a]
+                   : (mode == kOriginPadF64 ? (float)__dsub_rn((double)mn[a], __dmul_rn(1.5, (double)cell))
+                                            : __fsub_rn(mn[a], __fmul_rn(1.5f, cell)));
+    return make_float3(o[0], o[1], o[2]);
 }
 
-__global__ void k_grid_keys(const float4 *__restrict__ pos, const int32_t *seg_off, const float3 *origin,
-                            const KeyLayout *lay, float cell, uint64_t *keys, int32_t *vals, int ib_cap, int *d_ib,
-                            int *d_kshift)
+// the largest cell per axis of a set with bounds mn, mx (untouched when the set is empty);
+// error bits
+__device__ __forceinline__ int grid_extent(const float mn[3], const float mx[3], float3 origin, float cell,
+                                           uint32_t cells[3])
 {
-    const int seg = blockIdx.y;
-    const int b = seg_off[seg], e = seg_off[seg + 1];
-    const KeyLayout L = *lay;
-    const int ib = packed_index_bits(L.total_bits, ib_cap);
-    if (seg == 0 && blockIdx.x == 0 && threadIdx.x == 0)
-        *d_ib = *d_kshift = ib;
-    const float3 o = origin[seg];
-    const uint64_t mask_x = (1ull << L.bx) - 1, mask_y = (1ull << L.by) - 1, mask_z = (1ull << L.bz) - 1;
-    for (int i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x)
+    if (!(mx[0] >= mn[0]))
+        return 0; // empty
+    int err = 0;
+    const float o[3] = {origin.x, origin.y, origin.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
     {
-        float4 p = pos[i];
-        // clamp defends the key fields against points outside the declared origin
-        uint64_t cx = (uint64_t)max(cell_of(p.x, o.x, cell), 0) & mask_x;
-        uint64_t cy = (uint64_t)max(cell_of(p.y, o.y, cell), 0) & mask_y;
-        uint64_t cz = (uint64_t)max(cell_of(p.z, o.z, cell), 0) & mask_z;
-        sort_store(keys, vals, i, ((uint64_t)seg << (L.bx + L.by + L.bz)) | (cx << (L.by + L.bz)) | (cy << L.bz) | cz,
-                   ib);
+        const int lo = cell_of(mn[a], o[a], cell);
+        int hi = cell_of(mx[a], o[a], cell);
+        if (lo < 0 || hi >= (1 << 21))
+        {
+            err = kErrKeyBits;
+            hi = (1 << 21) - 1;
+        }
+        cells[a] = (uint32_t)max(hi, 0);
     }
+    return err;
 }
+
+__device__ __forceinline__ uint64_t grid_key(float4 p, int seg, const KeyLayout &L, float3 o, float cell, float inv)
+{
+    // clamp defends the key fields against points outside the declared origin
+    const uint64_t cx = (uint64_t)max(cell_of_inv(p.x, o.x, cell, inv), 0) & ((1ull << L.bx) - 1);
+    const uint64_t cy = (uint64_t)max(cell_of_inv(p.y, o.y, cell, inv), 0) & ((1ull << L.by) - 1);
+    const uint64_t cz = (uint64_t)max(cell_of_inv(p.z, o.z, cell, inv), 0) & ((1ull << L.bz) - 1);
+    return ((uint64_t)seg << (L.bx + L.by + L.bz)) | (cx << (L.by + L.bz)) | (cy << L.bz) | cz;
+}
+
+// the grid keys of P sets; one set may come with its count alone (its offsets are then
+// written by begin)
+struct GridMaker
+{
+    const float4 *pos;
+    int32_t *seg_off;
+    const int32_t *d_count; // or null
+    float cell, inv;
+    int mode;
+    float3 given;
+    __device__ int2 range(int seg) const
+    {
+        return d_count ? make_int2(0, *d_count) : make_int2(seg_off[seg], seg_off[seg + 1]);
+    }
+    __device__ float4 point(int, int i) const { return __ldg(&pos[i]); }
+    __device__ int sub_bits() const { return 0; }
+    __device__ void begin(int n) const
+    {
+        if (d_count)
+        {
+            seg_off[0] = 0;
+            seg_off[1] = n;
+        }
+    }
+    __device__ int segment(const float mn[3], const float mx[3], float3 &o, uint32_t cells[3]) const
+    {
+        o = grid_origin(mn, cell, mode, given);
+        return grid_extent(mn, mx, o, cell, cells);
+    }
+    __device__ int layout(const uint32_t cells[3], int P, KeyLayout &L) const
+    {
+        L.bseg = bitlen_u32((uint32_t)(P - 1));
+        L.bx = bitlen_u32(max(cells[0], 1u));
+        L.by = bitlen_u32(max(cells[1], 1u));
+        L.bz = bitlen_u32(max(cells[2], 1u));
+        L.total_bits = L.bseg + L.bx + L.by + L.bz;
+        L.morton = 0;
+        return L.total_bits > 64 ? kErrKeyBits : 0;
+    }
+    __device__ uint64_t key(float4 p, int seg, const KeyLayout &L, float3 o, int *) const
+    {
+        return grid_key(p, seg, L, o, cell, inv);
+    }
+};
+
+bool grid_cluster_enable() { return cluster_sort_enable<GridMaker>(); }
 
 __global__ void k_grid_scatter(SortBuffers sb, const int32_t *d_n, const KeyLayout *lay, const float4 *__restrict__ pos,
                                float4 *spos, int32_t *sidx, float *sint, int *scz, uint64_t *skey, int *err)
@@ -201,7 +215,6 @@ int grid_build(gca3d_context *ctx, const Batch &b, float cell, int origin_mode, 
     d.seg_off = b.seg_off;
     d.d_n = b.seg_off + P;
     d.err = ctx->d_err;
-    int *ord = A.get<int>(6 * P);
     SortBuffers sb;
     sb.keys[0] = A.get<uint64_t>(cap);
     sb.keys[1] = A.get<uint64_t>(cap);
@@ -210,22 +223,20 @@ int grid_build(gca3d_context *ctx, const Batch &b, float cell, int origin_mode, 
     sb.d_sel = A.get<int>(1);
     sb.d_ib = A.get<int>(1);
     sb.d_kshift = A.get<int>(1);
-    if (!d.gmin || !d.layout || !d.spos || !d.sidx || !d.sint || !d.scz || !d.skey || !d.slots || !ord || !sb.keys[1] ||
+    if (!d.gmin || !d.layout || !d.spos || !d.sidx || !d.sint || !d.scz || !d.skey || !d.slots || !sb.keys[1] ||
         !sb.vals[1] || !sb.d_sel || !sb.d_ib || !sb.d_kshift)
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "grid_build: scratch");
     cudaStream_t s = ctx->stream;
-    int st = seg_bounds(ctx, b.pos, b.seg_off, P, b.max_seg_cap, ord);
-    if (st)
-        return st;
-    float3 given = host_origin ? make_float3(host_origin[0], host_origin[1], host_origin[2]) : make_float3(0, 0, 0);
-    k_grid_layout<<<1, 256, 0, s>>>(ord, P, cell, origin_mode, given, d.gmin, d.layout, ctx->d_err);
-    GCA_CHECK_LAUNCH(ctx);
-    const int gx = std::min(grid_for(b.max_seg_cap, kBlock * 4), ctx->num_sms * 4);
-    k_grid_keys<<<dim3(gx, P), kBlock, 0, s>>>(b.pos, b.seg_off, d.gmin, d.layout, cell, sb.keys[0], sb.vals[0],
-                                               index_bits(cap), sb.d_ib, sb.d_kshift);
-    GCA_CHECK_LAUNCH(ctx);
+    const float3 given = host_origin ? make_float3(host_origin[0], host_origin[1], host_origin[2]) : make_float3(0, 0, 0);
     const int32_t *d_n = b.seg_off + P;
-    st = radix_sort(ctx, sb, b.seg_off, P, cap, b.max_seg_cap, 64);
+    const GridMaker mk{b.pos, b.seg_off, b.d_count, cell, 1.0f / cell, origin_mode, given};
+    int st;
+    if (cluster_sortable(ctx, P, cap))
+        st = cluster_sort(ctx, mk, cap,
+                          ClusterOut{sb.keys[0], sb.vals[0], sb.d_sel, sb.d_ib, sb.d_kshift, d.layout, d.gmin,
+                                     ctx->d_err, nullptr, nullptr, nullptr, nullptr});
+    else
+        st = sort_by_keys(ctx, mk, sb, b.seg_off, P, cap, b.max_seg_cap, d.layout, d.gmin, 0, nullptr);
     if (st)
         return st;
     const int gs = std::min(grid_for(cap), ctx->num_sms * 8);

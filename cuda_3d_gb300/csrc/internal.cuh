@@ -115,6 +115,7 @@ struct gca3d_context
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int num_sms = 0;
+    bool cluster_sort = false; // the device runs the one-launch sort (cluster_sort.cuh)
     gca3d::Arena arena;
     // device control words: [0] error bits (kErr*, set with atomicOr by kernels and
     // consumed by the host), [1] polls after which a cross-block wait gives up
@@ -252,6 +253,20 @@ __device__ __forceinline__ float dist2_ref(float qx, float qy, float qz, float p
 __device__ __forceinline__ int cell_of(float p, float mn, float cell)
 {
     return __float2int_rd(__fdiv_rn(__fsub_rn(p, mn), cell));
+}
+
+// cell_of with inv = 1 / cell (rounded): the product is within three rounding units of
+// (p - mn) / cell and the quotient within one, so where the product is further than that
+// from an integer the two have the same floor; only the others are divided (a division is
+// three times the instructions, and a key has three)
+__device__ __forceinline__ int cell_of_inv(float p, float mn, float cell, float inv)
+{
+    const float d = __fsub_rn(p, mn);
+    const float q = __fmul_rn(d, inv), f = floorf(q);
+    const float r = __fsub_rn(q, f), slack = __fmul_rn(fabsf(q), 4.0e-7f);
+    if (r > slack && __fsub_rn(1.0f, r) > slack && fabsf(q) < 4.0e6f && fabsf(q) > 1.0e-30f)
+        return (int)f;
+    return __float2int_rd(__fdiv_rn(d, cell));
 }
 
 __device__ __forceinline__ int bitlen_u32(uint32_t v) { return v ? 32 - __clz(v) : 0; }
@@ -461,20 +476,17 @@ __device__ __forceinline__ SortedView sorted_view(const SortBuffers &sb)
     return SortedView{sb.keys[sel], sb.vals[sel], *sb.d_ib, *sb.d_kshift};
 }
 
-// stable LSD sort of the keys in sb.keys[0] (and sb.vals[0]) in place, segment by
-// segment: seg_off[P + 1] (device) holds the segments' element ranges, at most cap
-// elements in all and max_seg_cap in one segment; the segment index must be the keys'
-// most significant field
-int radix_sort(gca3d_context *ctx, SortBuffers &sb, const int32_t *seg_off, int P, int64_t cap, int64_t max_seg_cap,
-               int max_bits);
-
 // exclusive scan of int32 values (n on the device), writes total to *d_total
 int exclusive_scan(gca3d_context *ctx, const int32_t *in, int32_t *out, const int32_t *d_n,
                    int64_t cap, int32_t *d_total);
 // the runs of equal keys of a sorted view in one scan: starts[r] the first position of
 // run r, starts[runs] = n, *d_runs the number of runs, seg_first[s] the first run of
-// segment s (left untouched, e.g. -1, for an empty segment)
+// segment s (left untouched, e.g. -1, for an empty segment; may be null).  For one segment
+// seg_off receives {0, runs} and *d_count the number of runs (either may be null).
+// zeroed: run_scan_zero_bytes(cap) of memory that the caller has cleared, or null.
+size_t run_scan_zero_bytes(int64_t cap);
 int run_scan(gca3d_context *ctx, const SortBuffers &sb, const int32_t *d_n, int64_t cap, const KeyLayout *lay,
-             int32_t *starts, int32_t *seg_first, int32_t *d_runs);
+             int32_t *starts, int32_t *seg_first, int32_t *d_runs, int32_t *seg_off = nullptr,
+             int32_t *d_count = nullptr, void *zeroed = nullptr);
 
 } // namespace gca3d

@@ -168,7 +168,7 @@ int gca3d_radius_outlier_removal(gca3d_context *ctx, gca3d_cloud *in, float radi
         return fail(ctx, GCA3D_ERR_CAPACITY, "radius_outlier_removal: output capacity below the input's");
     ctx->arena.reset();
     Batch b;
-    int st = cloud_batch(ctx, in, b);
+    int st = cloud_batch(ctx, in, b, true);
     if (st)
         return st;
     Grid g;

@@ -121,6 +121,7 @@ SubLevels finer_scales(const gca3d_icp_params &p, int si)
         const float w = p.scales[k].voxel;
         if (!(w > 0.0f) || w * 2.0f != v)
             break;
+        sub.inv[sub.n] = 1.0f / w;
         sub.voxel[sub.n++] = w;
         v = w;
     }

@@ -11,47 +11,17 @@
 // error word and treats the missing state as the end of its look-back -- the partial
 // prefix only lowers the offsets it writes, which stay inside the output -- so a
 // scheduling fault shows up as a status, never as a hung GPU.
-#include "internal.cuh"
+#include "sort_keys.cuh"
+
+#include <algorithm>
 
 namespace gca3d
 {
-
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 12;
-constexpr int kSortTile = kSortThreads * kSortItems; // 3072 keys per tile
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kLookWindow = 8; // predecessor tiles read at once in the look-back
 
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagInc = 2u << 30;
 constexpr uint32_t kFlagMask = 3u << 30;
 constexpr uint32_t kCountMask = (1u << 30) - 1;
-
-// Control words of one sort.  The keys come in P segments ([seg_off[s], seg_off[s+1]),
-// the segment index being the key's most significant field, each segment's keys in
-// ascending index order), so a segment's keys end up in its own range: the sort runs
-// per segment -- digit offsets per segment, tiles that never straddle two segments,
-// and a look-back that ends at the segment's first tile, so the look-back chains are
-// as long as a segment, not as the batch.  A pass is skipped when every segment's
-// keys share its digit (the segment field's digits always do).
-struct SortCtl
-{
-    int nontrivial[8];
-    int in_sel[8];
-    uint32_t tile_ctr[8];
-    uint32_t prep_ticket;
-    int ntiles; // tiles over all segments
-};
-
-// per-segment scratch of a sort: hist[s][d][b] digit counts, doff[s][d][b] the first
-// output position of bucket b of digit d in segment s, tile_first[s] the segment's
-// first tile (P + 1 entries)
-struct SortSeg
-{
-    uint32_t *hist;
-    uint32_t *doff;
-    int32_t *tile_first;
-};
 
 // a status word carries its flag and count together in one aligned 32-bit word, and
 // nothing else is read on the strength of it, so publishing needs no release fence
@@ -76,163 +46,6 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
-}
-
-// the byte-digit d of a sort word: bits [ks + 8 d, ks + 8 d + 8), ks the key's lowest bit
-// (SortBuffers::d_kshift), zero above bit 63
-__device__ __forceinline__ uint32_t sort_digit(uint64_t k, int ks, int d)
-{
-    const int sh = ks + 8 * d;
-    return sh < 64 ? (uint32_t)(k >> sh) & 255u : 0u;
-}
-
-// per-segment histograms of all 8 byte-digits (block (x, s): segment s); also clears
-// the first look-back status buffer
-__global__ void k_sort_hist(const uint64_t *__restrict__ keys, const int32_t *seg_off, const int *d_kshift, SortSeg S,
-                            uint32_t *status0, int64_t status_words)
-{
-    __shared__ uint32_t h[8][256];
-    for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x)
-        (&h[0][0])[i] = 0;
-    __syncthreads();
-    const int seg = blockIdx.y;
-    const int b = seg_off[seg], e = seg_off[seg + 1];
-    const int ks = *d_kshift;
-    for (int i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x)
-    {
-        uint64_t k = keys[i];
-#pragma unroll
-        for (int d = 0; d < 8; ++d)
-            atomicAdd(&h[d][sort_digit(k, ks, d)], 1u);
-    }
-    const int64_t nb = (int64_t)gridDim.x * gridDim.y, bid = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
-    for (int64_t i = bid * blockDim.x + threadIdx.x; i < status_words; i += nb * blockDim.x)
-        status0[i] = 0;
-    __syncthreads();
-    uint32_t *gh = S.hist + (size_t)seg * 8 * 256;
-    for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x)
-    {
-        uint32_t c = (&h[0][0])[i];
-        if (c)
-            atomicAdd(&gh[i], c);
-    }
-}
-
-// per segment (block s): bucket offsets of every digit, whether the segment's digit
-// varies, and its tile count; the last block: the segments' first tiles and the
-// ping-pong bookkeeping.  One warp per digit, each lane scanning 8 consecutive buckets.
-__global__ void k_sort_prep(SortCtl *ctl, SortSeg S, const int32_t *seg_off, int P, int npasses, int *d_sel)
-{
-    const int seg = blockIdx.x;
-    const int b = seg_off[seg], n = seg_off[seg + 1] - b;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t *gh = S.hist + (size_t)seg * 8 * 256;
-    uint32_t *go = S.doff + (size_t)seg * 8 * 256;
-    for (int d = warp; d < npasses; d += blockDim.x >> 5)
-    {
-        uint32_t c[8], sum = 0;
-        bool triv = n <= 1;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-        {
-            c[k] = gh[d * 256 + 8 * lane + k];
-            sum += c[k];
-            triv |= (int)c[k] == n;
-        }
-        uint32_t incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o)
-                incl += y;
-        }
-        uint32_t run = (uint32_t)b + incl - sum;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-        {
-            go[d * 256 + 8 * lane + k] = run;
-            run += c[k];
-        }
-        triv = __any_sync(0xffffffffu, triv);
-        if (lane == 0 && !triv)
-            atomicOr(&ctl->nontrivial[d], 1);
-    }
-    if (threadIdx.x == 0)
-        S.tile_first[seg + 1] = (n + kSortTile - 1) / kSortTile;
-    __shared__ int s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0)
-        s_last = atomicAdd(&ctl->prep_ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last)
-        return;
-    __threadfence();
-    // exclusive prefix of the tile counts (P <= 4096: 16 per thread, then a block scan)
-    __shared__ int s_part[256];
-    constexpr int kPer = (kMaxSegments + 255) / 256;
-    const int p0 = threadIdx.x * kPer;
-    int cnt[kPer], sum = 0;
-#pragma unroll
-    for (int k = 0; k < kPer; ++k)
-    {
-        cnt[k] = p0 + k < P ? __ldcg(&S.tile_first[p0 + k + 1]) : 0;
-        sum += cnt[k];
-    }
-    s_part[threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.x < 32)
-    {
-        int v[8], t = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-        {
-            v[k] = s_part[threadIdx.x * 8 + k];
-            t += v[k];
-        }
-        int incl = t;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((int)threadIdx.x >= o)
-                incl += y;
-        }
-        int run = incl - t;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-        {
-            s_part[threadIdx.x * 8 + k] = run;
-            run += v[k];
-        }
-    }
-    __syncthreads();
-    int run = s_part[threadIdx.x];
-#pragma unroll
-    for (int k = 0; k < kPer; ++k)
-        if (p0 + k < P)
-        {
-            S.tile_first[p0 + k] = run;
-            run += cnt[k];
-        }
-    if (threadIdx.x == 255)
-    {
-        // the last thread's running sum is the total
-        ctl->ntiles = run;
-        S.tile_first[P] = run;
-    }
-    if (threadIdx.x == 0)
-    {
-        int sel = 0;
-        for (int d = 0; d < npasses; ++d)
-        {
-            ctl->in_sel[d] = sel;
-            if (__ldcg(&ctl->nontrivial[d]))
-                sel ^= 1;
-        }
-        *d_sel = sel;
-    }
 }
 
 // the lanes of the warp whose value equals this lane's, for values below 512: one
@@ -264,7 +77,7 @@ struct TileJob
 
 // one tile of a pass: rank, stage in tile order, look back, scatter.  Packed keys carry
 // their index, so that variant holds no value registers.
-template <bool Packed>
+template <bool Packed, int kLook>
 __device__ __forceinline__ void sort_tile(const TileJob &J, SortCtl *ctl, const SortSeg &S, int *d_err,
                                           uint32_t (*s_whist)[256], uint32_t *s_excl, uint32_t *s_gbase,
                                           uint64_t *s_keys, int32_t *s_vals, uint32_t *s_wsum)
@@ -365,19 +178,19 @@ __device__ __forceinline__ void sort_tile(const TileJob &J, SortCtl *ctl, const 
     uint32_t excl = 0;
     if ((int)tile > first)
     {
-        // the predecessors' states for this digit, kLookWindow at a time (independent
+        // the predecessors' states for this digit, kLook at a time (independent
         // relaxed loads), consumed nearest first up to the nearest inclusive one (the
         // segment's first tile publishes an inclusive state at once)
         bool found = false;
         const uint32_t limit = wait_limit(d_err);
-        for (int64_t p = (int64_t)tile - 1; p >= first && !found; p -= kLookWindow)
+        for (int64_t p = (int64_t)tile - 1; p >= first && !found; p -= kLook)
         {
-            uint32_t s[kLookWindow];
+            uint32_t s[kLook];
 #pragma unroll
-            for (int j = 0; j < kLookWindow; ++j)
+            for (int j = 0; j < kLook; ++j)
                 s[j] = p - j >= first ? ld_relaxed(status + (p - j) * 256 + t) : kFlagInc;
 #pragma unroll
-            for (int j = 0; j < kLookWindow; ++j)
+            for (int j = 0; j < kLook; ++j)
             {
                 if (found)
                     break;
@@ -415,7 +228,8 @@ __device__ __forceinline__ void sort_tile(const TileJob &J, SortCtl *ctl, const 
     }
 }
 
-__global__ void __launch_bounds__(kSortThreads, 4) k_sort_pass(
+template <int kLook>
+__global__ void __launch_bounds__(kSortThreads, kLook == kLookWindow ? 4 : 2) k_sort_pass(
     uint64_t *keys0, int32_t *vals0, uint64_t *keys1, int32_t *vals1, SortCtl *ctl, SortSeg S,
     const int32_t *seg_off, int P, uint32_t *status_base, int64_t status_words, int pass, const int *d_ib,
     const int *d_kshift, int *d_err)
@@ -473,51 +287,62 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_pass(
     const int shift = *d_kshift + pass * 8;
     const TileJob J{tile, first, seg, seg_b, seg_e, tile_base, cnt, shift, pass, kin, vin, kout, vout, status};
     if (*d_ib != 0)
-        sort_tile<true>(J, ctl, S, d_err, s_whist, s_excl, s_gbase, s_keys, s_vals, s_wsum);
+        sort_tile<true, kLook>(J, ctl, S, d_err, s_whist, s_excl, s_gbase, s_keys, s_vals, s_wsum);
     else
-        sort_tile<false>(J, ctl, S, d_err, s_whist, s_excl, s_gbase, s_keys, s_vals, s_wsum);
+        sort_tile<false, kLook>(J, ctl, S, d_err, s_whist, s_excl, s_gbase, s_keys, s_vals, s_wsum);
 }
 
-int radix_sort(gca3d_context *ctx, SortBuffers &sb, const int32_t *seg_off, int P, int64_t cap, int64_t max_seg_cap,
-               int max_bits)
+int sort_plan(gca3d_context *ctx, int P, int64_t cap, size_t zero_bytes, SortPlan &sp)
+{
+    if (P < 1 || P > kMaxSegments)
+        return fail(ctx, GCA3D_ERR_INVALID_VALUE, "radix sort: segment count");
+    // tiles never straddle segments: at most one partial tile per segment more
+    sp.ntiles = (cap + kSortTile - 1) / kSortTile + P;
+    sp.status_words = sp.ntiles * 256;
+    sp.status = ctx->arena.get<uint32_t>(2 * sp.status_words);
+    sp.S.doff = ctx->arena.get<uint32_t>((size_t)P * 8 * 256);
+    sp.S.tile_first = ctx->arena.get<int32_t>(P + 1);
+    // everything that starts at zero, in one block: control words, histograms, tickets, and
+    // what the caller adds
+    const size_t hist = sizeof(SortCtl), ticket = hist + sizeof(uint32_t) * (size_t)P * 8 * 256,
+                 extra = (ticket + sizeof(uint32_t) * 2 * (size_t)P + 15) & ~size_t(15);
+    char *zero = ctx->arena.get<char>(extra + zero_bytes);
+    if (!sp.status || !sp.S.doff || !sp.S.tile_first || !zero)
+        return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "radix sort: scratch");
+    sp.ctl = reinterpret_cast<SortCtl *>(zero);
+    sp.S.hist = reinterpret_cast<uint32_t *>(zero + hist);
+    sp.S.ticket = reinterpret_cast<uint32_t *>(zero + ticket);
+    sp.zeroed = zero + extra;
+    GCA_CUDA(ctx, cudaMemsetAsync(zero, 0, extra + zero_bytes, ctx->stream));
+    return GCA3D_OK;
+}
+
+int sort_passes(gca3d_context *ctx, SortBuffers &sb, const SortPlan &sp, const int32_t *seg_off, int P)
 {
     // four resident tiles per SM (47 KB of shared memory each) need the shared-memory side
     // of the L1 carveout
-    static const bool carveout = cudaFuncSetAttribute(k_sort_pass, cudaFuncAttributePreferredSharedMemoryCarveout,
+    static const bool carveout = cudaFuncSetAttribute(k_sort_pass<kLookWindow>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                                       cudaSharedmemCarveoutMaxShared) == cudaSuccess;
     (void)carveout;
-    if (P < 1 || P > kMaxSegments)
-        return fail(ctx, GCA3D_ERR_INVALID_VALUE, "radix_sort: segment count");
-    const int npasses = max_bits <= 0 ? 1 : (max_bits + 7) / 8;
-    // tiles never straddle segments: at most one partial tile per segment more
-    const int64_t ntiles = (cap + kSortTile - 1) / kSortTile + P;
-    const int64_t status_words = ntiles * 256;
-    SortCtl *ctl = ctx->arena.get<SortCtl>(1);
-    uint32_t *status = ctx->arena.get<uint32_t>(2 * status_words);
-    SortSeg S;
-    S.hist = ctx->arena.get<uint32_t>((size_t)P * 8 * 256);
-    S.doff = ctx->arena.get<uint32_t>((size_t)P * 8 * 256);
-    S.tile_first = ctx->arena.get<int32_t>(P + 1);
-    if (!ctl || !status || !sb.d_sel || !S.hist || !S.doff || !S.tile_first)
-        return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "radix_sort: scratch");
-    GCA_CUDA(ctx, cudaMemsetAsync(ctl, 0, sizeof(SortCtl), ctx->stream));
-    GCA_CUDA(ctx, cudaMemsetAsync(S.hist, 0, sizeof(uint32_t) * (size_t)P * 8 * 256, ctx->stream));
-    // about 16 keys per thread in the largest segment (blocks past a smaller segment's end
-    // return at once), so uneven segments do not leave one segment's blocks looping
-    const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(grid_for(max_seg_cap, kBlock * 16),
-                                                               ((int64_t)ctx->num_sms * 32 + P - 1) / P));
-    k_sort_hist<<<dim3(gx, P), kBlock, 0, ctx->stream>>>(sb.keys[0], seg_off, sb.d_kshift, S, status, status_words);
-    GCA_CHECK_LAUNCH(ctx);
     // a trivial pass returns at once (conditional graph nodes around the passes, which
     // would skip the launch, measured slower: 13.4 against 13.0 ms per batch64 execute)
-    k_sort_prep<<<P, 256, 0, ctx->stream>>>(ctl, S, seg_off, P, npasses, sb.d_sel);
-    GCA_CHECK_LAUNCH(ctx);
-    for (int p = 0; p < npasses; ++p)
+    for (int p = 0; p < 8; ++p)
     {
         GCA_PROF_BEGIN(ctx, kKidSortPass);
-        k_sort_pass<<<(int)ntiles, kSortThreads, 0, ctx->stream>>>(sb.keys[0], sb.vals[0], sb.keys[1], sb.vals[1],
-                                                                   ctl, S, seg_off, P, status, status_words, p,
-                                                                   sb.d_ib, sb.d_kshift, ctx->d_err);
+        auto pass = [&](auto kernel) {
+            kernel<<<(int)sp.ntiles, kSortThreads, 0, ctx->stream>>>(sb.keys[0], sb.vals[0], sb.keys[1], sb.vals[1],
+                                                                    sp.ctl, sp.S, seg_off, P, sp.status,
+                                                                    sp.status_words, p, sb.d_ib, sb.d_kshift,
+                                                                    ctx->d_err);
+        };
+        // with at most one tile per resident block slot every tile starts at once, so a late
+        // tile's look-back reads all its predecessors: 32 at a time.  With more tiles most
+        // predecessors are done, and the wider window's registers cost more than it saves
+        // (batch64 +2 % at 16, +7 % at 32)
+        if (sp.ntiles <= 2 * ctx->num_sms)
+            pass(k_sort_pass<kLookWide>);
+        else
+            pass(k_sort_pass<kLookWindow>);
         GCA_CHECK_LAUNCH(ctx);
         GCA_PROF_END(ctx, kKidSortPass);
     }
@@ -686,7 +511,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const Op op_in, const int
 // its first position (starts[runs] = n) and seg_first[seg] the segment's first run
 __global__ void __launch_bounds__(kScanThreads) k_run_scan(SortBuffers sb, const KeyLayout *lay, const int32_t *d_n,
                                                            ScanCtl *ctl, unsigned long long *status, int32_t *starts,
-                                                           int32_t *seg_first, int32_t *d_runs, int *d_err)
+                                                           int32_t *seg_first, int32_t *d_runs, int32_t *seg_off,
+                                                           int32_t *d_count, int *d_err)
 {
     __shared__ uint32_t s_tile;
     __shared__ long long s_wsum[kScanThreads / 32];
@@ -704,6 +530,10 @@ __global__ void __launch_bounds__(kScanThreads) k_run_scan(SortBuffers sb, const
         {
             *d_runs = 0; // empty input
             starts[0] = 0;
+            if (seg_off)
+                seg_off[0] = seg_off[1] = 0;
+            if (d_count)
+                *d_count = 0;
         }
         return;
     }
@@ -757,6 +587,13 @@ __global__ void __launch_bounds__(kScanThreads) k_run_scan(SortBuffers sb, const
             {
                 *d_runs = (int32_t)(excl + agg);
                 starts[excl + agg] = n;
+                if (seg_off)
+                {
+                    seg_off[0] = 0;
+                    seg_off[1] = (int32_t)(excl + agg);
+                }
+                if (d_count)
+                    *d_count = (int32_t)(excl + agg);
             }
         }
     }
@@ -772,7 +609,7 @@ __global__ void __launch_bounds__(kScanThreads) k_run_scan(SortBuffers sb, const
         if (f & 1u)
         {
             starts[run] = base + j;
-            if (f & 2u || base + j == 0)
+            if (seg_first && (f & 2u || base + j == 0))
                 seg_first[L.bseg ? (int)(sv.key(base + j) >> segshift) : 0] = (int32_t)run;
             ++run;
         }
@@ -795,18 +632,26 @@ int exclusive_scan(gca3d_context *ctx, const int32_t *in, int32_t *out, const in
     return GCA3D_OK;
 }
 
-int run_scan(gca3d_context *ctx, const SortBuffers &sb, const int32_t *d_n, int64_t cap, const KeyLayout *lay,
-             int32_t *starts, int32_t *seg_first, int32_t *d_runs)
+size_t run_scan_zero_bytes(int64_t cap)
 {
-    const int64_t ntiles = (cap + kScanTile - 1) / kScanTile;
-    ScanCtl *ctl = ctx->arena.get<ScanCtl>(1);
-    unsigned long long *status = ctx->arena.get<unsigned long long>(ntiles > 0 ? ntiles : 1);
-    if (!ctl || !status)
-        return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "run_scan: scratch");
-    GCA_CUDA(ctx, cudaMemsetAsync(ctl, 0, sizeof(ScanCtl), ctx->stream));
-    GCA_CUDA(ctx, cudaMemsetAsync(status, 0, sizeof(unsigned long long) * (ntiles > 0 ? ntiles : 1), ctx->stream));
-    k_run_scan<<<(int)(ntiles > 0 ? ntiles : 1), kScanThreads, 0, ctx->stream>>>(sb, lay, d_n, ctl, status, starts,
-                                                                                 seg_first, d_runs, ctx->d_err);
+    return sizeof(unsigned long long) * (size_t)((cap + kScanTile - 1) / kScanTile + 2);
+}
+
+int run_scan(gca3d_context *ctx, const SortBuffers &sb, const int32_t *d_n, int64_t cap, const KeyLayout *lay,
+             int32_t *starts, int32_t *seg_first, int32_t *d_runs, int32_t *seg_off, int32_t *d_count, void *zeroed)
+{
+    const int64_t ntiles = std::max<int64_t>((cap + kScanTile - 1) / kScanTile, 1);
+    if (!zeroed)
+    {
+        zeroed = ctx->arena.get<char>(run_scan_zero_bytes(cap));
+        if (!zeroed)
+            return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "run_scan: scratch");
+        GCA_CUDA(ctx, cudaMemsetAsync(zeroed, 0, run_scan_zero_bytes(cap), ctx->stream));
+    }
+    unsigned long long *words = static_cast<unsigned long long *>(zeroed); // the tile ticket, then a state per tile
+    k_run_scan<<<(int)ntiles, kScanThreads, 0, ctx->stream>>>(sb, lay, d_n, reinterpret_cast<ScanCtl *>(words),
+                                                              words + 1, starts, seg_first, d_runs, seg_off, d_count,
+                                                              ctx->d_err);
     GCA_CHECK_LAUNCH(ctx);
     return GCA3D_OK;
 }

@@ -22,6 +22,8 @@ struct Batch
     int P = 0;
     int64_t cap = 0;         // total capacity
     int64_t max_seg_cap = 0; // largest segment capacity
+    // set: seg_off is still to be written as {0, *d_count}, by the batch's grid build
+    const int32_t *d_count = nullptr;
 };
 
 // a source cloud of a batched stage, read through a device pointer table
@@ -89,8 +91,9 @@ int icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *const *src,
                              const gca3d_icp_params *params, bool capture, PlanPrologue prologue,
                              gca3d_icp_plan **out, const PlanVoxels *voxels = nullptr);
 
-// a single-segment batch view of a cloud (no copy; segment offsets from the arena)
-int cloud_batch(gca3d_context *ctx, gca3d_cloud *c, Batch &b);
+// a single-segment batch view of a cloud (no copy; segment offsets from the arena, with
+// by_grid written by the batch's grid build)
+int cloud_batch(gca3d_context *ctx, gca3d_cloud *c, Batch &b, bool by_grid);
 
 // allocate a batch from the context arena
 int batch_alloc(gca3d_context *ctx, Batch &b, int P, int64_t cap, int64_t max_seg_cap, bool nrm, bool grd);
@@ -105,6 +108,7 @@ struct SubLevels
 {
     int n = 0;
     float voxel[kMaxSubLevels] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float inv[kMaxSubLevels] = {0.0f, 0.0f, 0.0f, 0.0f}; // 1 / voxel
 };
 
 // the sorted state of a voxel stage that finer scales refine instead of sorting again
@@ -122,9 +126,11 @@ struct VoxelChain
 // voxel-grid downsampling of P segments; morton: Z-order keys; finer (with morton):
 // carry the sub-cell bits of finer scales and record the sorted state in *chain, which
 // voxel_refine then turns into each finer scale's downsampling, in order
-int voxel_stage(gca3d_context *ctx, const SegSrc *d_src, int P, int64_t total_cap, int64_t max_seg_cap,
+// one: the single source by value (P = 1), in place of a table already in d_src, which the
+// stage then writes; d_count: the output count goes there too
+int voxel_stage(gca3d_context *ctx, SegSrc *d_src, int P, int64_t total_cap, int64_t max_seg_cap,
                 float voxel, Batch &out, bool morton = false, const SubLevels *finer = nullptr,
-                VoxelChain *chain = nullptr);
+                VoxelChain *chain = nullptr, const SegSrc *one = nullptr, int32_t *d_count = nullptr);
 int voxel_refine(gca3d_context *ctx, const SegSrc *d_src, VoxelChain &chain, Batch &out);
 int gather_stage(gca3d_context *ctx, const SegSrc *d_src, int P, int64_t max_seg_cap, Batch &out,
                  bool with_normals);

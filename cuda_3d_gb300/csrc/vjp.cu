@@ -410,7 +410,7 @@ extern "C" int gca3d_color_icp_vjp(gca3d_context *ctx, gca3d_cloud *src, gca3d_c
 
     Batch bs, bt;
     int st;
-    if ((st = cloud_batch(ctx, src, bs)) || (st = cloud_batch(ctx, tgt, bt)))
+    if ((st = cloud_batch(ctx, src, bs, false)) || (st = cloud_batch(ctx, tgt, bt, true)))
         return st;
     Grid g;
     if ((st = grid_build(ctx, bt, p->max_corr, kOriginPadF32, nullptr, g)))

@@ -11,6 +11,7 @@
 // ascending original index (the sort is stable), so the downsampled set is
 // bit-exact against the oracle; the mean is xyz / n and rgb * (1 / n) as in
 // src/geometry/type.hpp:58-62.
+#include "cluster_sort.cuh"
 #include "stages.cuh"
 
 #include <algorithm>
@@ -68,89 +69,6 @@ __global__ void k_src_prefix(const SegSrc *src, int P, int32_t *off)
         off[P] = s_base;
 }
 
-__global__ void k_src_bounds_init(int *ord, int P)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 6 * P)
-        ord[i] = (i % 6) < 3 ? float_to_ordered(3.402823466e38f) : float_to_ordered(-3.402823466e38f);
-}
-
-__global__ void k_src_bounds(const SegSrc *src, int *ord)
-{
-    const int seg = blockIdx.y;
-    const int n = *src[seg].d_n;
-    if ((int64_t)blockIdx.x * blockDim.x >= n)
-        return;
-    const float4 *pos = src[seg].pos;
-    float mn[3] = {3.402823466e38f, 3.402823466e38f, 3.402823466e38f};
-    float mx[3] = {-3.402823466e38f, -3.402823466e38f, -3.402823466e38f};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        float4 p = pos[i];
-        mn[0] = fminf(mn[0], p.x), mn[1] = fminf(mn[1], p.y), mn[2] = fminf(mn[2], p.z);
-        mx[0] = fmaxf(mx[0], p.x), mx[1] = fmaxf(mx[1], p.y), mx[2] = fmaxf(mx[2], p.z);
-    }
-    block_bounds_commit(mn, mx, ord + 6 * seg);
-}
-
-// key layout shared by all segments; per-segment origin = unpadded aabb min.  With
-// morton (and room in 64 bits) the three axis keys are bit-interleaved below the
-// segment index instead: the voxels then come out in Z-order, so runs of
-// consecutive output points are compact in space (the correspondence search of the
-// ICP stages a block's target cells once for such a run).
-__global__ void k_voxel_layout(const int *ord, int P, float voxel, bool morton, int sub_bits, float3 *origin,
-                               KeyLayout *lay, int *d_err)
-{
-    __shared__ uint32_t s_max[3];
-    if (threadIdx.x < 3)
-        s_max[threadIdx.x] = 0;
-    __syncthreads();
-    for (int s = threadIdx.x; s < P; s += blockDim.x)
-    {
-        float mn[3], mx[3];
-        for (int a = 0; a < 3; ++a)
-        {
-            mn[a] = ordered_to_float(ord[6 * s + a]);
-            mx[a] = ordered_to_float(ord[6 * s + 3 + a]);
-        }
-        origin[s] = make_float3(mn[0], mn[1], mn[2]);
-        if (!(mx[0] >= mn[0])) // empty segment
-            continue;
-        for (int a = 0; a < 3; ++a)
-        {
-            int k = cell_of(mx[a], mn[a], voxel);
-            if (k < 0 || k >= (1 << 21))
-            {
-                atomicOr(d_err, kErrKeyBits);
-                k = (1 << 21) - 1;
-            }
-            atomicMax(&s_max[a], (uint32_t)k);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        KeyLayout L;
-        L.bseg = bitlen_u32((uint32_t)(P - 1));
-        L.bx = max(1, bitlen_u32(s_max[0]));
-        L.by = max(1, bitlen_u32(s_max[1]));
-        L.bz = max(1, bitlen_u32(s_max[2]));
-        L.total_bits = L.bseg + L.bx + L.by + L.bz;
-        L.morton = 0;
-        const int b = max(L.bx, max(L.by, L.bz));
-        if (morton && L.bseg + 3 * b + sub_bits <= 64)
-        {
-            L.bx = L.by = L.bz = b;
-            L.total_bits = L.bseg + 3 * b;
-            L.morton = 1;
-        }
-        // sub-cell bits for finer scales ride below a Z-order key
-        if (L.total_bits + sub_bits > 64 || (sub_bits && !L.morton))
-            atomicOr(d_err, kErrKeyBits);
-        *lay = L;
-    }
-}
-
 // the bits of v (up to 21) at every third position (bit interleaving by masks)
 __device__ __forceinline__ uint64_t spread3(uint64_t v)
 {
@@ -163,47 +81,119 @@ __device__ __forceinline__ uint64_t spread3(uint64_t v)
     return v;
 }
 
-__global__ void k_voxel_keys(const SegSrc *src, const int32_t *off, const float3 *origin, const KeyLayout *lay,
-                             float voxel, SubLevels sub, uint64_t *keys, int32_t *vals, int ib_cap, int *d_ib,
-                             int *d_kshift, int *d_err)
+// the largest voxel key per axis of a set with bounds mn, mx (untouched when it is empty);
+// error bits
+__device__ __forceinline__ int voxel_extent(const float mn[3], const float mx[3], float voxel, uint32_t cells[3])
 {
-    const int seg = blockIdx.y;
-    const int n = *src[seg].d_n;
-    const int base = off[seg];
-    const KeyLayout L = *lay;
-    const int sb = 3 * sub.n;
-    const int ib = packed_index_bits(L.total_bits + sb, ib_cap);
-    if (seg == 0 && blockIdx.x == 0 && threadIdx.x == 0)
+    if (!(mx[0] >= mn[0]))
+        return 0;
+    int err = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
     {
-        *d_ib = ib;
-        *d_kshift = ib + sb;
-    }
-    const float3 o = origin[seg];
-    const float4 *pos = src[seg].pos;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        float4 p = pos[i];
-        uint64_t kx = (uint32_t)cell_of(p.x, o.x, voxel), ky = (uint32_t)cell_of(p.y, o.y, voxel),
-                 kz = (uint32_t)cell_of(p.z, o.z, voxel);
-        uint64_t key = ((uint64_t)seg << (L.bx + L.by + L.bz)) |
-                       (L.morton ? (spread3(kx) << 2) | (spread3(ky) << 1) | spread3(kz)
-                                 : (kx << (L.by + L.bz)) | (ky << L.bz) | kz);
-        // each finer scale's cells, as that scale computes them: with its voxel half the
-        // previous one, its quotient is exactly twice the previous one, so each axis adds
-        // one bit (x, y, z -- the next three bits of the finer Z-order key)
-        for (int l = 0; l < sub.n; ++l)
+        int k = cell_of(mx[a], mn[a], voxel);
+        if (k < 0 || k >= (1 << 21))
         {
-            const uint64_t fx = (uint32_t)cell_of(p.x, o.x, sub.voxel[l]), fy = (uint32_t)cell_of(p.y, o.y, sub.voxel[l]),
-                           fz = (uint32_t)cell_of(p.z, o.z, sub.voxel[l]);
-            const uint64_t bx = fx - 2 * kx, by = fy - 2 * ky, bz = fz - 2 * kz;
-            if ((bx | by | bz) > 1)
-                atomicOr(d_err, kErrInvalid);
-            key = (key << 3) | ((bx & 1) << 2) | ((by & 1) << 1) | (bz & 1);
-            kx = fx, ky = fy, kz = fz;
+            err = kErrKeyBits;
+            k = (1 << 21) - 1;
         }
-        sort_store(keys, vals, base + i, key, ib);
+        cells[a] = (uint32_t)k;
     }
+    return err;
 }
+
+// a point's voxel key with the sub-cell bits of the finer scales below it
+__device__ __forceinline__ uint64_t voxel_key(float4 p, int seg, const KeyLayout &L, float3 o, float voxel,
+                                              float inv, const SubLevels &sub, int *d_err)
+{
+    uint64_t kx = (uint32_t)cell_of_inv(p.x, o.x, voxel, inv), ky = (uint32_t)cell_of_inv(p.y, o.y, voxel, inv),
+             kz = (uint32_t)cell_of_inv(p.z, o.z, voxel, inv);
+    uint64_t key = ((uint64_t)seg << (L.bx + L.by + L.bz)) |
+                   (L.morton ? (spread3(kx) << 2) | (spread3(ky) << 1) | spread3(kz)
+                             : (kx << (L.by + L.bz)) | (ky << L.bz) | kz);
+    // each finer scale's cells, as that scale computes them: with its voxel half the
+    // previous one, its quotient is exactly twice the previous one, so each axis adds
+    // one bit (x, y, z -- the next three bits of the finer Z-order key)
+#pragma unroll
+    for (int l = 0; l < kMaxSubLevels; ++l)
+    {
+        if (l >= sub.n)
+            break;
+        const float fv = sub.voxel[l], fi = sub.inv[l];
+        const uint64_t fx = (uint32_t)cell_of_inv(p.x, o.x, fv, fi), fy = (uint32_t)cell_of_inv(p.y, o.y, fv, fi),
+                       fz = (uint32_t)cell_of_inv(p.z, o.z, fv, fi);
+        const uint64_t bx = fx - 2 * kx, by = fy - 2 * ky, bz = fz - 2 * kz;
+        if ((bx | by | bz) > 1)
+            atomicOr(d_err, kErrInvalid);
+        key = (key << 3) | ((bx & 1) << 2) | ((by & 1) << 1) | (bz & 1);
+        kx = fx, ky = fy, kz = fz;
+    }
+    return key;
+}
+
+// the voxel keys of P sets, read through the source table; a single source may come by value
+// instead (begin then writes the table, which the reduction reads)
+struct VoxelMaker
+{
+    SegSrc *table;
+    SegSrc one;
+    bool single, by_value;
+    int32_t *in_off; // element ranges; written {0, n} by begin for a single source
+    float voxel, inv;
+    bool morton;
+    SubLevels sub;
+    __device__ int2 range(int seg) const
+    {
+        return single ? make_int2(0, by_value ? *one.d_n : *table->d_n) : make_int2(in_off[seg], in_off[seg + 1]);
+    }
+    __device__ float4 point(int seg, int i) const
+    {
+        return single ? __ldg((by_value ? one.pos : table->pos) + i) : __ldg(table[seg].pos + (i - in_off[seg]));
+    }
+    __device__ int sub_bits() const { return 3 * sub.n; }
+    __device__ void begin(int n) const
+    {
+        in_off[0] = 0;
+        in_off[1] = n;
+        if (by_value)
+            *table = one;
+    }
+    // the origin is the unpadded aabb min
+    __device__ int segment(const float mn[3], const float mx[3], float3 &o, uint32_t cells[3]) const
+    {
+        o = make_float3(mn[0], mn[1], mn[2]);
+        return voxel_extent(mn, mx, voxel, cells);
+    }
+    // With morton (and room in 64 bits) the three axis keys are bit-interleaved below the
+    // segment index: the voxels then come out in Z-order, so runs of consecutive output
+    // points are compact in space (the correspondence search of the ICP stages a block's
+    // target cells once for such a run).
+    __device__ int layout(const uint32_t cells[3], int P, KeyLayout &L) const
+    {
+        const int sub_bits = 3 * sub.n;
+        L.bseg = bitlen_u32((uint32_t)(P - 1));
+        L.bx = max(1, bitlen_u32(cells[0]));
+        L.by = max(1, bitlen_u32(cells[1]));
+        L.bz = max(1, bitlen_u32(cells[2]));
+        L.total_bits = L.bseg + L.bx + L.by + L.bz;
+        L.morton = 0;
+        const int b = max(L.bx, max(L.by, L.bz));
+        if (morton && L.bseg + 3 * b + sub_bits <= 64)
+        {
+            L.bx = L.by = L.bz = b;
+            L.total_bits = L.bseg + 3 * b;
+            L.morton = 1;
+        }
+        // sub-cell bits for finer scales ride below a Z-order key
+        return L.total_bits + sub_bits > 64 || (sub_bits && !L.morton) ? kErrKeyBits : 0;
+    }
+    __device__ uint64_t key(float4 p, int seg, const KeyLayout &L, float3 o, int *d_err) const
+    {
+        return voxel_key(p, seg, L, o, voxel, inv, sub, d_err);
+    }
+};
+
+bool voxel_cluster_enable() { return cluster_sort_enable<VoxelMaker>(); }
 
 // segment offsets of the output; empty segments start where the next one does
 __global__ void k_seg_first_to_offsets(const int32_t *seg_first, int P, const int32_t *d_m, int32_t *off)
@@ -333,28 +323,43 @@ __global__ void k_voxel_refine(SortBuffers sb, const int32_t *starts, const int3
     }
 }
 
+// the sums of the voxels whose runs are known
+static int voxel_sums(gca3d_context *ctx, const SegSrc *d_src, int64_t total_cap, const int32_t *in_off,
+                      const SortBuffers &sb, const KeyLayout *lay, Batch &out, const int32_t *starts, const int32_t *d_m)
+{
+    const int gs = std::min(grid_for(total_cap), ctx->num_sms * 8);
+    GCA_PROF_BEGIN(ctx, kKidVoxelReduce);
+    k_voxel_reduce<<<gs, kBlock, 0, ctx->stream>>>(d_src, in_off, sb, starts, d_m, lay, out.pos, out.col, ctx->d_err);
+    GCA_CHECK_LAUNCH(ctx);
+    GCA_PROF_END(ctx, kKidVoxelReduce);
+    return GCA3D_OK;
+}
+
 // the runs of equal keys (voxels) of the sorted view and their sums: the part of a voxel
 // stage after its order is known
 static int voxel_reduce_stage(gca3d_context *ctx, const SegSrc *d_src, int P, int64_t total_cap,
                               const int32_t *in_off, const SortBuffers &sb, const KeyLayout *lay, Batch &out,
-                              int32_t *starts, int32_t *d_m)
+                              int32_t *starts, int32_t *d_m, int32_t *d_count = nullptr, void *zeroed = nullptr)
 {
     Arena &A = ctx->arena;
     const int64_t cap = std::max<int64_t>(total_cap, 1);
+    const int32_t *d_n = in_off + P;
+    int st;
+    if (P == 1) // the scan writes the one segment's offsets itself
+    {
+        if ((st = run_scan(ctx, sb, d_n, cap, lay, starts, nullptr, d_m, out.seg_off, d_count, zeroed)))
+            return st;
+        return voxel_sums(ctx, d_src, total_cap, in_off, sb, lay, out, starts, d_m);
+    }
     int32_t *seg_count = A.get<int32_t>(P);
     if (!seg_count)
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "voxel_stage: scratch");
     cudaStream_t s = ctx->stream;
-    const int32_t *d_n = in_off + P;
-    const int gs = std::min(grid_for(total_cap), ctx->num_sms * 8);
     GCA_CUDA(ctx, cudaMemsetAsync(seg_count, 0xFF, sizeof(int32_t) * P, s));
-    int st = run_scan(ctx, sb, d_n, cap, lay, starts, seg_count, d_m);
-    if (st)
+    if ((st = run_scan(ctx, sb, d_n, cap, lay, starts, seg_count, d_m, nullptr, nullptr, zeroed)))
         return st;
-    GCA_PROF_BEGIN(ctx, kKidVoxelReduce);
-    k_voxel_reduce<<<gs, kBlock, 0, s>>>(d_src, in_off, sb, starts, d_m, lay, out.pos, out.col, ctx->d_err);
-    GCA_CHECK_LAUNCH(ctx);
-    GCA_PROF_END(ctx, kKidVoxelReduce);
+    if ((st = voxel_sums(ctx, d_src, total_cap, in_off, sb, lay, out, starts, d_m)))
+        return st;
     k_seg_first_to_offsets<<<1, 32, 0, s>>>(seg_count, P, d_m, out.seg_off);
     GCA_CHECK_LAUNCH(ctx);
     return GCA3D_OK;
@@ -394,15 +399,15 @@ int voxel_refine(gca3d_context *ctx, const SegSrc *d_src, VoxelChain &c, Batch &
     return GCA3D_OK;
 }
 
-int voxel_stage(gca3d_context *ctx, const SegSrc *d_src, int P, int64_t total_cap, int64_t max_seg_cap,
-                float voxel, Batch &out, bool morton, const SubLevels *finer, VoxelChain *chain)
+int voxel_stage(gca3d_context *ctx, SegSrc *d_src, int P, int64_t total_cap, int64_t max_seg_cap,
+                float voxel, Batch &out, bool morton, const SubLevels *finer, VoxelChain *chain, const SegSrc *one,
+                int32_t *d_count)
 {
     if (!(voxel > 0.0f))
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "voxel size must be > 0");
     Arena &A = ctx->arena;
     const int64_t cap = std::max<int64_t>(total_cap, 1);
     int32_t *in_off = A.get<int32_t>(P + 1);
-    int *ord = A.get<int>(6 * P);
     float3 *origin = A.get<float3>(P);
     KeyLayout *lay = A.get<KeyLayout>(1);
     SortBuffers sb;
@@ -415,7 +420,7 @@ int voxel_stage(gca3d_context *ctx, const SegSrc *d_src, int P, int64_t total_ca
     sb.d_kshift = A.get<int>(1);
     int32_t *starts = A.get<int32_t>(cap + 1);
     int32_t *d_m = A.get<int32_t>(1);
-    if (!in_off || !ord || !origin || !lay || !sb.keys[1] || !sb.vals[1] || !sb.d_sel || !sb.d_ib || !sb.d_kshift ||
+    if (!in_off || !origin || !lay || !sb.keys[1] || !sb.vals[1] || !sb.d_sel || !sb.d_ib || !sb.d_kshift ||
         !starts || !d_m)
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "voxel_stage: scratch");
     const SubLevels sub = finer ? *finer : SubLevels{};
@@ -427,25 +432,28 @@ int voxel_stage(gca3d_context *ctx, const SegSrc *d_src, int P, int64_t total_ca
         if (st)
             return st;
     }
-    cudaStream_t s = ctx->stream;
-    k_src_prefix<<<1, 256, 0, s>>>(d_src, P, in_off);
-    GCA_CHECK_LAUNCH(ctx);
-    k_src_bounds_init<<<grid_for(6 * P), kBlock, 0, s>>>(ord, P);
-    GCA_CHECK_LAUNCH(ctx);
-    const int gx = std::min(grid_for(max_seg_cap, kBlock * 4), ctx->num_sms * 4);
-    k_src_bounds<<<dim3(gx, P), kBlock, 0, s>>>(d_src, ord);
-    GCA_CHECK_LAUNCH(ctx);
-    k_voxel_layout<<<1, 256, 0, s>>>(ord, P, voxel, morton, 3 * sub.n, origin, lay, ctx->d_err);
-    GCA_CHECK_LAUNCH(ctx);
-    k_voxel_keys<<<dim3(gx, P), kBlock, 0, s>>>(d_src, in_off, origin, lay, voxel, sub, sb.keys[0], sb.vals[0],
-                                                index_bits(cap), sb.d_ib, sb.d_kshift, ctx->d_err);
-    GCA_CHECK_LAUNCH(ctx);
-    int st = radix_sort(ctx, sb, in_off, P, total_cap, max_seg_cap, 64);
-    if (st)
-        return st;
-    st = voxel_reduce_stage(ctx, d_src, P, total_cap, in_off, sb, lay, out, starts, d_m);
-    if (st)
-        return st;
+    const VoxelMaker mk{d_src, one ? *one : SegSrc{}, P == 1, one != nullptr, in_off, voxel, 1.0f / voxel, morton, sub};
+    int st;
+    if (cluster_sortable(ctx, P, cap))
+    {
+        const ClusterOut co{sb.keys[0], sb.vals[0], sb.d_sel,     sb.d_ib,     sb.d_kshift, lay,
+                            origin,     ctx->d_err, starts,       d_m,         out.seg_off, d_count};
+        if ((st = cluster_sort(ctx, mk, cap, co)) ||
+            (st = voxel_sums(ctx, d_src, total_cap, in_off, sb, lay, out, starts, d_m)))
+            return st;
+    }
+    else
+    {
+        if (P > 1)
+        {
+            k_src_prefix<<<1, 256, 0, ctx->stream>>>(d_src, P, in_off);
+            GCA_CHECK_LAUNCH(ctx);
+        }
+        void *zeroed = nullptr;
+        if ((st = sort_by_keys(ctx, mk, sb, in_off, P, cap, max_seg_cap, lay, origin, run_scan_zero_bytes(cap), &zeroed)) ||
+            (st = voxel_reduce_stage(ctx, d_src, P, total_cap, in_off, sb, lay, out, starts, d_m, d_count, zeroed)))
+            return st;
+    }
     if (chain)
     {
         chain->sb = sb;

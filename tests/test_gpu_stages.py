@@ -210,6 +210,24 @@ def test_voxel_full_size_vs_oracle(ctx, orc, room, v):
     np.testing.assert_array_equal(d["rgb"], oc)
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 1023, 16 * 1024, 16 * 1024 + 1, 13 * 16 * 1024, 13 * 16 * 1024 + 1])
+@pytest.mark.parametrize("extent,voxel", [(2.0, 0.05), (900.0, 0.002), (900.0, 0.0005)])
+def test_voxel_sort_sizes_and_key_widths_vs_oracle(ctx, orc, n, extent, voxel):
+    """both sorts around the line between them (13 x 16 x 1024 points) and at the edges of a
+    block's share, with keys of 18, 57 (sorted in two parts beside the index) and 63 bits; a
+    tenth of the points are repeated, so the order within a voxel shows"""
+    rng = np.random.default_rng(n)
+    xyz = (rng.random((n, 3)) * extent).astype(np.float32)
+    xyz[rng.integers(0, n, n // 10)] = xyz[rng.integers(0, n, n // 10)]
+    rgb = rng.random((n, 3)).astype(np.float32)
+    src, out = ctx.cloud_from(xyz, rgb), ctx.cloud(n)
+    ctx.check(ctx.L.gca3d_voxel_downsample(ctx.h, src.h, voxel, out.h))
+    d = out.download()
+    ox, oc, _, _ = orc.voxel_downsample(xyz, rgb, voxel)
+    np.testing.assert_array_equal(d["xyz"], ox)
+    np.testing.assert_array_equal(d["rgb"], oc)
+
+
 def test_voxel_empty_and_invalid(ctx, N):
     c = ctx.cloud(16)
     out = ctx.cloud(16)
@@ -257,6 +275,24 @@ def test_nn_full_size_vs_oracle(ctx, orc, room):
     for rad in (0.015, 0.05):
         idx = nn_gpu(ctx, q, r, rad)
         np.testing.assert_array_equal(idx, orc.nn_search(q, r, rad, tie=orc.TIE_MIN_INDEX))
+
+
+@pytest.mark.parametrize("n", [17, 16 * 1024 + 1, 13 * 16 * 1024, 13 * 16 * 1024 + 1])
+@pytest.mark.parametrize("extent,radius", [(2.0, 0.1), (800.0, 0.0009)])
+def test_nn_grid_sort_sizes(ctx, n, extent, radius):
+    """grids on both sides of the sorts' line, with short keys and with keys
+    that fill a word, against all distances in FP32"""
+    rng = np.random.default_rng(n)
+    r = (rng.random((n, 3)) * extent).astype(np.float32)
+    q = (r[rng.integers(0, n, 300)] + rng.normal(size=(300, 3)) * radius * 0.3).astype(np.float32)
+    d2 = np.zeros((len(q), n), np.float32)
+    for k in range(3):
+        d = q[:, k, None] - r[None, :, k]
+        d2 += d * d
+    best = d2.argmin(1)
+    want = np.where(d2[np.arange(len(q)), best] < np.float32(radius) * np.float32(radius), best, -1)
+    assert (want >= 0).mean() > 0.5
+    np.testing.assert_array_equal(nn_gpu(ctx, q, r, radius), want)
 
 
 def test_nn_queries_outside_grid(ctx, orc):
