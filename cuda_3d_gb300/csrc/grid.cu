@@ -77,6 +77,7 @@ struct GridMaker
     float cell, inv;
     int mode;
     float3 given;
+    int table_bits; // a direct row table may have 2^table_bits entries
     __device__ int2 range(int seg) const
     {
         return d_count ? make_int2(0, *d_count) : make_int2(seg_off[seg], seg_off[seg + 1]);
@@ -104,6 +105,10 @@ struct GridMaker
         L.bz = bitlen_u32(max(cells[2], 1u));
         L.total_bits = L.bseg + L.bx + L.by + L.bz;
         L.morton = 0;
+        // the shortest runs that fit the table, of four cells at least (a search's window of
+        // three cells then lies in one run or two); without room for whole rows, the hash
+        L.zs = max(min(2, L.bz), L.total_bits - table_bits);
+        L.direct = L.zs <= L.bz && L.bz >= 1 && L.zs >= 1;
         return L.total_bits > 64 ? kErrKeyBits : 0;
     }
     __device__ uint64_t key(float4 p, int seg, const KeyLayout &L, float3 o, int *) const
@@ -114,42 +119,39 @@ struct GridMaker
 
 bool grid_cluster_enable() { return cluster_sort_enable<GridMaker>(); }
 
-__global__ void k_grid_scatter(SortBuffers sb, const int32_t *d_n, const KeyLayout *lay, const float4 *__restrict__ pos,
-                               float4 *spos, int32_t *sidx, float *sint, int *scz, uint64_t *skey, int *err)
+// the points in grid order, and the row table: the first point of a run (direct) or of a row
+// (hash) finds its end by galloping and writes the entry
+__global__ void __launch_bounds__(kBlock) k_grid_scatter(SortBuffers sb, const int32_t *d_n, const KeyLayout *lay,
+                                                         const float4 *__restrict__ pos, float4 *spos, int32_t *sidx,
+                                                         float *sint, int *scz, uint64_t *skey, RowSlot *slots,
+                                                         uint32_t hmask, int *err)
 {
     const int n = *d_n;
     const SortedView sv = sorted_view(sb);
     const KeyLayout L = *lay;
     const uint64_t mz = (1ull << L.bz) - 1;
+    const int shift = L.direct ? L.zs : L.bz;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
     {
-        uint64_t k = sv.key(s);
-        int g = sv.val(s);
+        const uint64_t k = sv.key(s);
+        const int g = sv.val(s);
         if (!GCA_INDEX_OK(g, n, err))
             continue;
-        float4 p = pos[g];
+        const float4 p = __ldg(&pos[g]);
+        const unsigned long long rk = k >> shift;
+        const bool first = s == 0 || (sv.key(s - 1) >> shift) != rk;
         spos[s] = make_float4(p.x, p.y, p.z, __int_as_float((int)(k & mz)));
         sidx[s] = g;
         sint[s] = p.w;
         scz[s] = (int)(k & mz);
-        skey[s] = k;
-    }
-}
-
-__global__ void k_hash_insert(const uint64_t *skey, const int32_t *d_n, const KeyLayout *lay, RowSlot *slots,
-                              uint32_t hmask, int *d_err)
-{
-    const int n = *d_n;
-    const int bz = lay->bz;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
-    {
-        const unsigned long long rk = skey[s] >> bz;
-        if (s > 0 && (skey[s - 1] >> bz) == rk)
+        if (skey)
+            skey[s] = k;
+        if (!first)
             continue;
-        // the end of the row (the keys are sorted): galloping from s, then bisection
-        // of (lo, hi], where lo is in the row and hi is past it or n
+        // the end of the run (the keys are sorted): galloping from s, then bisection
+        // of (lo, hi], where lo is in the run and hi is past it or n
         int lo = s, hi = s + 1, step = 1;
-        while (hi < n && (skey[hi] >> bz) == rk)
+        while (hi < n && (sv.key(hi) >> shift) == rk)
         {
             lo = hi;
             step <<= 1;
@@ -159,29 +161,42 @@ __global__ void k_hash_insert(const uint64_t *skey, const int32_t *d_n, const Ke
         while (hi - lo > 1)
         {
             const int m = (lo + hi) >> 1;
-            if ((skey[m] >> bz) == rk)
+            if ((sv.key(m) >> shift) == rk)
                 lo = m;
             else
                 hi = m;
         }
-        const int e = hi;
+        if (L.direct)
+        {
+            reinterpret_cast<int2 *>(slots)[rk] = make_int2(s, hi);
+            continue;
+        }
         uint32_t h = hash_u64(rk) & hmask;
         bool done = false;
-        for (uint32_t probe = 0; probe <= hmask; ++probe)
+        for (uint32_t probe = 0; probe <= hmask && !done; ++probe)
         {
             const unsigned long long prev = atomicCAS(&slots[h].key, kEmptyKey, rk);
             if (prev == kEmptyKey || prev == rk)
             {
                 slots[h].start = s;
-                slots[h].end = e;
+                slots[h].end = hi;
                 done = true;
-                break;
             }
             h = (h + 1) & hmask;
         }
         if (!done)
-            atomicOr(d_err, kErrCapacity);
+            atomicOr(err, kErrCapacity);
     }
+}
+
+// an empty row table of the size its layout takes
+__global__ void __launch_bounds__(kBlock) k_grid_clear(const KeyLayout *lay, uint4 *slots, uint32_t hcap)
+{
+    const KeyLayout L = *lay;
+    const uint32_t n = L.direct ? max(1u << (L.total_bits - L.zs) >> 1, 1u) : hcap; // 16-byte words
+    const uint32_t ones = 0xffffffffu;
+    for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock)
+        slots[i] = make_uint4(ones, ones, ones, ones);
 }
 
 int grid_build(gca3d_context *ctx, const Batch &b, float cell, int origin_mode, const float *host_origin,
@@ -195,8 +210,12 @@ int grid_build(gca3d_context *ctx, const Batch &b, float cell, int origin_mode, 
     const int P = b.P;
     const int64_t cap = std::max<int64_t>(b.cap, 1);
     uint32_t hcap = 1024;
+    int table_bits = 10; // a direct table takes at most half the hash's memory: 8 bytes per entry
     while ((int64_t)hcap < 2 * cap)
+    {
         hcap <<= 1;
+        ++table_bits;
+    }
     g.cap = cap;
     g.P = P;
     g.hcap = hcap;
@@ -228,8 +247,7 @@ int grid_build(gca3d_context *ctx, const Batch &b, float cell, int origin_mode, 
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "grid_build: scratch");
     cudaStream_t s = ctx->stream;
     const float3 given = host_origin ? make_float3(host_origin[0], host_origin[1], host_origin[2]) : make_float3(0, 0, 0);
-    const int32_t *d_n = b.seg_off + P;
-    const GridMaker mk{b.pos, b.seg_off, b.d_count, cell, 1.0f / cell, origin_mode, given};
+    const GridMaker mk{b.pos, b.seg_off, b.d_count, cell, 1.0f / cell, origin_mode, given, table_bits};
     int st;
     if (cluster_sortable(ctx, P, cap))
         st = cluster_sort(ctx, mk, cap,
@@ -239,14 +257,14 @@ int grid_build(gca3d_context *ctx, const Batch &b, float cell, int origin_mode, 
         st = sort_by_keys(ctx, mk, sb, b.seg_off, P, cap, b.max_seg_cap, d.layout, d.gmin, 0, nullptr);
     if (st)
         return st;
-    const int gs = std::min(grid_for(cap), ctx->num_sms * 8);
+    k_grid_clear<<<ctx->num_sms * 4, kBlock, 0, s>>>(d.layout, reinterpret_cast<uint4 *>(d.slots), hcap);
+    GCA_CHECK_LAUNCH(ctx);
     GCA_PROF_BEGIN(ctx, kKidGridScatter);
-    k_grid_scatter<<<gs, kBlock, 0, s>>>(sb, d_n, d.layout, b.pos, d.spos, d.sidx, d.sint, d.scz, d.skey, ctx->d_err);
+    k_grid_scatter<<<std::min(grid_for(cap), ctx->num_sms * 8), kBlock, 0, s>>>(
+        sb, b.seg_off + P, d.layout, b.pos, d.spos, d.sidx, d.sint, d.scz, P > 1 ? d.skey : nullptr, d.slots, d.hmask,
+        ctx->d_err);
     GCA_CHECK_LAUNCH(ctx);
     GCA_PROF_END(ctx, kKidGridScatter);
-    GCA_CUDA(ctx, cudaMemsetAsync(d.slots, 0xFF, sizeof(RowSlot) * hcap, s));
-    k_hash_insert<<<gs, kBlock, 0, s>>>(d.skey, d_n, d.layout, d.slots, d.hmask, ctx->d_err);
-    GCA_CHECK_LAUNCH(ctx);
     return GCA3D_OK;
 }
 

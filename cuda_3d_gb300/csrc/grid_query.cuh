@@ -14,42 +14,88 @@ struct GridRows
     int lo, hi;
 };
 
-// Probe all 9 rows with independent 16-byte loads (one round of memory latency for
-// the common case where the first slot answers), then resolve the rare collisions.
-// Returns false when p lies outside the grid's key range.
+// What the rows (x, y) of a search hold, N of them at once so that their loads overlap: the
+// part of each row that can contain the z cells [zlo, zhi] (all of it when the table is a
+// hash), as [start, end) in the sorted arrays; empty for a row outside the grid.  row(j, x, y)
+// gives row j and whether it is wanted.
+// A direct table is a load of eight bytes at an index of a few shifts, or two where the
+// window crosses a run; the hash costs about 35 instructions a row for its 64-bit mixing
+// alone, which was a fifth of a correspondence search (batch64: correspondences 6.58 to 5.59
+// ms of an eager execute, normals 2.52 to 2.06; the batch 13.33 to 11.77 ms).  It stays for
+// sets too wide for a table of a few entries per point.
+template <int N, class Row>
+__device__ __forceinline__ void load_rows(const GridDev &g, const KeyLayout &L, int seg, int zlo, int zhi, int2 *out,
+                                          Row &&row)
+{
+    const int mx = (1 << L.bx) - 1, my = (1 << L.by) - 1;
+    if (L.direct)
+    {
+        const int runs = L.bz - L.zs; // bits of the run index within a row
+        const int mz = (1 << L.bz) - 1;
+        const uint32_t b0 = (uint32_t)min(max(zlo, 0), mz) >> L.zs, b1 = (uint32_t)min(max(zhi, 0), mz) >> L.zs;
+        int2 v[N], w[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+        {
+            int x, y;
+            const bool ok = row(j, x, y) && x >= 0 && x <= mx && y >= 0 && y <= my;
+            const uint32_t i = ((((uint32_t)seg << L.bx | (uint32_t)x) << L.by) | (uint32_t)y) << runs;
+            v[j] = ok ? run_load(g.slots, i + b0) : make_int2(-1, -1);
+            w[j] = ok && b1 != b0 ? run_load(g.slots, i + b1) : make_int2(-1, -1);
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            out[j] = make_int2(v[j].x >= 0 ? v[j].x : w[j].x, w[j].x >= 0 ? w[j].y : v[j].y);
+        return;
+    }
+    const unsigned long long segbits = (unsigned long long)seg << (L.bx + L.by);
+    const uint32_t hmask = g.hmask;
+    unsigned long long rk[N];
+    uint32_t h[N];
+    ulonglong2 v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+    {
+        int x, y;
+        const bool ok = row(j, x, y) && x >= 0 && x <= mx && y >= 0 && y <= my;
+        rk[j] = ok ? (segbits | ((unsigned long long)x << L.by) | (unsigned long long)y) : kEmptyKey;
+        h[j] = hash_u64(rk[j]) & hmask;
+        v[j] = ok ? slot_load(g.slots, h[j]) : make_ulonglong2(kEmptyKey, 0ull);
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+    {
+        out[j] = make_int2(0, 0);
+        if (rk[j] != kEmptyKey && v[j].x == rk[j])
+            out[j] = make_int2((int)(uint32_t)v[j].y, (int)(uint32_t)(v[j].y >> 32));
+        else if (rk[j] != kEmptyKey && v[j].x != kEmptyKey)
+            out[j] = row_probe_rest(g.slots, hmask, rk[j], h[j]);
+    }
+}
+
+// the cell of p; false when p lies outside the grid's key range
+__device__ __forceinline__ bool grid_cell(const GridDev &g, const KeyLayout &L, float3 o, float3 p, int &cx, int &cy,
+                                          int &cz)
+{
+    cx = cell_of_inv(p.x, o.x, g.cell, g.inv_cell), cy = cell_of_inv(p.y, o.y, g.cell, g.inv_cell),
+    cz = cell_of_inv(p.z, o.z, g.cell, g.inv_cell);
+    const int mx = (1 << L.bx) - 1, my = (1 << L.by) - 1, mz = (1 << L.bz) - 1;
+    return !(cx < -1 || cx > mx + 1 || cy < -1 || cy > my + 1 || cz < -1 || cz > mz + 1);
+}
+
+// the 9 rows around p and its z window; false when p lies outside the grid's key range
 __device__ __forceinline__ bool grid_rows(const GridDev &g, const KeyLayout &L, int seg, float3 o, float3 p,
                                           GridRows &R)
 {
-    const int cx = cell_of(p.x, o.x, g.cell), cy = cell_of(p.y, o.y, g.cell), cz = cell_of(p.z, o.z, g.cell);
-    const int mx = (1 << L.bx) - 1, my = (1 << L.by) - 1, mz = (1 << L.bz) - 1;
-    if (cx < -1 || cx > mx + 1 || cy < -1 || cy > my + 1 || cz < -1 || cz > mz + 1)
+    int cx, cy, cz;
+    if (!grid_cell(g, L, o, p, cx, cy, cz))
         return false;
-    const unsigned long long segbits = (unsigned long long)seg << (L.bx + L.by);
-    unsigned long long rk[9];
-    uint32_t h[9];
-    ulonglong2 v[9];
-    const uint32_t hmask = g.hmask;
-#pragma unroll
-    for (int k = 0; k < 9; ++k)
-    {
-        const int x = cx + k / 3 - 1, y = cy + k % 3 - 1;
-        const bool ok = x >= 0 && x <= mx && y >= 0 && y <= my;
-        rk[k] = ok ? (segbits | ((unsigned long long)x << L.by) | (unsigned long long)y) : kEmptyKey;
-        h[k] = hash_u64(rk[k]) & hmask;
-        v[k] = ok ? slot_load(g.slots, h[k]) : make_ulonglong2(kEmptyKey, 0ull);
-    }
-#pragma unroll
-    for (int k = 0; k < 9; ++k)
-    {
-        if (rk[k] != kEmptyKey && v[k].x == rk[k])
-            R.r[k] = make_int2((int)(uint32_t)v[k].y, (int)(uint32_t)(v[k].y >> 32));
-        else if (rk[k] != kEmptyKey && v[k].x != kEmptyKey)
-            R.r[k] = row_probe_rest(g.slots, hmask, rk[k], h[k]);
-        else
-            R.r[k] = make_int2(0, 0);
-    }
     R.lo = cz - 1;
     R.hi = cz + 1;
+    load_rows<9>(g, L, seg, R.lo, R.hi, R.r, [&](int k, int &x, int &y) {
+        x = cx + k / 3 - 1, y = cy + k % 3 - 1;
+        return true;
+    });
     return true;
 }
 
@@ -165,49 +211,28 @@ struct CellBox
     int x0, nx, y0, ny, zlo, zhi;
 };
 
-// the rows of a box, split over the 4 lanes of a group as grid_rows_sub does
+// the rows of a box, split over the 4 lanes of a group
 __device__ __forceinline__ void grid_rows_box(const GridDev &g, const KeyLayout &L, int seg, const CellBox &B,
                                               int sub, SubRows &R)
 {
-    const int mx = (1 << L.bx) - 1, my = (1 << L.by) - 1;
-    const unsigned long long segbits = (unsigned long long)seg << (L.bx + L.by);
-    const int nrows = B.nx * B.ny;
-    unsigned long long rk[kSubRows];
-    uint32_t h[kSubRows];
-    ulonglong2 v[kSubRows];
-    const uint32_t hmask = g.hmask;
-#pragma unroll
-    for (int j = 0; j < kSubRows; ++j)
-    {
+    R.lo = B.zlo;
+    R.hi = B.zhi;
+    load_rows<kSubRows>(g, L, seg, B.zlo, B.zhi, R.r, [&](int j, int &x, int &y) {
         const int k = sub + kSub * j;
         // k / ny for k < 9 and ny <= 3 by a multiply: (k * ceil(256 / ny)) >> 8
         const int kx = (k * (B.ny == 1 ? 256 : (B.ny == 2 ? 128 : 86))) >> 8;
-        const int x = B.x0 + kx, y = B.y0 + (k - kx * B.ny);
-        const bool ok = k < nrows && x >= 0 && x <= mx && y >= 0 && y <= my;
-        rk[j] = ok ? (segbits | ((unsigned long long)x << L.by) | (unsigned long long)y) : kEmptyKey;
-        h[j] = hash_u64(rk[j]) & hmask;
-        v[j] = ok ? slot_load(g.slots, h[j]) : make_ulonglong2(kEmptyKey, 0ull);
-    }
-#pragma unroll
-    for (int j = 0; j < kSubRows; ++j)
-    {
-        R.r[j] = make_int2(0, 0);
-        if (rk[j] != kEmptyKey && v[j].x == rk[j])
-            R.r[j] = make_int2((int)(uint32_t)v[j].y, (int)(uint32_t)(v[j].y >> 32));
-        else if (rk[j] != kEmptyKey && v[j].x != kEmptyKey)
-            R.r[j] = row_probe_rest(g.slots, hmask, rk[j], h[j]);
-    }
-    R.lo = B.zlo;
-    R.hi = B.zhi;
+        x = B.x0 + kx, y = B.y0 + (k - kx * B.ny);
+        return k < B.nx * B.ny;
+    });
 }
 
 // the 3 x 3 x 3 cells around p's cell; false when p lies outside the grid's range
 __device__ __forceinline__ bool nn_full_box(const GridDev &g, const KeyLayout &L, float3 o, float3 p, CellBox &B)
 {
-    const int cx = cell_of(p.x, o.x, g.cell), cy = cell_of(p.y, o.y, g.cell), cz = cell_of(p.z, o.z, g.cell);
-    const int mx = (1 << L.bx) - 1, my = (1 << L.by) - 1, mz = (1 << L.bz) - 1;
+    int cx, cy, cz;
+    const bool in = grid_cell(g, L, o, p, cx, cy, cz);
     B = CellBox{cx - 1, 3, cy - 1, 3, cz - 1, cz + 1};
-    return !(cx < -1 || cx > mx + 1 || cy < -1 || cy > my + 1 || cz < -1 || cz > mz + 1);
+    return in;
 }
 
 // cell bounds without a division: the cell that cell_of assigns to any value v'
@@ -405,7 +430,7 @@ __device__ __forceinline__ bool nn_certified(const GridDev &g, float3 o, float3 
         return true;
     }
     // t1 must also be one of the candidates of the 27-cell search around p
-    const int qx = cell_of(q.x, o.x, g.cell), qy = cell_of(q.y, o.y, g.cell), qz = __float_as_int(q.w);
+    const int qx = cell_of_inv(q.x, o.x, g.cell, g.inv_cell), qy = cell_of_inv(q.y, o.y, g.cell, g.inv_cell), qz = __float_as_int(q.w);
     if (qx < B.x0 || qx >= B.x0 + B.nx || qy < B.y0 || qy >= B.y0 + B.ny || qz < B.zlo || qz > B.zhi)
         return false;
     t = t1;

@@ -344,6 +344,9 @@ struct KeyLayout
     int bseg, bx, by, bz; // bits per field; key = seg|cx|cy|cz from MSB to LSB
     int total_bits;
     int morton; // voxel keys only: seg | bit-interleaved (cx, cy, cz), bx = by = bz
+    // grid keys only: the row table is indexed by key >> zs, runs of 2^zs z cells of a row
+    // (direct = 1), or is a hash of whole rows (direct = 0)
+    int direct, zs;
 };
 
 // one open-addressing slot of the row hash: the key and the row's [start, end) in
@@ -369,8 +372,9 @@ struct GridDev
     float *sint;   // intensity in sorted order
     int *scz;      // z cell in sorted order (compact copy for the in-row binary search)
     uint64_t *skey;
-    // row hash: key = (seg, cx, cy) -> [start, end) in one 16-byte slot; at least
-    // twice as many slots as points, so the first probe nearly always decides
+    // the row table (KeyLayout::direct): [start, end) per run of z cells, or a hash
+    // (seg, cx, cy) -> [start, end) in 16-byte slots, at least twice as many as points, so
+    // the first probe nearly always decides.  One memory serves both; empty is all ones.
     RowSlot *slots;
     uint32_t hmask;
     const int32_t *seg_off; // [P + 1] offsets of the segments in the sorted arrays
@@ -393,6 +397,12 @@ __device__ __forceinline__ uint32_t hash_u64(unsigned long long k)
 __device__ __forceinline__ ulonglong2 slot_load(const RowSlot *slots, uint32_t h)
 {
     return __ldg(reinterpret_cast<const ulonglong2 *>(slots + h));
+}
+
+// entry i of a direct row table; {-1, -1} when it is empty
+__device__ __forceinline__ int2 run_load(const RowSlot *slots, uint32_t i)
+{
+    return __ldg(reinterpret_cast<const int2 *>(slots) + i);
 }
 
 // continue a linear probe after the first slot missed

@@ -7,10 +7,10 @@
 // looks at its own cell and the neighbour on the side it is nearer to (the cell's
 // lower corner computed fused as cell * c + origin, as the reference does), so
 // 2 x 2 x 2 cells; it counts the points with d^2 < r^2, itself included, and
-// survives with more than min_neighbors.  The reference stops counting once the
-// threshold is passed, which does not change the outcome.  Survivors keep input
-// order: flags, exclusive scan, scatter.  Here the grid is the row-hashed one
-// (4 row probes, a 2-cell z window per row).
+// survives with more than min_neighbors.  Counting stops once the threshold is passed, as
+// in the reference.  Survivors keep input
+// order: flags, exclusive scan, scatter.  Here the grid is the one with the row table
+// (4 row lookups, a 2-cell z window per row).
 #include "grid_query.cuh"
 #include "stages.cuh"
 
@@ -33,57 +33,60 @@ __device__ __forceinline__ Side near_side(float p, float o, float cell, int c, f
     return Side{off >= radius ? 0 : -1, off < radius ? 1 : 2};
 }
 
-__global__ void k_ror_flags(const float4 *__restrict__ pos, const int32_t *d_n, GridDev g, float radius, int min_nn,
-                            int32_t *keep)
+// Threads take the points in grid order: a warp's points share their rows, and its lanes'
+// counts are alike (in the cloud's order the 180k points of a frame took 44 us, bound by
+// uncoalesced reads; now 29, a chain of dependent loads: the threads of 700 blocks are all
+// resident and 6 blocks' worth of registers per SM keep them so).
+__global__ void __launch_bounds__(kBlock, 6) k_ror_flags(GridDev g, float radius, int min_nn, int32_t *keep)
 {
-    const int n = *d_n;
+    const int n = *g.d_n;
     const KeyLayout L = *g.layout;
     const float3 o = g.gmin[0];
     const float cell = g.cell;
     const float rr = __fmul_rn(radius, radius);
-    const int mx = (1 << L.bx) - 1, my = (1 << L.by) - 1;
-    const uint32_t hmask = g.hmask;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
     {
-        const float4 p = pos[i];
-        const int cx = cell_of(p.x, o.x, cell), cy = cell_of(p.y, o.y, cell), cz = cell_of(p.z, o.z, cell);
+        const float4 p = __ldg(&g.spos[s]);
+        const int cx = cell_of_inv(p.x, o.x, cell, g.inv_cell), cy = cell_of_inv(p.y, o.y, cell, g.inv_cell),
+                  cz = cell_of_inv(p.z, o.z, cell, g.inv_cell);
         const Side sx = near_side(p.x, o.x, cell, cx, radius);
         const Side sy = near_side(p.y, o.y, cell, cy, radius);
         const Side sz = near_side(p.z, o.z, cell, cz, radius);
         const int zlo = cz + sz.b, zhi = cz + sz.e - 1;
+        // the two cells per axis are the point's own and the one on its nearer side; its own
+        // row comes first (a NaN has no side, and no neighbours either)
+        const int ox = sx.b == 0 ? 1 : -1, oy = sy.b == 0 ? 1 : -1;
+        int2 rows[4];
+        load_rows<4>(g, L, 0, zlo, zhi, rows, [&](int j, int &x, int &y) {
+            x = cx + (j & 1 ? ox : 0), y = cy + (j & 2 ? oy : 0);
+            return true;
+        });
         int count = 0;
-        for (int dx = sx.b; dx < sx.e; ++dx)
-            for (int dy = sy.b; dy < sy.e; ++dy)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            if (count > min_nn || rows[j].x >= rows[j].y || !GCA_INDEX_OK(rows[j].x, n, g.err) || !GCA_INDEX_OK(rows[j].y - 1, n, g.err))
+                continue;
+            // a row holds few candidates (two cells of the window), so it is entered at the
+            // first of them and read one by one
+            int a = rows[j].x, b = rows[j].y;
+            while (a < b)
             {
-                const int x = cx + dx, y = cy + dy;
-                if (x < 0 || x > mx || y < 0 || y > my)
-                    continue;
-                const unsigned long long rk = ((unsigned long long)x << L.by) | (unsigned long long)y;
-                const uint32_t h = hash_u64(rk) & hmask;
-                const ulonglong2 v = slot_load(g.slots, h);
-                int2 r = make_int2(0, 0);
-                if (v.x == rk)
-                    r = make_int2((int)(uint32_t)v.y, (int)(uint32_t)(v.y >> 32));
-                else if (v.x != kEmptyKey)
-                    r = row_probe_rest(g.slots, hmask, rk, h);
-                int a = r.x, b = r.y;
-                while (a < b) // first point of the row with z cell >= zlo
-                {
-                    const int m = (a + b) >> 1;
-                    if (__ldg(&g.scz[m]) < zlo)
-                        a = m + 1;
-                    else
-                        b = m;
-                }
-                for (int t = a; t < r.y; ++t)
-                {
-                    const float4 q = __ldg(&g.spos[t]);
-                    if (__float_as_int(q.w) > zhi)
-                        break;
-                    count += dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z) < rr;
-                }
+                const int m = (a + b) >> 1;
+                if (__ldg(&g.scz[m]) < zlo)
+                    a = m + 1;
+                else
+                    b = m;
             }
-        keep[i] = count > min_nn ? 1 : 0;
+            for (int t = a; t < rows[j].y && count <= min_nn; ++t) // more do not change the outcome
+            {
+                const float4 q = __ldg(&g.spos[t]);
+                if (__float_as_int(q.w) > zhi)
+                    break;
+                count += dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z) < rr;
+            }
+        }
+        keep[g.sidx[s]] = count > min_nn ? 1 : 0;
     }
 }
 
@@ -179,7 +182,7 @@ int gca3d_radius_outlier_removal(gca3d_context *ctx, gca3d_cloud *in, float radi
     if (!keep || !at)
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "radius_outlier_removal: scratch");
     const int gs = std::min(grid_for(in->capacity), ctx->num_sms * 16);
-    k_ror_flags<<<gs, kBlock, 0, ctx->stream>>>(in->pos, in->d_count, g.dev, radius, min_neighbors, keep);
+    k_ror_flags<<<gs, kBlock, 0, ctx->stream>>>(g.dev, radius, min_neighbors, keep);
     GCA_CHECK_LAUNCH(ctx);
     if ((st = exclusive_scan(ctx, keep, at, in->d_count, in->capacity, out->d_count)))
         return st;

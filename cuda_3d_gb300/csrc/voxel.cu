@@ -176,7 +176,7 @@ struct VoxelMaker
         L.by = max(1, bitlen_u32(cells[1]));
         L.bz = max(1, bitlen_u32(cells[2]));
         L.total_bits = L.bseg + L.bx + L.by + L.bz;
-        L.morton = 0;
+        L.morton = L.direct = L.zs = 0;
         const int b = max(L.bx, max(L.by, L.bz));
         if (morton && L.bseg + 3 * b + sub_bits <= 64)
         {

@@ -593,6 +593,27 @@ def test_radius_outlier_removal_full_size_vs_oracle(ctx, orc, room, radius, min_
     np.testing.assert_array_equal(d["rgb"], oc)
 
 
+@pytest.mark.parametrize("extent", [0.3, 3.0, 500.0])
+@pytest.mark.parametrize("min_nn", [0, 3, 12])
+def test_radius_outlier_removal_row_tables(ctx, extent, min_nn):
+    """the direct row table with short and long runs, and the row hash (a set too wide for
+    the table), against all distances in FP32"""
+    rng = np.random.default_rng(int(extent))
+    r, n = 0.01, 4000
+    c = (rng.random((250, 3)) * extent).astype(np.float32)
+    xyz = (c[rng.integers(0, len(c), n)] + rng.normal(size=(n, 3)) * r * 0.6).astype(np.float32)
+    rgb = rng.random((n, 3)).astype(np.float32)
+    d2 = np.zeros((n, n), np.float32)
+    for k in range(3):
+        d = xyz[:, k, None] - xyz[None, :, k]
+        d2 += d * d
+    keep = (d2 < np.float32(r) * np.float32(r)).sum(1) > min_nn
+    assert keep.any() and (min_nn == 0 or not keep.all())
+    d = _ror(ctx, xyz, rgb, r, min_nn)
+    np.testing.assert_array_equal(d["xyz"], xyz[keep])
+    np.testing.assert_array_equal(d["rgb"], rgb[keep])
+
+
 def test_radius_outlier_removal_invalid(ctx, N, golden):
     c = ctx.cloud_from(golden["cloud_xyz"][:100], golden["cloud_rgb"][:100])
     small = ctx.cloud(10)
