@@ -211,9 +211,11 @@ struct CellBox
     int x0, nx, y0, ny, zlo, zhi;
 };
 
-// the rows of a box, split over the 4 lanes of a group
+// the rows of a box, split over the 4 lanes of a group; with Skip the row (sx, sy), which
+// has been searched, is left out
+template <bool Skip>
 __device__ __forceinline__ void grid_rows_box(const GridDev &g, const KeyLayout &L, int seg, const CellBox &B,
-                                              int sub, SubRows &R)
+                                              int sub, SubRows &R, int sx = 0, int sy = 0)
 {
     R.lo = B.zlo;
     R.hi = B.zhi;
@@ -222,7 +224,7 @@ __device__ __forceinline__ void grid_rows_box(const GridDev &g, const KeyLayout 
         // k / ny for k < 9 and ny <= 3 by a multiply: (k * ceil(256 / ny)) >> 8
         const int kx = (k * (B.ny == 1 ? 256 : (B.ny == 2 ? 128 : 86))) >> 8;
         x = B.x0 + kx, y = B.y0 + (k - kx * B.ny);
-        return k < B.nx * B.ny;
+        return k < B.nx * B.ny && !(Skip && x == sx && y == sy);
     });
 }
 
@@ -270,28 +272,9 @@ __device__ __forceinline__ void nn_shrink_box(const GridDev &g, float3 o, float3
     B.y0 = y0, B.ny = y1 - y0 + 1;
 }
 
-// the nearest grid point with d^2 < rr inside box B over the whole 4-lane group;
-// every lane of the group returns the same answer (ties on d^2 go to the smaller
-// original index).  All 32 lanes of the warp must call it (invalid lanes pass
-// valid = false).
-__device__ __forceinline__ NNBest nn_search_box(const GridDev &g, const KeyLayout &L, int seg, const CellBox &B,
-                                                float3 p, float rr, bool valid)
+// the group's nearest of its lanes' candidates (ties on d^2 go to the smaller original index)
+__device__ __forceinline__ NNBest nn_group_best(const GridDev &g, NNBest b)
 {
-    const int sub = threadIdx.x & (kSub - 1);
-    NNBest b{rr, -1};
-    SubRows R;
-    if (valid)
-    {
-        grid_rows_box(g, L, seg, B, sub, R);
-        grid_scan_sub(g, R, [&](int t, float4 q) {
-            const float d2 = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
-            if (d2 < b.d2 || (d2 == b.d2 && b.t >= 0 && __ldg(&g.sidx[t]) < __ldg(&g.sidx[b.t])))
-            {
-                b.d2 = d2;
-                b.t = t;
-            }
-        });
-    }
 #pragma unroll
     for (int off = 1; off < kSub; off <<= 1)
     {
@@ -304,6 +287,41 @@ __device__ __forceinline__ NNBest nn_search_box(const GridDev &g, const KeyLayou
         }
     }
     return b;
+}
+
+__device__ __forceinline__ void nn_take(const GridDev &g, NNBest &b, int t, float d2)
+{
+    if (d2 < b.d2 || (d2 == b.d2 && b.t >= 0 && __ldg(&g.sidx[t]) < __ldg(&g.sidx[b.t])))
+    {
+        b.d2 = d2;
+        b.t = t;
+    }
+}
+
+// the points of row (x, y) with z cell in [zlo, zhi], dealt out to the 4 lanes of a group one
+// by one.  f(t, spos[t]).
+template <class F>
+__device__ __forceinline__ void own_row_scan(const GridDev &g, const KeyLayout &L, int seg, int x, int y, int zlo,
+                                             int zhi, int sub, F &&f)
+{
+    int2 r;
+    load_rows<1>(g, L, seg, zlo, zhi, &r, [&](int, int &rx, int &ry) {
+        rx = x, ry = y;
+        return true;
+    });
+    if (r.x >= r.y || !GCA_INDEX_OK(r.x, *g.d_n, g.err) || !GCA_INDEX_OK(r.y - 1, *g.d_n, g.err))
+        return;
+    if (r.y - r.x > 8)
+        r.x = row_seek_z(g.scz, r.x, r.y, zlo);
+    for (int t = r.x + sub; t < r.y; t += kSub)
+    {
+        const float4 q = __ldg(&g.spos[t]);
+        const int qz = __float_as_int(q.w);
+        if (qz > zhi)
+            break;
+        if (qz >= zlo)
+            f(t, q);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -346,30 +364,21 @@ __device__ __forceinline__ float box_cover(const GridDev &g, float3 o, float3 p,
     return r > 0.0f ? r * 0.99999f : 0.0f;
 }
 
-// the nearest grid point inside box B at any distance (ties to the smaller original
-// index, as nn_search_box) and the second-smallest squared distance, over the
-// 4-lane group; all 32 lanes of the warp call it
-__device__ __forceinline__ NNBest2 nn_search_box2(const GridDev &g, const KeyLayout &L, int seg, const CellBox &B,
-                                                  float3 p, bool valid)
+__device__ __forceinline__ void nn_take2(const GridDev &g, NNBest2 &b, int t, float d2)
 {
-    const int sub = threadIdx.x & (kSub - 1);
-    NNBest2 b{INFINITY, -1, INFINITY};
-    SubRows R;
-    if (valid)
+    if (b.t < 0 || d2 < b.d2 || (d2 == b.d2 && __ldg(&g.sidx[t]) < __ldg(&g.sidx[b.t])))
     {
-        grid_rows_box(g, L, seg, B, sub, R);
-        grid_scan_sub(g, R, [&](int t, float4 q) {
-            const float d2 = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
-            if (b.t < 0 || d2 < b.d2 || (d2 == b.d2 && __ldg(&g.sidx[t]) < __ldg(&g.sidx[b.t])))
-            {
-                b.s2 = b.d2;
-                b.d2 = d2;
-                b.t = t;
-            }
-            else
-                b.s2 = fminf(b.s2, d2);
-        });
+        b.s2 = b.d2;
+        b.d2 = d2;
+        b.t = t;
     }
+    else
+        b.s2 = fminf(b.s2, d2);
+}
+
+// the two nearest over the 4-lane group (its lanes' candidates are disjoint)
+__device__ __forceinline__ NNBest2 nn_group_best2(const GridDev &g, NNBest2 b)
+{
 #pragma unroll
     for (int off = 1; off < kSub; off <<= 1)
     {
@@ -386,6 +395,39 @@ __device__ __forceinline__ NNBest2 nn_search_box2(const GridDev &g, const KeyLay
             b.s2 = fminf(b.s2, od2);
     }
     return b;
+}
+
+// the nearest grid point inside box B at any distance (ties to the smaller original
+// index) and the second-smallest squared distance, over the 4-lane group; all 32 lanes of
+// the warp call it.  Cold (B is the 27 cells around p): p's own row is searched first, and
+// the box then shrunk to the ball through that row's second-nearest point, which holds the
+// two nearest of all and their ties; B returns the shrunk box.
+template <bool Cold>
+__device__ __forceinline__ NNBest2 nn_search_box2(const GridDev &g, const KeyLayout &L, int seg, float3 o, CellBox &B,
+                                                  float3 p, bool valid)
+{
+    const int sub = threadIdx.x & (kSub - 1);
+    NNBest2 b{INFINITY, -1, INFINITY};
+    const int sx = B.x0 + 1, sy = B.y0 + 1;
+    if (Cold)
+    {
+        if (valid)
+            own_row_scan(g, L, seg, sx, sy, B.zlo, B.zhi, sub, [&](int t, float4 q) {
+                nn_take2(g, b, t, dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z));
+            });
+        b = nn_group_best2(g, b);
+        if (b.s2 < INFINITY)
+            nn_shrink_box(g, o, p, sqrtf(b.s2), B);
+        if (sub != 0) // one lane carries the row's result into the group's
+            b = NNBest2{INFINITY, -1, INFINITY};
+    }
+    if (valid)
+    {
+        SubRows R;
+        grid_rows_box<Cold>(g, L, seg, B, sub, R, sx, sy);
+        grid_scan_sub(g, R, [&](int t, float4 q) { nn_take2(g, b, t, dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z)); });
+    }
+    return nn_group_best2(g, b);
 }
 
 // G of a search at p over box B (see NNCerts)
@@ -437,13 +479,32 @@ __device__ __forceinline__ bool nn_certified(const GridDev &g, float3 o, float3 
     return true;
 }
 
-// the nearest grid point with d^2 < rr in the 27 cells around p (4-lane group)
+// the nearest grid point with d^2 < rr in the 27 cells around p (4-lane group, ties on d^2 to
+// the smaller original index; every lane returns it).  p's own row first: the ball through
+// its nearest point holds the answer and its ties, and with a cell of the search radius that
+// ball rarely leaves the middle cells, so most of the 27 are never read.
 __device__ __forceinline__ NNBest nn_search_sub(const GridDev &g, const KeyLayout &L, int seg, float3 o, float3 p,
                                                 float rr, bool valid)
 {
+    const int sub = threadIdx.x & (kSub - 1);
     CellBox B;
-    const bool in = nn_full_box(g, L, o, p, B);
-    return nn_search_box(g, L, seg, B, p, rr, valid && in);
+    valid = nn_full_box(g, L, o, p, B) && valid;
+    const int sx = B.x0 + 1, sy = B.y0 + 1;
+    NNBest b{rr, -1};
+    if (valid)
+        own_row_scan(g, L, seg, sx, sy, B.zlo, B.zhi, sub, [&](int t, float4 q) {
+            nn_take(g, b, t, dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z));
+        });
+    b = nn_group_best(g, b);
+    if (b.t >= 0)
+        nn_shrink_box(g, o, p, sqrtf(b.d2), B);
+    if (valid)
+    {
+        SubRows R;
+        grid_rows_box<true>(g, L, seg, B, sub, R, sx, sy);
+        grid_scan_sub(g, R, [&](int t, float4 q) { nn_take(g, b, t, dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z)); });
+    }
+    return nn_group_best(g, b);
 }
 
 } // namespace gca3d

@@ -378,6 +378,10 @@ __device__ __forceinline__ BlockPair item_pair(int w, const int32_t *src_off, co
 // list of the others: the search, shrunk to the cells that overlap the ball
 // through the last nearest point when that one is within max_corr (the ball holds
 // the nearest point and all its ties); it renews the point's certificate.
+// Cold: the first search of a scale, without certificates or last nearest points, in a
+// kernel of its own, so that the second row loop of its search costs the warm ones no
+// registers.
+template <bool Cold>
 __global__ void __launch_bounds__(kIcpThreads, 5) k_icp_nn(const float4 *__restrict__ src_pos, const int32_t *src_off,
                                                         GridDev g, const PairState *st, const int *bmap, int P,
                                                         float max_corr, int2 *corr, NNCerts cert, int32_t *nn_out,
@@ -416,7 +420,7 @@ __global__ void __launch_bounds__(kIcpThreads, 5) k_icp_nn(const float4 *__restr
     __syncthreads();
     const float3 o = g.gmin[b.pair];
     const int tbase = g.seg_off[b.pair];
-    const bool warm = st[b.pair].nn_warm;
+    const bool warm = !Cold && st[b.pair].nn_warm;
     for (int base = b.start; base < b.end; base += kIcpThreads)
     {
         const int i = base + (int)threadIdx.x;
@@ -480,11 +484,14 @@ __global__ void __launch_bounds__(kIcpThreads, 5) k_icp_nn(const float4 *__restr
         const bool valid = k < n;
         const int kk = valid ? k : 0;
         NNBest2 best;
+        CellBox searched;
         {
             const int4 bx = s_box[kk];
             const float4 p4 = s_p[kk];
-            const CellBox B{bx.x, bx.w & 0xff, bx.y, (bx.w >> 8) & 0xff, bx.z, bx.z + (bx.w >> 16) - 1};
-            best = nn_search_box2(g, L, b.pair, B, make_float3(p4.x, p4.y, p4.z), valid);
+            CellBox B{bx.x, bx.w & 0xff, bx.y, (bx.w >> 8) & 0xff, bx.z, bx.z + (bx.w >> 16) - 1};
+            best = nn_search_box2<Cold>(g, L, b.pair, o, B, make_float3(p4.x, p4.y, p4.z), valid);
+            if (Cold)
+                searched = B;
         }
         if (valid && (threadIdx.x & (kSub - 1)) == 0)
         {
@@ -495,7 +502,8 @@ __global__ void __launch_bounds__(kIcpThreads, 5) k_icp_nn(const float4 *__restr
             const volatile float *vp = reinterpret_cast<const volatile float *>(&s_p[kk]);
             const int i = vl[kk];
             const int bw = vb[3];
-            const CellBox B{vb[0], bw & 0xff, vb[1], (bw >> 8) & 0xff, vb[2], vb[2] + (bw >> 16) - 1};
+            const CellBox B = Cold ? searched
+                                   : CellBox{vb[0], bw & 0xff, vb[1], (bw >> 8) & 0xff, vb[2], vb[2] + (bw >> 16) - 1};
             const float3 p = make_float3(vp[0], vp[1], vp[2]);
             const float3 og = g.gmin[b.pair];
             const bool hit = best.t >= 0 && best.d2 < rr;
@@ -857,15 +865,21 @@ int icp_state_init(gca3d_context *ctx, PairState *st, int P, const double *d_Tin
 
 int icp_search(gca3d_context *ctx, const Batch &src, const Grid &g, PairState *st, int *bmap_nn, int max_blocks_nn,
                int2 *corr, const NNCerts &cert, const IcpScale &prm, int32_t *nn_out, const IcpLoop *guard,
-               const IcpShape &shape)
+               const IcpShape &shape, bool cold)
 {
     // work-item loop: enough blocks to fill the SMs a few times over, never more than
     // the items the capacity can produce
     const int grid_nn = std::max(std::min(max_blocks_nn, ctx->num_sms * shape.nn_bps), 1);
     GCA_PROF_BEGIN(ctx, kKidIcpIter);
-    k_icp_nn<<<grid_nn, kIcpThreads, 0, ctx->stream>>>(src.pos, src.seg_off, g.dev, st, bmap_nn, src.P, prm.max_corr,
-                                                       corr, cert, nn_out, shape.nn_chunk, bmap_nn + src.P + 1,
-                                                       guard ? guard->iter : nullptr, guard ? guard->max_iter : 0);
+    auto search = [&](auto kernel) {
+        kernel<<<grid_nn, kIcpThreads, 0, ctx->stream>>>(src.pos, src.seg_off, g.dev, st, bmap_nn, src.P, prm.max_corr,
+                                                         corr, cert, nn_out, shape.nn_chunk, bmap_nn + src.P + 1,
+                                                         guard ? guard->iter : nullptr, guard ? guard->max_iter : 0);
+    };
+    if (cold)
+        search(k_icp_nn<true>);
+    else
+        search(k_icp_nn<false>);
     GCA_CHECK_LAUNCH(ctx);
     GCA_PROF_END(ctx, kKidIcpIter);
     return GCA3D_OK;
@@ -918,11 +932,11 @@ int icp_update(gca3d_context *ctx, const Batch &src, const Grid &g, const float4
 int icp_iteration(gca3d_context *ctx, const Batch &src, const Grid &g, const float4 *attr0, const float4 *attr1,
                   PairState *st, int *bmap, int max_blocks, int *bmap_nn, int max_blocks_nn, double *partials,
                   int2 *corr, const NNCerts &cert, const IcpScale &prm, bool compensated, int32_t *nn_out,
-                  const IcpLoop &loop, const IcpShape &shape)
+                  const IcpLoop &loop, const IcpShape &shape, bool cold)
 {
     if (!loop.ticket)
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: iteration without a finalize ticket");
-    int st_ = icp_search(ctx, src, g, st, bmap_nn, max_blocks_nn, corr, cert, prm, nn_out, nullptr, shape);
+    int st_ = icp_search(ctx, src, g, st, bmap_nn, max_blocks_nn, corr, cert, prm, nn_out, nullptr, shape, cold);
     if (!st_)
         st_ = icp_update(ctx, src, g, attr0, attr1, st, bmap, max_blocks, bmap_nn, partials, corr, prm, compensated,
                          loop, shape);

@@ -94,13 +94,13 @@ int icp_setup(gca3d_context *ctx, PairState *st, int P, const int32_t *src_off, 
 int icp_iteration(gca3d_context *ctx, const Batch &src, const Grid &g, const float4 *attr0, const float4 *attr1,
                   PairState *st, int *bmap, int max_blocks, int *bmap_nn, int max_blocks_nn, double *partials,
                   int2 *corr, const NNCerts &cert, const IcpScale &prm, bool compensated, int32_t *nn_out,
-                  const IcpLoop &loop, const IcpShape &shape);
-// the two halves of an iteration: the correspondence search (skipped on the device when
-// guard is given and its iteration count has reached the budget), and the accumulation
+                  const IcpLoop &loop, const IcpShape &shape, bool cold);
+// the two halves of an iteration: the correspondence search (cold: the first of a scale;
+// skipped on the device when guard is given and its iteration count has reached the budget), and the accumulation
 // with the solve and pose update
 int icp_search(gca3d_context *ctx, const Batch &src, const Grid &g, PairState *st, int *bmap_nn, int max_blocks_nn,
                int2 *corr, const NNCerts &cert, const IcpScale &prm, int32_t *nn_out, const IcpLoop *guard,
-               const IcpShape &shape);
+               const IcpShape &shape, bool cold);
 int icp_update(gca3d_context *ctx, const Batch &src, const Grid &g, const float4 *attr0, const float4 *attr1,
                PairState *st, int *bmap, int max_blocks, int *bmap_nn, double *partials, const int2 *corr,
                const IcpScale &prm, bool compensated, const IcpLoop &loop, const IcpShape &shape);

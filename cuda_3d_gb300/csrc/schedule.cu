@@ -390,7 +390,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
             loop.ticket = reinterpret_cast<unsigned *>(iter + 1);
             if (S.max_iter > 0 &&
                 (st = icp_search(ctx, bs, gicp, pl->d_state, bmap_nn, pl->max_blocks_nn, corr, cert, prm, nullptr,
-                                 nullptr, shape)))
+                                 nullptr, shape, true)))
                 return st;
             if (!serial)
                 GCA_CUDA(ctx, cudaStreamWaitEvent(main_stream, pl->ev_scale[si], 0));
@@ -426,7 +426,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
                                 corr, prm, p.compensated != 0, loop, shape);
                 if (!st)
                     st = icp_search(ctx, bs, gicp, pl->d_state, bmap_nn, pl->max_blocks_nn, corr, cert, prm,
-                                    nullptr, &loop, shape);
+                                    nullptr, &loop, shape, false);
                 pl->kernels_static -= ctx->launches - l0; // counted per iteration instead
                 ctx->stream = main_stream;
                 cudaGraph_t captured = nullptr;
@@ -459,7 +459,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
                 }
                 if (it + 1 < S.max_iter &&
                     (st = icp_search(ctx, bs, gicp, pl->d_state, bmap_nn, pl->max_blocks_nn, corr, cert, prm,
-                                     nullptr, nullptr, shape)))
+                                     nullptr, nullptr, shape, false)))
                     return st;
             }
         }
