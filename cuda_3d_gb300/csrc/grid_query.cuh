@@ -99,12 +99,12 @@ __device__ __forceinline__ bool grid_rows(const GridDev &g, const KeyLayout &L, 
     return true;
 }
 
-// a position in [t, e] at most 8 before the first one whose z cell is >= lo (the
+// a position in [t, e] at most 2 before the first one whose z cell is >= lo (the
 // row is sorted by z cell): a 4-way search, its three probes loaded together
 __device__ __forceinline__ int row_seek_z(const int *scz, int t, int e, int lo)
 {
     int a = t, n = e - t; // the first z cell >= lo is in [a, a + n]
-    while (n > 8)
+    while (n > 2)
     {
         const int s = n >> 2;
         const int c1 = __ldg(&scz[a + s]), c2 = __ldg(&scz[a + 2 * s]), c3 = __ldg(&scz[a + 3 * s]);
@@ -139,7 +139,7 @@ __device__ __forceinline__ void row_scan(const GridDev &g, int t, int e, int lo,
         return;
     if (!GCA_INDEX_OK(t, *g.d_n, g.err) || !GCA_INDEX_OK(e - 1, *g.d_n, g.err))
         return;
-    if (e - t > 8)
+    if (e - t > 4)
         t = row_seek_z(g.scz, t, e, lo);
     for (bool more = true; more && t < e; t += Batch)
     {
@@ -311,7 +311,7 @@ __device__ __forceinline__ void own_row_scan(const GridDev &g, const KeyLayout &
     });
     if (r.x >= r.y || !GCA_INDEX_OK(r.x, *g.d_n, g.err) || !GCA_INDEX_OK(r.y - 1, *g.d_n, g.err))
         return;
-    if (r.y - r.x > 8)
+    if (r.y - r.x > 4)
         r.x = row_seek_z(g.scz, r.x, r.y, zlo);
     for (int t = r.x + sub; t < r.y; t += kSub)
     {

@@ -185,22 +185,6 @@ __device__ __forceinline__ void block_reduce_store(Acc<Comp> &acc, double *part)
     }
 }
 
-__device__ __forceinline__ int find_pair(const int *bmap, int P, int b)
-{
-    if (b >= bmap[P])
-        return -1;
-    int lo = 0, hi = P - 1;
-    while (lo < hi)
-    {
-        int mid = (lo + hi + 1) >> 1;
-        if (bmap[mid] <= b)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
 // exclusive prefix over the block's kIcpThreads threads of two per-thread counts: each
 // thread gets its own prefixes back in a and b, and every thread the two totals
 __device__ __forceinline__ void block_prefix2(int &a, int &b, int &ta, int &tb)
@@ -329,44 +313,53 @@ __global__ void k_state_init(PairState *st, int P, const double *T_init)
         return;
     for (int k = 0; k < 16; ++k)
         st[p].T[k] = T_init ? T_init[16 * p + k] : (k % 5 == 0 ? 1.0 : 0.0);
+    for (int k = 0; k < 12; ++k)
+        st[p].Tf[k] = (float)st[p].T[k];
     st[p].iters = 0;
     st[p].status = 0;
     st[p].rmse_ref = st[p].fitness = st[p].inlier_rmse = 0.0;
 }
 
-// work item w -> (pair, chunk) of the pair's source points; the pair's pose as
-// FP32 in shared memory.  Every thread of the block must call it (it synchronises).
-// Blocks take items in a strided order, so blocks running at the same time work
-// on neighbouring points and share their target rows in L2.
+// work item w -> (pair, chunk) of the pair's source points; the pair's pose as FP32 in shared
+// memory.  Warp 0 does it, all lanes at once (its loads are the item's latency: one thread
+// searching the map and converting the pose held a 256-point item for about 2 us); the block
+// meets before it, so that the previous item's readers are done, and after it.
 struct BlockPair
 {
     int pair, start, end;
 };
 
-__device__ __forceinline__ BlockPair item_pair(int w, const int32_t *src_off, const PairState *st, const int *bmap,
-                                               int P, int chunk, float *s_T, int *s_pair)
+__device__ __forceinline__ void item_setup(int w, int items, const int32_t *src_off, const PairState *st,
+                                           const int *bmap, int P, int chunk, float *s_T, BlockPair *s_item)
 {
-    __syncthreads(); // the previous item's readers of s_T / s_pair are done
-    if (threadIdx.x == 0)
+    const int lane = threadIdx.x & 31;
+    int p = -1;
+    if (w < items)
     {
-        int p = find_pair(bmap, P, w);
+        // the last pair whose first item is <= w (pairs without items share theirs with the next)
+        for (int base = 0; base < P; base += 32)
+        {
+            const bool le = base + lane < P && bmap[base + lane] <= w;
+            const int c = __popc(__ballot_sync(0xffffffffu, le));
+            p += c;
+            if (c < 32)
+                break;
+        }
         if (p >= 0 && !st[p].active)
             p = -1;
-        *s_pair = p;
-        if (p >= 0)
-            for (int k = 0; k < 12; ++k)
-                s_T[k] = (float)st[p].T[k];
     }
-    __syncthreads();
-    BlockPair b;
-    b.pair = *s_pair;
-    b.start = b.end = 0;
-    if (b.pair >= 0)
+    if (p >= 0 && lane < 12)
+        s_T[lane] = st[p].Tf[lane];
+    if (lane == 0)
     {
-        b.start = src_off[b.pair] + (w - bmap[b.pair]) * chunk;
-        b.end = min(b.start + chunk, src_off[b.pair + 1]);
+        BlockPair b{p, 0, 0};
+        if (p >= 0)
+        {
+            b.start = src_off[p] + (w - bmap[p]) * chunk;
+            b.end = min(b.start + chunk, src_off[p + 1]);
+        }
+        *s_item = b;
     }
-    return b;
 }
 
 // step 1 of an iteration: the correspondence of every active source point
@@ -390,7 +383,8 @@ __global__ void __launch_bounds__(kIcpThreads, 5) k_icp_nn(const float4 *__restr
     // a search queued behind the iteration that spent the scale's budget has nothing to do
     if (stop_iter && *stop_iter >= stop_at)
         return;
-    __shared__ int s_pair, s_w;
+    __shared__ BlockPair s_item;
+    __shared__ int s_w;
     __shared__ float s_T[12];
     __shared__ int s_list[kNNChunkMax];
     __shared__ int4 s_box[kNNChunkMax]; // x0, y0, zlo, nx | ny << 8 | nz << 16 of the search box
@@ -400,24 +394,31 @@ __global__ void __launch_bounds__(kIcpThreads, 5) k_icp_nn(const float4 *__restr
     const float rr = __fmul_rn(max_corr, max_corr);
     const int items = bmap[P];
     const int lane = threadIdx.x & 31;
-    for (int first = 1;; first = 0)
-    {
     // a block's first work item is its own index, the later ones come from the
-    // iteration's queue: blocks that draw quick items (mostly certified points) take
-    // more of them
+    // iteration's queue (drawn while the item before is searched): blocks that draw quick
+    // items (mostly certified points) take more of them
+    int next = (int)blockIdx.x;
+    for (;;)
+    {
     __syncthreads();
-    if (threadIdx.x == 0)
-        s_w = first ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(queue, 1);
+    if (threadIdx.x < 32)
+    {
+        const int w = __shfl_sync(0xffffffffu, next, 0);
+        item_setup(w, items, src_off, st, bmap, P, nn_chunk, s_T, &s_item);
+        if (lane == 0)
+        {
+            s_w = w;
+            s_cnt = 0;
+        }
+    }
     __syncthreads();
-    const int w = s_w;
-    if (w >= items)
+    if (s_w >= items)
         break;
-    const BlockPair b = item_pair(w, src_off, st, bmap, P, nn_chunk, s_T, &s_pair);
+    if (threadIdx.x == 0)
+        next = (int)gridDim.x + atomicAdd(queue, 1);
+    const BlockPair b = s_item;
     if (b.pair < 0)
         continue;
-    if (threadIdx.x == 0)
-        s_cnt = 0;
-    __syncthreads();
     const float3 o = g.gmin[b.pair];
     const int tbase = g.seg_off[b.pair];
     const bool warm = !Cold && st[b.pair].nn_warm;
@@ -609,6 +610,8 @@ __device__ __forceinline__ void finalize_pair_body(PairState *st, int P, int pai
         __syncwarp();
         if (lane < 16)
             Ps.T[lane] = v;
+        if (lane < 12)
+            Ps.Tf[lane] = (float)v;
         if (lane == 0)
         {
             if (s_S[28] == 0.0)
@@ -727,7 +730,7 @@ __global__ void __launch_bounds__(kIcpThreads, 3) k_icp_accum(const float4 *__re
                                                            float slg, float slc, const int32_t *d_nt, int *err,
                                                            IcpScale prm, IcpLoop loop)
 {
-    __shared__ int s_pair;
+    __shared__ BlockPair s_item;
     __shared__ float s_T[12];
     __shared__ int s_fin;
     const int items = bmap[P];
@@ -741,7 +744,11 @@ __global__ void __launch_bounds__(kIcpThreads, 3) k_icp_accum(const float4 *__re
     }
     for (int w = blockIdx.x; w < items; w += gridDim.x)
     {
-    const BlockPair b = item_pair(w, src_off, st, bmap, P, kIcpChunk, s_T, &s_pair);
+    __syncthreads();
+    if (threadIdx.x < 32)
+        item_setup(w, items, src_off, st, bmap, P, kIcpChunk, s_T, &s_item);
+    __syncthreads();
+    const BlockPair b = s_item;
     if (b.pair < 0)
         continue;
     Acc<Comp> acc;
@@ -835,9 +842,10 @@ __global__ void __launch_bounds__(kIcpThreads) k_icp_finalize(PairState *st, int
     rebuild_maps_body(st, P, bmap, bmap_nn, loop);
 }
 
-IcpShape icp_shape(const gca3d_tuning &t)
+IcpShape icp_shape(const gca3d_tuning &t, int P)
 {
     IcpShape s;
+    s.nn_chunk = P == 1 ? kNNChunkSingle : kNNChunk;
     if (t.nn_item_points == 64 || t.nn_item_points == 128 || t.nn_item_points == 256 || t.nn_item_points == 512)
         s.nn_chunk = t.nn_item_points;
     if (t.nn_blocks_per_sm > 0)

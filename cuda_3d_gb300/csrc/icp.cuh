@@ -9,25 +9,31 @@ namespace gca3d
 
 constexpr int kIcpThreads = 256;
 constexpr int kIcpChunk = 1024; // source points per accumulate work item (one partial each)
-constexpr int kNNChunk = 256;   // default source points per correspondence work item
+// source points per correspondence work item by default: a single pair's points make few
+// items of 256 (200k points: 800, of which 760 run at once and the rest after them), so they
+// are halved (frame pair -3 %, 250k pair -6 %); a batch has items enough, and pays for each
+// (batch64 +5 % at 128)
+constexpr int kNNChunk = 256, kNNChunkSingle = 128;
 constexpr int kNNChunkMin = 64; // the smallest item size a tuning may choose
 constexpr int kNNChunkMax = 512; // the largest
 
 // the launch shape in force (defaults filled in)
 struct IcpShape
 {
-    int nn_chunk = kNNChunk;
+    int nn_chunk = kNNChunkSingle;
     int nn_bps = 10;
     int acc_bps = 6;
     bool fused = false; // the accumulate's last block of each pair finalizes it
 };
-IcpShape icp_shape(const gca3d_tuning &t);
+IcpShape icp_shape(const gca3d_tuning &t, int P);
 constexpr int kTerms = 30;      // 21 JTJ (upper) + 6 JTr + r^2 + correspondences + sum d^2
 constexpr int kTermsPad = 32;
 
 struct PairState
 {
     double T[16];
+    float Tf[12]; // rows 0-2 of T rounded, for the point kernels: a block that converts them
+                  // itself waits on twelve FP64 conversions of 64 cycles each
     double rmse_ref, fitness, inlier_rmse;
     int iters;
     int converged;

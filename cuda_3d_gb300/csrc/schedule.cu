@@ -371,7 +371,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
             int2 *corr = sp[si].corr;
             const NNCerts cert = sp[si].cert;
             int *bmap = sp[si].bmap, *bmap_nn = sp[si].bmap_nn;
-            const IcpShape shape = icp_shape(p.tuning);
+            const IcpShape shape = icp_shape(p.tuning, P);
             if ((st = icp_setup(ctx, pl->d_state, P, bs.seg_off, bt.seg_off, bmap, bmap_nn, si, shape.nn_chunk)))
                 return st;
             IcpScale prm;
@@ -618,7 +618,7 @@ int gca3d::icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *cons
         pl->src_max = std::max(pl->src_max, src[k]->capacity);
         pl->tgt_max = std::max(pl->tgt_max, tgt[k]->capacity);
         nb += div_up(src[k]->capacity, kIcpChunk);
-        pl->max_blocks_nn += div_up(src[k]->capacity, icp_shape(params->tuning).nn_chunk);
+        pl->max_blocks_nn += div_up(src[k]->capacity, icp_shape(params->tuning, P).nn_chunk);
     }
     pl->max_blocks = std::max(nb, 1);
     pl->max_blocks_nn = std::max(pl->max_blocks_nn, 1);
@@ -849,7 +849,7 @@ extern "C" int gca3d_icp_autotune(gca3d_context *ctx, int n_pairs, gca3d_cloud *
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "autotune: bad arguments");
     reps = std::max(reps, 1);
     gca3d_icp_params p = *params;
-    const IcpShape s0 = icp_shape(p.tuning);
+    const IcpShape s0 = icp_shape(p.tuning, n_pairs);
     gca3d_tuning cur{s0.nn_chunk, s0.nn_bps, s0.acc_bps, p.tuning.voxel_resort, s0.fused ? 1 : 0,
                      p.tuning.serial_prep};
     cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -79,6 +79,8 @@ __global__ void k_vjp_init(PairState *st, Vec6 xi0)
     pose_from_x_device(xi0.v, GCA3D_UPDATE_SE3_EXP, T);
     for (int k = 0; k < 16; ++k)
         st[0].T[k] = T[k];
+    for (int k = 0; k < 12; ++k)
+        st[0].Tf[k] = (float)T[k];
     st[0].iters = 0;
     st[0].status = 0;
     st[0].rmse_ref = st[0].fitness = st[0].inlier_rmse = 0.0;
@@ -416,7 +418,7 @@ extern "C" int gca3d_color_icp_vjp(gca3d_context *ctx, gca3d_cloud *src, gca3d_c
     if ((st = grid_build(ctx, bt, p->max_corr, kOriginPadF32, nullptr, g)))
         return st;
     const int max_blocks = std::max(div_up(src->capacity, kIcpChunk), 1);
-    const int max_blocks_nn = std::max(div_up(src->capacity, kNNChunk), 1);
+    const int max_blocks_nn = std::max(div_up(src->capacity, kNNChunkSingle), 1);
     float4 *attr0 = ctx->arena.get<float4>(g.cap);
     float4 *attr1 = ctx->arena.get<float4>(g.cap);
     PairState *pst = ctx->arena.get<PairState>(1);

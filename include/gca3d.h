@@ -83,7 +83,8 @@ typedef struct {
 /* launch shape of the ICP iterations (0 = default).  Only the shape changes: results are
  * bit-identical for every setting.  gca3d_icp_autotune picks one for a workload. */
 typedef struct {
-    int nn_item_points;      /* source points per correspondence work item: 64, 128, 256 (default), 512 */
+    int nn_item_points;      /* source points per correspondence work item: 64, 128, 256, 512
+                                (default 128 for one pair, 256 for several) */
     int nn_blocks_per_sm;    /* correspondence grid = SMs x this (default 10), at most the items */
     int accum_blocks_per_sm; /* accumulate grid = SMs x this (default 6), at most the items */
     int voxel_resort;        /* 1: sort every scale's voxels anew; 0 (default): where the next
