@@ -28,6 +28,7 @@
 #include "stages.cuh"
 
 #include <algorithm>
+#include <cooperative_groups.h>
 
 namespace gca3d
 {
@@ -185,19 +186,19 @@ __device__ __forceinline__ void block_reduce_store(Acc<Comp> &acc, double *part)
     }
 }
 
-// exclusive prefix over the block's kIcpThreads threads of two per-thread counts: each
+// exclusive prefix over the block's Threads threads of two per-thread counts: each
 // thread gets its own prefixes back in a and b, and every thread the two totals
-__device__ __forceinline__ void block_prefix2(int &a, int &b, int &ta, int &tb)
+template <int Threads> __device__ __forceinline__ void block_prefix2(int &a, int &b, int &ta, int &tb)
 {
-    __shared__ int s_a[kIcpThreads], s_b[kIcpThreads];
+    __shared__ int s_a[Threads], s_b[Threads];
     __shared__ int s_ta, s_tb;
     s_a[threadIdx.x] = a;
     s_b[threadIdx.x] = b;
     __syncthreads();
     if (threadIdx.x < 32)
     {
-        // 8 per lane, then across the warp
-        constexpr int kPer = kIcpThreads / 32;
+        // a few per lane, then across the warp
+        constexpr int kPer = Threads / 32;
         const int l = threadIdx.x;
         int va[kPer], vb[kPer], sa = 0, sb = 0;
 #pragma unroll
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(kIcpThreads) k_icp_setup(PairState *st, int P,
     if (na)
         atomicAdd(&s_nact, na);
     int tb, tbn;
-    block_prefix2(b, bn, tb, tbn);
+    block_prefix2<kIcpThreads>(b, bn, tb, tbn);
     for (int p = p0; p < p1; ++p)
     {
         bmap[p] = b;
@@ -518,54 +519,80 @@ __global__ void __launch_bounds__(kIcpThreads, 5) k_icp_nn(const float4 *__restr
     }
 }
 
-// one pair's finalize, by one whole block: the pair's block partials summed in FP64
-// in block order, the 6x6 solve, the step map, the FP64 pose update and the
-// reference's convergence test (color_icp.cu:216-228).  The partials are read from
-// L2: in the fused accumulate other blocks of the same launch wrote them.
-template <bool Comp>
-__device__ __forceinline__ void finalize_pair_body(PairState *st, int P, int pair, const int *bmap,
-                                                   const double *partials, const IcpScale &prm)
+// the pair's block partials in FP64, in a fixed order: group g of 8 takes blocks g, g + 8, ...
+// as four running sums, (0 + 1) + (2 + 3), and the groups are added in order.  (Plain: FP32,
+// one sum per group.)  The element of group g's running sum r at step q is block
+// g + 8 (4 q + r); a remainder of fewer than four blocks goes to running sum 0.
+constexpr int kSumGroups = 8;
+
+// running sum `chain` of group grp (lane: term); chain 0 takes the remainder too.  Eight
+// loads are in flight at once; an FP64 addition takes 64 cycles of the warp.
+__device__ __forceinline__ double partial_chain(const double *src, int nb, int grp, int chain)
 {
-    PairState &Ps = st[pair];
-    __shared__ double s_red[kIcpThreads / 32][kTermsPad];
-    const int nb = Ps.nblocks, bstart = bmap[pair];
+    constexpr int kW = kSumGroups, kAhead = 8;
+    const int x = nb - grp - 3 * kW;
+    const int full = x > 0 ? (x + 4 * kW - 1) / (4 * kW) : 0; // whole steps of four
+    const int tail = grp + 4 * kW * full;                     // the remainder's first block
+    const int rest = chain == 0 && nb > tail ? (nb - tail + kW - 1) / kW : 0;
+    double v = 0.0;
+    for (int q0 = 0; q0 < full + rest; q0 += kAhead)
+    {
+        double p[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+        {
+            const int q = q0 + u;
+            const int j = q < full ? grp + kW * (4 * q + chain) : tail + kW * (q - full);
+            p[u] = q < full + rest ? __ldcg(src + (size_t)j * kTermsPad) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (q0 + u < full + rest)
+                v += p[u];
+    }
+    return v;
+}
+
+// one pair's sums by one whole block into s_S (the fused accumulate).  The partials are
+// read from L2: other blocks of the same launch wrote them.
+template <bool Comp>
+__device__ __forceinline__ void finalize_sums(const PairState &Ps, const double *src, double *s_S)
+{
+    __shared__ double s_red[kSumGroups][kTermsPad];
+    static_assert(kSumGroups == kIcpThreads / 32, "one warp per group");
+    const int nb = Ps.nblocks;
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
     if (lane < kTerms)
     {
-        constexpr int kW = kIcpThreads / 32;
-        const double *src = partials + (size_t)bstart * kTermsPad + lane;
         if (Comp)
         {
-            // four running sums (blocks grp + 8 (4 q + r), r = 0..3), added in a fixed order
-            double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
+            // the four chains side by side (each in its own order)
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+            constexpr int kW = kSumGroups;
             int j = grp;
             for (; j + 3 * kW < nb; j += 4 * kW)
-            {
-                v0 += __ldcg(src + (size_t)j * kTermsPad);
-                v1 += __ldcg(src + (size_t)(j + kW) * kTermsPad);
-                v2 += __ldcg(src + (size_t)(j + 2 * kW) * kTermsPad);
-                v3 += __ldcg(src + (size_t)(j + 3 * kW) * kTermsPad);
-            }
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    v[r] += __ldcg(src + (size_t)(j + r * kW) * kTermsPad + lane);
             for (; j < nb; j += kW)
-                v0 += __ldcg(src + (size_t)j * kTermsPad);
-            s_red[grp][lane] = (v0 + v1) + (v2 + v3);
+                v[0] += __ldcg(src + (size_t)j * kTermsPad + lane);
+            s_red[grp][lane] = (v[0] + v[1]) + (v[2] + v[3]);
         }
         else
         {
             float vf = 0.0f;
-            for (int j = grp; j < nb; j += kW)
-                vf += (float)__ldcg(src + (size_t)j * kTermsPad);
+            for (int j = grp; j < nb; j += kSumGroups)
+                vf += (float)__ldcg(src + (size_t)j * kTermsPad + lane);
             s_red[grp][lane] = (double)vf;
         }
     }
     __syncthreads();
-    __shared__ double s_S[kTermsPad];
     if (threadIdx.x < kTerms)
     {
         const int k = threadIdx.x;
         double v = 0.0;
         float vf = 0.0f;
-        for (int w = 0; w < kIcpThreads / 32; ++w)
+        for (int w = 0; w < kSumGroups; ++w)
         {
             if (Comp)
                 v += s_red[w][k];
@@ -575,7 +602,34 @@ __device__ __forceinline__ void finalize_pair_body(PairState *st, int P, int pai
         s_S[k] = Comp ? v : (double)vf;
     }
     __syncthreads();
-    const int warp = grp;
+}
+
+// what a pair's finalize reads of its state, read before the sums are there
+struct FinalizeIn
+{
+    double T; // entry `lane` of the pose (lanes 0..15)
+    int iters, scale, scale_iter, status, nsrc;
+};
+__device__ __forceinline__ FinalizeIn finalize_in(const PairState &Ps)
+{
+    const int lane = threadIdx.x & 31;
+    FinalizeIn in;
+    in.T = lane < 16 ? Ps.T[lane] : 0.0;
+    in.iters = Ps.iters;
+    in.scale = Ps.scale;
+    in.status = Ps.status;
+    in.nsrc = Ps.nsrc;
+    in.scale_iter = Ps.scale_iters[in.scale];
+    return in;
+}
+
+// one pair's finalize from its sums: the 6x6 solve, the step map, the FP64 pose update and
+// the reference's convergence test (color_icp.cu:216-228) by warp 0, the statistics by
+// warp 1; other warps return at once
+__device__ __forceinline__ void finalize_solve(PairState &Ps, int P, int pair, const double *s_S, const IcpScale &prm,
+                                               const FinalizeIn &in)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0)
     {
         // solve, step map and composition over the lanes of warp 0
@@ -583,15 +637,21 @@ __device__ __forceinline__ void finalize_pair_body(PairState *st, int P, int pai
         const int singular = solve6_warp(s_S, x);
         const double Ti = pose_from_x_warp(x, prm.update_map); // lanes 0..15: Ti[lane]
         const int r = (lane >> 2) & 3, c = lane & 3;
-        const double Told = lane < 16 ? Ps.T[lane] : 0.0;
+        const double Told = in.T;
         double v = 0.0;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             v += __shfl_sync(0xffffffffu, Ti, 4 * r + k) * __shfl_sync(0xffffffffu, Told, 4 * k + c);
-        const double t00 = __shfl_sync(0xffffffffu, Ti, 0), t11 = __shfl_sync(0xffffffffu, Ti, 5),
-                     t22 = __shfl_sync(0xffffffffu, Ti, 10), t03 = __shfl_sync(0xffffffffu, Ti, 3),
-                     t13 = __shfl_sync(0xffffffffu, Ti, 7), t23 = __shfl_sync(0xffffffffu, Ti, 11);
-        const int iters = Ps.iters;
+        // lane 0: the step's cosine, 0.5 (trace - 1); lane 1: its squared translation, negated
+        // (compared as >= with cos_min and -trans_eps)
+        const double d0 = __shfl_sync(0xffffffffu, Ti, lane == 1 ? 3 : 0),
+                     d1 = __shfl_sync(0xffffffffu, Ti, lane == 1 ? 7 : 5),
+                     d2 = __shfl_sync(0xffffffffu, Ti, lane == 1 ? 11 : 10);
+        const double w0 = lane == 1 ? d0 : 1.0, w1 = lane == 1 ? d1 : 1.0, w2 = lane == 1 ? d2 : 1.0;
+        const double dsum = fma(d2, w2, fma(d1, w1, d0 * w0));
+        const double measure = fma(dsum, lane == 1 ? -1.0 : 0.5, lane == 1 ? 0.0 : -0.5);
+        const unsigned small = __ballot_sync(0xffffffffu, measure >= (lane == 1 ? -prm.trans_eps : prm.cos_min));
+        const int iters = in.iters;
         if (prm.trace && iters < prm.trace_cap)
         {
             IcpTrace &tr = prm.trace[(size_t)iters * P + pair];
@@ -614,16 +674,14 @@ __device__ __forceinline__ void finalize_pair_body(PairState *st, int P, int pai
             Ps.Tf[lane] = (float)v;
         if (lane == 0)
         {
-            if (s_S[28] == 0.0)
+            if (__double_as_longlong(s_S[28]) == 0ll) // a count: never -0
                 Ps.status = GCA3D_ERR_NO_CORRESPONDENCES;
-            else if (singular && Ps.status == 0)
+            else if (singular && in.status == 0)
                 Ps.status = GCA3D_ERR_SINGULAR;
             Ps.iters = iters + 1;
-            Ps.scale_iters[Ps.scale] += 1;
+            Ps.scale_iters[in.scale] = in.scale_iter + 1;
             Ps.nn_warm = 1;
-            const double cth = 0.5 * (t00 + t11 + t22 - 1.0);
-            const double tsq = t03 * t03 + t13 * t13 + t23 * t23;
-            if (cth >= 1.0 - prm.rot_eps && tsq <= prm.trans_eps)
+            if ((small & 3u) == 3u)
             {
                 Ps.converged = 1;
                 Ps.active = 0;
@@ -633,7 +691,7 @@ __device__ __forceinline__ void finalize_pair_body(PairState *st, int P, int pai
     else if (warp == 1)
     {
         // the statistics, on their own warp (one division per lane)
-        const double ns = (double)Ps.nsrc;
+        const double ns = (double)in.nsrc;
         const int m = lane % 3;
         const double num = m == 0 ? s_S[27] : (m == 1 ? s_S[28] : s_S[29]);
         const double den = m == 2 ? s_S[28] : ns;
@@ -653,13 +711,14 @@ __device__ __forceinline__ void finalize_pair_body(PairState *st, int P, int pai
 // launches get no items for converged pairs), their count and, in a captured
 // schedule, the loop condition.  Run by one whole block once every pair of the
 // iteration is finalized.
+template <int Threads>
 __device__ __forceinline__ void rebuild_maps_body(PairState *st, int P, int *bmap, int *bmap_nn, const IcpLoop &loop)
 {
     __shared__ int s_nact;
     if (threadIdx.x == 0)
         s_nact = 0;
     __syncthreads();
-    const int per = (P + kIcpThreads - 1) / kIcpThreads;
+    const int per = (P + Threads - 1) / Threads;
     const int p0 = min(P, (int)threadIdx.x * per), p1 = min(P, p0 + per);
     int a = 0, an = 0, na = 0;
     for (int q = p0; q < p1; ++q)
@@ -672,7 +731,7 @@ __device__ __forceinline__ void rebuild_maps_body(PairState *st, int P, int *bma
     if (na)
         atomicAdd(&s_nact, na);
     int ta, tn;
-    block_prefix2(a, an, ta, tn);
+    block_prefix2<Threads>(a, an, ta, tn);
     if (threadIdx.x == 0)
     {
         bmap[P] = ta;
@@ -698,19 +757,39 @@ __device__ __forceinline__ void rebuild_maps_body(PairState *st, int P, int *bma
     }
 }
 
+// rebuild_maps_body for a single pair, by one thread; iter: the loop count so far
+__device__ __forceinline__ void rebuild_single(int act, int nblocks, int nblocks_nn, int iter, int *bmap, int *bmap_nn,
+                                               const IcpLoop &loop)
+{
+    const int tn = act ? nblocks_nn : 0;
+    bmap[0] = bmap_nn[0] = 0;
+    bmap[1] = act ? nblocks : 0;
+    bmap[2] = act ? 1 : 0;
+    bmap_nn[1] = tn;
+    bmap_nn[2] = 0;
+    *loop.ticket = 0u;
+    if (loop.iter)
+    {
+        *loop.iter = iter + 1;
+        cudaGraphSetConditional(loop.handle, (tn > 0 && iter + 1 < loop.max_iter) ? 1u : 0u);
+    }
+}
+
 // the same two steps as calls, for the fused accumulate: compiled apart from the
 // accumulation loop, whose registers they would otherwise crowd (the separate finalize
-// kernel inlines the bodies)
+// kernel has its own sums)
 template <bool Comp>
 __device__ __noinline__ void finalize_pair(PairState *st, int P, int pair, const int *bmap, const double *partials,
                                            IcpScale prm)
 {
-    finalize_pair_body<Comp>(st, P, pair, bmap, partials, prm);
+    __shared__ double s_S[kTermsPad];
+    finalize_sums<Comp>(st[pair], partials + (size_t)bmap[pair] * kTermsPad, s_S);
+    finalize_solve(st[pair], P, pair, s_S, prm, finalize_in(st[pair]));
 }
 
 __device__ __noinline__ void rebuild_maps(PairState *st, int P, int *bmap, int *bmap_nn, IcpLoop loop)
 {
-    rebuild_maps_body(st, P, bmap, bmap_nn, loop);
+    rebuild_maps_body<kIcpThreads>(st, P, bmap, bmap_nn, loop);
 }
 
 // step 2: residuals, Jacobians, block sums (one partial per block); three resident
@@ -818,28 +897,92 @@ __global__ void __launch_bounds__(kIcpThreads, 3) k_icp_accum(const float4 *__re
     }
 }
 
-// the finalize as a launch of its own (one block per pair); the last block to
-// finish rebuilds the work maps
+// the finalize as a launch of its own: a cluster of eight blocks per pair, block g summing
+// group g with a warp per running sum (an SM adds one FP64 warp instruction in 19 cycles, so
+// 200 partials took one block 3 us; eight SMs take 1), then block 0 solves.  The last pair's
+// block rebuilds the work maps; a single pair's does so directly.  What bounds it is the chain
+// of FP64 operations at 64 cycles each: @@
 template <bool Comp>
-__global__ void __launch_bounds__(kIcpThreads) k_icp_finalize(PairState *st, int P, int *bmap, int *bmap_nn,
-                                                              const double *partials, IcpScale prm, IcpLoop loop)
+__global__ void __launch_bounds__(128) k_icp_finalize(PairState *st, int P, int *bmap, int *bmap_nn,
+                                                      const double *partials, IcpScale prm, IcpLoop loop)
 {
-    __shared__ int s_last;
-    if (st[blockIdx.x].active)
-        finalize_pair_body<Comp>(st, P, blockIdx.x, bmap, partials, prm);
-    if (gridDim.x > 1)
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ double s_part[4][kTermsPad];
+    __shared__ double s_group[kTermsPad]; // this block's group
+    __shared__ double s_S[kTermsPad];
+    const int grp = (int)cluster.block_rank(), pair = blockIdx.x / kSumGroups;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    PairState &Ps = st[pair];
+    // everything read of the state and the maps, at once (the loads of one another's results
+    // were half of the chain); the cluster's blocks see the same state: block 0 writes it
+    // after the last barrier
+    const bool active = Ps.active;
+    const int nb = Ps.nblocks, nb_nn = Ps.nblocks_nn, first = bmap[pair];
+    const int iter = loop.iter && P == 1 ? *loop.iter : 0;
+    FinalizeIn in{};
+    if (grp == 0)
+        in = finalize_in(Ps);
+    if (active)
     {
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0)
-            s_last = atomicAdd(loop.ticket, 1u) == gridDim.x - 1;
+        const double *src = partials + (size_t)first * kTermsPad + lane;
+        if (Comp)
+        {
+            if (lane < kTerms)
+                s_part[warp][lane] = partial_chain(src, nb, grp, warp);
+            __syncthreads();
+            if (threadIdx.x < kTerms)
+                s_group[threadIdx.x] = (s_part[0][threadIdx.x] + s_part[1][threadIdx.x]) +
+                                       (s_part[2][threadIdx.x] + s_part[3][threadIdx.x]);
+        }
+        else if (threadIdx.x < kTerms)
+        {
+            float vf = 0.0f;
+#pragma unroll 8
+            for (int j = grp; j < nb; j += kSumGroups)
+                vf += (float)__ldcg(src + (size_t)j * kTermsPad);
+            s_group[threadIdx.x] = (double)vf;
+        }
     }
-    else if (threadIdx.x == 0)
-        s_last = 1; // one pair: this block is the last, and its own writes are visible after the barrier
+    cluster.sync();
+    if (grp == 0 && active && threadIdx.x < kTerms)
+    {
+        double part[kSumGroups];
+#pragma unroll
+        for (int w = 0; w < kSumGroups; ++w)
+            part[w] = cluster.map_shared_rank(s_group, w)[threadIdx.x];
+        double v = 0.0;
+        float vf = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kSumGroups; ++w)
+        {
+            if (Comp)
+                v += part[w];
+            else
+                vf += (float)part[w];
+        }
+        s_S[threadIdx.x] = Comp ? v : (double)vf;
+    }
+    cluster.sync(); // the groups are read: the other blocks may leave
+    if (grp != 0)
+        return;
+    if (active)
+        finalize_solve(Ps, P, pair, s_S, prm, in);
+    if (P == 1)
+    {
+        if (threadIdx.x == 0) // thread 0 wrote the state's flag itself
+            rebuild_single(Ps.active, nb, nb_nn, iter, bmap, bmap_nn, loop);
+        return;
+    }
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        s_last = atomicAdd(loop.ticket, 1u) == (unsigned)(P - 1);
     __syncthreads();
     if (!s_last)
         return;
-    rebuild_maps_body(st, P, bmap, bmap_nn, loop);
+    rebuild_maps_body<128>(st, P, bmap, bmap_nn, loop);
 }
 
 IcpShape icp_shape(const gca3d_tuning &t, int P)
@@ -925,12 +1068,18 @@ int icp_update(gca3d_context *ctx, const Batch &src, const Grid &g, const float4
                 src.pos, src.seg_off, g.dev.spos, attr0, attr1, corr, st, bmap, bmap_nn, src.P, partials,
                 prm.sqrt_lg, prm.sqrt_lc, d_nt, ctx->d_err, prm, loop);
         GCA_CHECK_LAUNCH(ctx);
-        if (compensated)
-            k_icp_finalize<true><<<src.P, kIcpThreads, 0, ctx->stream>>>(st, src.P, bmap, bmap_nn, partials, prm,
-                                                                         loop);
-        else
-            k_icp_finalize<false><<<src.P, kIcpThreads, 0, ctx->stream>>>(st, src.P, bmap, bmap_nn, partials, prm,
-                                                                          loop);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kSumGroups * src.P);
+        cfg.blockDim = dim3(128);
+        cfg.stream = ctx->stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kSumGroups;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        GCA_CUDA(ctx, cudaLaunchKernelEx(&cfg, compensated ? k_icp_finalize<true> : k_icp_finalize<false>, st, src.P,
+                                         bmap, bmap_nn, partials, prm, loop));
         GCA_CHECK_LAUNCH(ctx);
     }
     GCA_PROF_END(ctx, kKidIcpIter);

@@ -67,7 +67,7 @@ struct IcpScale
     float max_corr;
     float sqrt_lg, sqrt_lc;
     int update_map;
-    double rot_eps, trans_eps;
+    double cos_min, trans_eps; // converged: cosine of the step angle and |step translation|^2
     IcpTrace *trace = nullptr; // [trace_cap iterations][P pairs] or null
     int trace_cap = 0;
 };

@@ -195,54 +195,51 @@ __device__ __forceinline__ double rcp_nr(double d)
     return fma(r, e, r);
 }
 
-// sin x and cos x for |x| <= kSmallAngle from their Taylor series (Horner in x^2,
-// through x^13 and x^14; the first omitted terms are below 1e-18 relative)
+// An FP64 instruction takes its warp 64 cycles however many lanes are active, so the series
+// below are evaluated for several results at once, one per lane: the same steps with the
+// lane's coefficients.
+
+// sin x (or cos x) for |x| <= kSmallAngle from its Taylor series (Horner in x^2, through
+// x^13 and x^14; the first omitted terms are below 1e-18 relative)
 constexpr double kSmallAngle = 0.25;
-__device__ __forceinline__ void sincos_small(double x, double &s, double &c)
+__device__ __forceinline__ double sin_or_cos_small(double x, bool cosine)
 {
     const double z = x * x;
-    double ps = 1.0 / 6227020800.0; // 1/13!
-    double pc = 1.0 / 87178291200.0; // 1/14!
-    ps = fma(ps, -z, 1.0 / 39916800.0);
-    pc = fma(pc, -z, 1.0 / 479001600.0);
-    ps = fma(ps, -z, 1.0 / 362880.0);
-    pc = fma(pc, -z, 1.0 / 3628800.0);
-    ps = fma(ps, -z, 1.0 / 5040.0);
-    pc = fma(pc, -z, 1.0 / 40320.0);
-    ps = fma(ps, -z, 1.0 / 120.0);
-    pc = fma(pc, -z, 1.0 / 720.0);
-    ps = fma(ps, -z, 1.0 / 6.0);
-    pc = fma(pc, -z, 1.0 / 24.0);
-    pc = fma(pc, -z, 0.5);
-    s = fma(-x * z, ps, x);
-    c = fma(-z, pc, 1.0);
+    double p = cosine ? 1.0 / 87178291200.0 : 1.0 / 6227020800.0; // 1/14!, 1/13!
+    p = fma(p, -z, cosine ? 1.0 / 479001600.0 : 1.0 / 39916800.0);
+    p = fma(p, -z, cosine ? 1.0 / 3628800.0 : 1.0 / 362880.0);
+    p = fma(p, -z, cosine ? 1.0 / 40320.0 : 1.0 / 5040.0);
+    p = fma(p, -z, cosine ? 1.0 / 720.0 : 1.0 / 120.0);
+    p = fma(p, -z, cosine ? 1.0 / 24.0 : 1.0 / 6.0);
+    const double last = fma(p, -z, 0.5); // the cosine has one coefficient more
+    return fma(cosine ? -z : -x * z, cosine ? last : p, cosine ? 1.0 : x);
+}
+__device__ __forceinline__ void sincos_small(double x, double &s, double &c)
+{
+    s = sin_or_cos_small(x, false);
+    c = sin_or_cos_small(x, true);
 }
 
 // the coefficients of the SO(3) / SE(3) exponential, A = sin t / t,
-// B = (1 - cos t) / t^2, C = (t - sin t) / t^3, as series in t2 = t^2 for
+// B = (1 - cos t) / t^2, C = (t - sin t) / t^3 (k = 0, 1, 2), as series in t2 = t^2 for
 // t2 <= kSmallAngle^2 (A = sum (-t2)^n / (2n+1)!, B = sum (-t2)^n / (2n+2)!,
 // C = sum (-t2)^n / (2n+3)!, n <= 6; the first omitted terms are below 1e-19)
+__device__ __forceinline__ double exp_coeff_small(double t2, int k)
+{
+    auto pick = [k](double a, double b, double c) { return k == 0 ? a : (k == 1 ? b : c); };
+    double p = pick(1.0 / 6227020800.0, 1.0 / 87178291200.0, 1.0 / 1307674368000.0); // 1/13!, 1/14!, 1/15!
+    p = fma(p, -t2, pick(1.0 / 39916800.0, 1.0 / 479001600.0, 1.0 / 6227020800.0));
+    p = fma(p, -t2, pick(1.0 / 362880.0, 1.0 / 3628800.0, 1.0 / 39916800.0));
+    p = fma(p, -t2, pick(1.0 / 5040.0, 1.0 / 40320.0, 1.0 / 362880.0));
+    p = fma(p, -t2, pick(1.0 / 120.0, 1.0 / 720.0, 1.0 / 5040.0));
+    p = fma(p, -t2, pick(1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0));
+    return fma(p, -t2, pick(1.0, 0.5, 1.0 / 6.0));
+}
 __device__ __forceinline__ void exp_coeffs_small(double t2, double &A, double &B, double &C)
 {
-    double a = 1.0 / 6227020800.0, b = 1.0 / 87178291200.0, c = 1.0 / 1307674368000.0; // 1/13!, 1/14!, 1/15!
-    a = fma(a, -t2, 1.0 / 39916800.0);
-    b = fma(b, -t2, 1.0 / 479001600.0);
-    c = fma(c, -t2, 1.0 / 6227020800.0);
-    a = fma(a, -t2, 1.0 / 362880.0);
-    b = fma(b, -t2, 1.0 / 3628800.0);
-    c = fma(c, -t2, 1.0 / 39916800.0);
-    a = fma(a, -t2, 1.0 / 5040.0);
-    b = fma(b, -t2, 1.0 / 40320.0);
-    c = fma(c, -t2, 1.0 / 362880.0);
-    a = fma(a, -t2, 1.0 / 120.0);
-    b = fma(b, -t2, 1.0 / 720.0);
-    c = fma(c, -t2, 1.0 / 5040.0);
-    a = fma(a, -t2, 1.0 / 6.0);
-    b = fma(b, -t2, 1.0 / 24.0);
-    c = fma(c, -t2, 1.0 / 120.0);
-    A = fma(a, -t2, 1.0);
-    B = fma(b, -t2, 0.5);
-    C = fma(c, -t2, 1.0 / 6.0);
+    A = exp_coeff_small(t2, 0);
+    B = exp_coeff_small(t2, 1);
+    C = exp_coeff_small(t2, 2);
 }
 
 // the solve over one warp (same symmetric pivots, factorisation and
@@ -280,20 +277,20 @@ __device__ inline int solve6_warp(const double *S /* 21 upper + 6 rhs */, double
         // chosen one is broadcast below, so the division is off the pivot's chain)
         const double ra = diag ? rcp_nr(a) : 0.0;
         // symmetric pivot: the largest remaining diagonal entry (first one on ties);
-        // magnitudes compared as the bit patterns of |A[i][i]|
-        const long long mag = diag ? (__double_as_longlong(a) & 0x7fffffffffffffffll) : -1ll;
-        int piv = k;
-        long long best = __shfl_sync(full, mag, tri_lane(k, k));
-#pragma unroll
-        for (int i = k + 1; i < 6; ++i)
+        // magnitudes compared as the bit patterns of |A[i][i]|, upper words first
+        const unsigned long long mag = __double_as_longlong(a) & 0x7fffffffffffffffull;
+        const unsigned hi = (unsigned)(mag >> 32), lo = (unsigned)mag;
+        const bool cand = diag && li >= k;
+        const unsigned top = __reduce_max_sync(full, cand ? hi : 0u);
+        unsigned at = __ballot_sync(full, cand && hi == top);
+        if (__popc(at) > 1)
         {
-            const long long v = __shfl_sync(full, mag, tri_lane(i, i));
-            if (v > best)
-            {
-                best = v;
-                piv = i;
-            }
+            const bool tied = cand && hi == top;
+            const unsigned low = __reduce_max_sync(full, tied ? lo : 0u);
+            at = __ballot_sync(full, tied && lo == low);
         }
+        const int plane = __ffs(at) - 1; // diagonal lanes ascend with their index
+        const int piv = __shfl_sync(full, li, plane);
         if (piv != k)
         {
             const int si = li == k ? piv : (li == piv ? k : li), sj = lj == k ? piv : (lj == piv ? k : lj);
@@ -303,9 +300,10 @@ __device__ inline int solve6_warp(const double *S /* 21 upper + 6 rhs */, double
             perm = (perm & ~((15u << (4 * k)) | (15u << (4 * piv)))) | (pp << (4 * k)) | (pk << (4 * piv));
         }
         const double Dk = __shfl_sync(full, a, tri_lane(k, k));
-        const double rk = __shfl_sync(full, ra, tri_lane(piv, piv)); // 1 / Dk (before the swap)
+        const double rk = __shfl_sync(full, ra, plane); // 1 / Dk (before the swap)
         const bool lcol = mat && lj == k && li > k;
-        if (fabs(Dk) <= kTiny)
+        // (magnitudes compared as bit patterns: an FP64 comparison takes 64 cycles too)
+        if ((__double_as_longlong(Dk) & 0x7fffffffffffffffll) <= __double_as_longlong(kTiny))
         {
             status = 1;
             if (lcol)
@@ -335,7 +333,7 @@ __device__ inline int solve6_warp(const double *S /* 21 upper + 6 rhs */, double
             acc -= lij * yj;
     }
     if (diag)
-        acc = fabs(a) > kTiny ? acc * rcp_nr(a) : 0.0;
+        acc = (__double_as_longlong(a) & 0x7fffffffffffffffll) > __double_as_longlong(kTiny) ? acc * rcp_nr(a) : 0.0;
     // L^T z = y, by columns from the last
 #pragma unroll
     for (int j = 5; j > 0; --j)
@@ -373,16 +371,22 @@ __device__ inline double pose_from_x_warp(const double x[6], int map)
     double Rrc, tr;
     if (map == GCA3D_UPDATE_EULER_ZYX)
     {
+        // lanes 0..2: the sines, 3..5: the cosines
         const int m = lane % 3;
+        const bool cosine = (lane / 3) & 1;
         const double xm = m == 0 ? x[0] : (m == 1 ? x[1] : x[2]);
-        double sn, cs;
+        double f;
         if (fabs(xm) <= kSmallAngle)
-            sincos_small(xm, sn, cs);
+            f = sin_or_cos_small(xm, cosine);
         else
+        {
+            double sn, cs;
             sincos(xm, &sn, &cs);
-        const double sa = __shfl_sync(full, sn, 0), ca = __shfl_sync(full, cs, 0);
-        const double sb = __shfl_sync(full, sn, 1), cb = __shfl_sync(full, cs, 1);
-        const double sc = __shfl_sync(full, sn, 2), ccz = __shfl_sync(full, cs, 2);
+            f = cosine ? cs : sn;
+        }
+        const double sa = __shfl_sync(full, f, 0), ca = __shfl_sync(full, f, 3);
+        const double sb = __shfl_sync(full, f, 1), cb = __shfl_sync(full, f, 4);
+        const double sc = __shfl_sync(full, f, 2), ccz = __shfl_sync(full, f, 5);
         // R = Rz(x2) Ry(x1) Rx(x0), entry (rr, cc) as u * v * w + g0 * g1 with
         // operands picked per lane (one uniform FP64 expression, no divergence)
         const int e = 3 * rr + cc;
@@ -398,23 +402,20 @@ __device__ inline double pose_from_x_warp(const double x[6], int map)
     {
         const double w0 = x[0], w1 = x[1], w2 = x[2];
         const double th2 = w0 * w0 + w1 * w1 + w2 * w2;
-        double A, B, C;
+        const int m = lane % 3; // the three coefficients on three lanes
+        double q;
         if (th2 <= kSmallAngle * kSmallAngle)
-            exp_coeffs_small(th2, A, B, C); // no root, sine or division on the chain
+            q = exp_coeff_small(th2, m); // no root, sine or division on the chain
         else
         {
             const double th = sqrt(th2);
             double sn, cs;
             sincos(th, &sn, &cs);
-            // the three coefficient divisions on three lanes
-            const int m = lane % 3;
             const double num = m == 0 ? sn : (m == 1 ? 1.0 - cs : th - sn);
             const double den = m == 0 ? th : (m == 1 ? th2 : th2 * th);
-            const double q = num * rcp_nr(den);
-            A = __shfl_sync(full, q, 0);
-            B = __shfl_sync(full, q, 1);
-            C = __shfl_sync(full, q, 2);
+            q = num * rcp_nr(den);
         }
+        const double A = __shfl_sync(full, q, 0), B = __shfl_sync(full, q, 1), C = __shfl_sync(full, q, 2);
         const double K[3][3] = {{0, -w2, w1}, {w2, 0, -w0}, {-w1, w0, 0}};
         auto Kat = [&](int i, int j) { return i == 0 ? (j == 0 ? K[0][0] : j == 1 ? K[0][1] : K[0][2])
                                              : i == 1 ? (j == 0 ? K[1][0] : j == 1 ? K[1][1] : K[1][2])

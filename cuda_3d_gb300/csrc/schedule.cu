@@ -379,7 +379,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
             prm.sqrt_lg = sqrtf(p.lambda);
             prm.sqrt_lc = sqrtf(1.0f - p.lambda);
             prm.update_map = p.update_map;
-            prm.rot_eps = p.rot_eps;
+            prm.cos_min = 1.0 - p.rot_eps;
             prm.trans_eps = p.trans_eps;
             // loop counter and finalize ticket
             int *iter = ctx->arena.get<int>(2);

@@ -457,7 +457,7 @@ extern "C" int gca3d_color_icp_vjp(gca3d_context *ctx, gca3d_cloud *src, gca3d_c
     prm.sqrt_lg = sqrtf(p->lambda);
     prm.sqrt_lc = sqrtf(1.0f - p->lambda);
     prm.update_map = p->update_map;
-    prm.rot_eps = -1.0; // never converged: exactly K steps
+    prm.cos_min = 2.0; // never converged: exactly K steps
     prm.trans_eps = -1.0;
     prm.trace = trace;
     prm.trace_cap = K + 1;
