@@ -290,6 +290,11 @@ struct NormalOut
     float grad_r2;
     float4 *attr1, *grd_out;
     float4 *degen_mom;
+    // points with more than max_nn neighbours (max_nn > 0), left to the selection pass, and
+    // their gradient moments as above
+    int *over_count;
+    int *over_list;
+    float4 *over_mom;
 };
 
 // The colour gradient from moments about the point p: G = sum d d^T (xx, xy, xz, yy,
@@ -361,6 +366,13 @@ struct PointMoments
     int k, gk;
 };
 
+__device__ __forceinline__ void keep_gradient_moments(float4 *at, const PointMoments &M)
+{
+    at[0] = make_float4(M.gxx, M.gxy, M.gxz, M.gyy);
+    at[1] = make_float4(M.gyz, M.gzz, M.mx, M.my);
+    at[2] = make_float4(M.mz, __int_as_float(M.gk), 0.0f, 0.0f);
+}
+
 // what follows a point's walk: the FP32 eigen-solve (or the queue for the FP64 pass),
 // the orientation, the gradient and the stores.  Compiled once and called by every
 // instantiation of the walk, so that the results round alike whichever walk summed
@@ -378,11 +390,7 @@ __device__ __noinline__ void finish_point(const int32_t *sidx, NormalOut O, int 
             const int slot = atomicAdd(O.degen_count, 1);
             O.degen_list[slot] = s;
             if (grad)
-            {
-                O.degen_mom[3 * slot] = make_float4(M.gxx, M.gxy, M.gxz, M.gyy);
-                O.degen_mom[3 * slot + 1] = make_float4(M.gyz, M.gzz, M.mx, M.my);
-                O.degen_mom[3 * slot + 2] = make_float4(M.mz, __int_as_float(M.gk), 0.0f, 0.0f);
-            }
+                keep_gradient_moments(O.degen_mom + 3 * slot, M);
             return; // written by the FP64 pass
         }
         // orient against (0, 0, -1) (cuda_estimate_normals.cu:131-151)
@@ -414,7 +422,6 @@ __global__ void __launch_bounds__(256, 4) k_normals32(GridDev g, const int32_t *
     const KeyLayout L = *g.layout;
     const int segshift = L.bx + L.by + L.bz;
     const float rn2 = __fmul_rn(rn, rn);
-    NbrEntry list[kMaxNN];
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
     {
         const float4 p4 = g.spos[s];
@@ -435,9 +442,8 @@ __global__ void __launch_bounds__(256, 4) k_normals32(GridDev g, const int32_t *
             syy = fmaf(dy, dy, syy), syz = fmaf(dy, dz, syz), szz = fmaf(dz, dz, szz);
             ++k;
         };
-        // every neighbour inside the radius; only when there are more than max_nn
-        // are the max_nn nearest selected instead (most points have fewer, and then
-        // the two sets are the same)
+        // every neighbour inside the radius; a point with more than max_nn of them goes to
+        // the selection pass (most have fewer, and then the two sets are the same)
         if (inside)
             grid_scan<kNormScanBatch>(g, R, [&](int t, float4 q) {
                 const float d2 = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
@@ -467,18 +473,194 @@ __global__ void __launch_bounds__(256, 4) k_normals32(GridDev g, const int32_t *
             gxx = sxx, gxy = sxy, gxz = sxz, gyy = syy, gyz = syz, gzz = szz;
             gk = k;
         }
-        if (inside && max_nn > 0 && k > max_nn)
+        const PointMoments M{s1x, s1y, s1z, sxx, sxy, sxz, syy, syz, szz, gxx, gxy, gxz, gyy, gyz, gzz, mx, my, mz, k, gk};
+        if (max_nn > 0 && k > max_nn)
         {
-            s1x = s1y = s1z = sxx = sxy = sxz = syy = syz = szz = 0.0f;
-            k = 0;
-            const int cnt = select_knn(g, R, p, rn2, max_nn, list);
-            for (int j = 0; j < cnt; ++j)
-                acc(g.spos[list[j].t]);
+            const int slot = atomicAdd(O.over_count, 1);
+            O.over_list[slot] = s;
+            if (Grad)
+                keep_gradient_moments(O.over_mom + 3 * slot, M);
+            continue; // written by the selection pass
         }
-        finish_point(g.sidx, O, s, Ip,
-                     PointMoments{s1x, s1y, s1z, sxx, sxy, sxz, syy, syz, szz, gxx, gxy, gxz, gyy, gyz, gzz, mx,
-                                  my, mz, k, gk},
-                     Grad);
+        finish_point(g.sidx, O, s, Ip, M, Grad);
+    }
+}
+
+// The points with more than max_nn neighbours: the max_nn nearest (distance, then index)
+// selected, then as in pass 1.  A warp per point: its lanes read the window's candidates side
+// by side, those inside the radius go to shared memory as (distance, index) keys, a
+// candidate's rank is the number of smaller keys, and nine lanes sum the nine moments over
+// the ranks in order (the order of an ordered list, so the sums round alike).  Up to 32
+// points' moments are then finished by one lane each.  A neighbourhood beyond the shared
+// list falls back to one lane with an ordered list in local memory.
+// One thread per point with such a list is bound by its local memory: inside pass 1 it held
+// every warp with one such lane (206k points, at most 30 neighbours: 119 us for the pass,
+// @@), and where most points exceed the cap (200k points, radius of three voxels) the call
+// took 2468 us, now @@.
+constexpr int kSelCand = 256;
+constexpr int kSelWarps = 4;
+
+template <bool Grad>
+__global__ void __launch_bounds__(32 * kSelWarps) k_normals_select(GridDev g, float rn, int max_nn, NormalOut O)
+{
+    __shared__ unsigned long long s_key[kSelWarps][kSelCand];
+    __shared__ int s_t[kSelWarps][kSelCand];
+    __shared__ float s_d[kSelWarps][4][kMaxNN]; // offsets by rank: x, y, z, 1
+    __shared__ int s_row[kSelWarps][9];
+    const int n = *O.over_count;
+    const KeyLayout L = *g.layout;
+    const int segshift = L.bx + L.by + L.bz;
+    const float rn2 = __fmul_rn(rn, rn);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    unsigned long long *key = s_key[warp];
+    int *cand = s_t[warp], *row0 = s_row[warp];
+    float(*off)[kMaxNN] = s_d[warp];
+    off[3][lane] = off[3][lane + 32] = 1.0f;
+    // this lane's moment is the sum of off[ma] * off[mb]: 1 with x, y, z; then the six products
+    const int ma = lane < 3 ? lane : (lane < 6 ? 0 : (lane < 8 ? 1 : 2));
+    const int mb = lane < 3 ? 3 : (lane < 6 ? lane - 3 : (lane < 8 ? lane - 5 : 2));
+    const int warps = gridDim.x * kSelWarps;
+    const int per = min(32, max(1, (n + warps - 1) / warps)); // points per warp before they are finished
+    for (int j0 = (blockIdx.x * kSelWarps + warp) * per; j0 < n; j0 += warps * per)
+    {
+        PointMoments M{};
+        for (int i = 0; i < per && j0 + i < n; ++i)
+        {
+            const int s = O.over_list[j0 + i];
+            const float4 p4 = g.spos[s];
+            const float3 p = make_float3(p4.x, p4.y, p4.z);
+            const int seg = L.bseg ? (int)(g.skey[s] >> segshift) : 0;
+            int cx, cy, cz;
+            grid_cell(g, L, g.gmin[seg], p, cx, cy, cz);
+            const int lo = cz - 1, hi = cz + 1;
+            // lane k < 9: the part of row k in the window, to within two points at either end
+            int2 r;
+            load_rows<1>(g, L, seg, lo, hi, &r, [&](int, int &x, int &y) {
+                x = cx + lane / 3 - 1, y = cy + lane % 3 - 1;
+                return lane < 9;
+            });
+            int len = 0;
+            if (r.x < r.y && GCA_INDEX_OK(r.x, *g.d_n, g.err) && GCA_INDEX_OK(r.y - 1, *g.d_n, g.err))
+            {
+                if (r.y - r.x > 4)
+                {
+                    r.x = row_seek_z(g.scz, r.x, r.y, lo);
+                    r.y = min(r.y, row_seek_z(g.scz, r.x, r.y, hi + 1) + 2);
+                }
+                len = r.y - r.x;
+            }
+            int end = len; // inclusive prefix over the rows
+#pragma unroll
+            for (int d = 1; d < 16; d <<= 1)
+            {
+                const int y = __shfl_up_sync(full, end, d);
+                if (lane >= d)
+                    end += y;
+            }
+            __syncwarp();
+            if (lane < 9)
+                row0[lane] = r.x - (end - len);
+            int ends[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                ends[k] = __shfl_sync(full, end, k);
+            const int total = __shfl_sync(full, end, 8);
+            __syncwarp();
+            int cnt = 0;
+            for (int c0 = 0; c0 < total; c0 += 32)
+            {
+                const int c = c0 + lane;
+                bool in = c < total;
+                int t = 0;
+                float d2 = 0.0f;
+                if (in)
+                {
+                    int k = 0;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        k += c >= ends[q];
+                    t = row0[k] + c;
+                    const float4 q = __ldg(&g.spos[t]);
+                    const int qz = __float_as_int(q.w);
+                    d2 = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
+                    in = qz >= lo && qz <= hi && d2 < rn2;
+                }
+                const unsigned m = __ballot_sync(full, in);
+                const int at = cnt + __popc(m & ((1u << lane) - 1u));
+                if (in && at < kSelCand)
+                {
+                    key[at] = (unsigned long long)__float_as_uint(d2) << 32 | (unsigned)__ldg(&g.sidx[t]);
+                    cand[at] = t;
+                }
+                cnt += __popc(m);
+            }
+            __syncwarp();
+            const int keep = min(cnt, max_nn);
+            float v = 0.0f;
+            if (cnt <= kSelCand)
+            {
+                for (int c = lane; c < cnt; c += 32)
+                {
+                    const unsigned long long mine = key[c];
+                    int rank = 0;
+#pragma unroll 4
+                    for (int o = 0; o < cnt; ++o)
+                        rank += key[o] < mine;
+                    if (rank < max_nn)
+                    {
+                        const float4 q = __ldg(&g.spos[cand[c]]);
+                        off[0][rank] = q.x - p.x, off[1][rank] = q.y - p.y, off[2][rank] = q.z - p.z;
+                    }
+                }
+                __syncwarp();
+                if (lane < 9)
+#pragma unroll 4
+                    for (int o = 0; o < keep; ++o)
+                        v = fmaf(off[ma][o], off[mb][o], v); // times 1: the sum of an addition
+            }
+            else
+            {
+                NbrEntry list[kMaxNN];
+                GridRows R;
+                if (lane == 0)
+                {
+                    grid_rows(g, L, seg, g.gmin[seg], p, R);
+                    select_knn(g, R, p, rn2, max_nn, list);
+                    for (int o = 0; o < keep; ++o)
+                    {
+                        const float4 q = __ldg(&g.spos[list[o].t]);
+                        off[0][o] = q.x - p.x, off[1][o] = q.y - p.y, off[2][o] = q.z - p.z;
+                    }
+                }
+                __syncwarp();
+                if (lane < 9)
+                    for (int o = 0; o < keep; ++o)
+                        v = fmaf(off[ma][o], off[mb][o], v);
+            }
+            float sum[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q)
+                sum[q] = __shfl_sync(full, v, q);
+            if (lane == i)
+            {
+                M.s1x = sum[0], M.s1y = sum[1], M.s1z = sum[2], M.sxx = sum[3], M.sxy = sum[4], M.sxz = sum[5];
+                M.syy = sum[6], M.syz = sum[7], M.szz = sum[8], M.k = keep;
+            }
+        }
+        const int j = j0 + lane;
+        if (lane < per && j < n)
+        {
+            if (Grad)
+            {
+                const float4 a = O.over_mom[3 * j], b = O.over_mom[3 * j + 1], c = O.over_mom[3 * j + 2];
+                M.gxx = a.x, M.gxy = a.y, M.gxz = a.z, M.gyy = a.w, M.gyz = b.x, M.gzz = b.y;
+                M.mx = b.z, M.my = b.w, M.mz = c.x, M.gk = __float_as_int(c.y);
+            }
+            const int s = O.over_list[j];
+            finish_point(g.sidx, O, s, g.sint[s], M, Grad);
+        }
+        __syncwarp();
     }
 }
 
@@ -763,16 +945,20 @@ int normals_stage(gca3d_context *ctx, const Batch &b, const Grid &g, bool do_nor
         NormalOut O;
         O.attr0 = attr0;
         O.nrm_out = nrm_out;
-        O.degen_count = ctx->arena.get<int>(1);
+        O.degen_count = ctx->arena.get<int>(2);
         O.degen_list = ctx->arena.get<int>(std::max<int64_t>(g.cap, 1));
         // the gradients in the same walk
         O.grad_r2 = do_grad ? grad_radius * grad_radius : 0.0f;
         O.attr1 = do_grad ? attr1 : nullptr;
         O.grd_out = do_grad ? grd_out : nullptr;
         O.degen_mom = do_grad ? ctx->arena.get<float4>(3 * (size_t)std::max<int64_t>(g.cap, 1)) : nullptr;
-        if (!O.degen_count || !O.degen_list || (do_grad && !O.degen_mom))
+        O.over_count = O.degen_count + 1;
+        O.over_list = max_nn > 0 ? ctx->arena.get<int>(std::max<int64_t>(g.cap, 1)) : nullptr;
+        O.over_mom = max_nn > 0 && do_grad ? ctx->arena.get<float4>(3 * (size_t)std::max<int64_t>(g.cap, 1)) : nullptr;
+        if (!O.degen_count || !O.degen_list || (do_grad && !O.degen_mom) || (max_nn > 0 && !O.over_list) ||
+            (max_nn > 0 && do_grad && !O.over_mom))
             return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "normals: scratch");
-        GCA_CUDA(ctx, cudaMemsetAsync(O.degen_count, 0, sizeof(int), ctx->stream));
+        GCA_CUDA(ctx, cudaMemsetAsync(O.degen_count, 0, 2 * sizeof(int), ctx->stream));
         // equal radii (the usual case): the gradient's second moments are the normal's
         if (do_grad && O.grad_r2 == normal_radius * normal_radius)
             k_normals32<true, true><<<gs, 256, 0, ctx->stream>>>(g.dev, d_n, normal_radius, max_nn, O);
@@ -781,6 +967,14 @@ int normals_stage(gca3d_context *ctx, const Batch &b, const Grid &g, bool do_nor
         else
             k_normals32<false, false><<<gs, 256, 0, ctx->stream>>>(g.dev, d_n, normal_radius, max_nn, O);
         GCA_CHECK_LAUNCH(ctx);
+        if (max_nn > 0)
+        {
+            if (do_grad)
+                k_normals_select<true><<<ctx->num_sms * 8, 32 * kSelWarps, 0, ctx->stream>>>(g.dev, normal_radius, max_nn, O);
+            else
+                k_normals_select<false><<<ctx->num_sms * 8, 32 * kSelWarps, 0, ctx->stream>>>(g.dev, normal_radius, max_nn, O);
+            GCA_CHECK_LAUNCH(ctx);
+        }
         // one warp per queued point and a long dependent FP64 chain per point: as many
         // resident blocks as the registers allow, to overlap the chains
         static const int blocks64 = [] {

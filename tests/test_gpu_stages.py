@@ -372,6 +372,40 @@ def test_normals_vs_f64(ctx, orc, room_v01, max_nn):
     np.testing.assert_allclose(np.linalg.norm(n[ok], axis=1), 1.0, atol=1e-5)
 
 
+@pytest.mark.parametrize("max_nn", [3, 31, 32, 33, 64])
+@pytest.mark.parametrize("density", [300, 3000])
+def test_capped_normals_vs_f64(ctx, max_nn, density):
+    """neighbourhoods around and far above the cap, within the selection pass's shared list
+    (256) and beyond it; repeated points make ties that the index decides.  The FP64 normal of
+    the max_nn nearest (FP32 distance, then index) is defined up to the gap between its two
+    smallest eigenvalues: FP32 sums of a few dozen terms (about 30 roundings of 2^-24 of the
+    largest entry) turn it by at most 2e-6 / relative gap, and a repeated triple (gap zero)
+    has none"""
+    rng = np.random.default_rng(density + max_nn)
+    uv = rng.random((density, 2)) * 0.1
+    xyz = np.stack([uv[:, 0], uv[:, 1], 0.5 * uv[:, 0] ** 2 + 0.02 * rng.random(density)], 1).astype(np.float32)
+    xyz = np.concatenate([xyz, xyz[:: 7]])
+    radius = np.float32(0.04)
+    d2 = np.zeros((len(xyz), len(xyz)), np.float32)
+    for k in range(3):
+        d = xyz[None, :, k] - xyz[:, None, k]
+        d2 += d * d
+    near = np.argsort(d2, axis=1, kind="stable")[:, :max_nn]
+    inside = np.take_along_axis(d2, near, 1) < radius * radius
+    assert inside.all(1).mean() > 0.9
+    n = normals_gpu(ctx, xyz, radius, max_nn).astype(np.float64)
+    off = xyz[near].astype(np.float64) - xyz[:, None].astype(np.float64)
+    w = inside[..., None] / inside.sum(1)[:, None, None]
+    mu = (off * w).sum(1)
+    cov = np.einsum("nki,nkj->nij", off * w, off) - mu[:, :, None] * mu[:, None, :]
+    val, vec = np.linalg.eigh(cov)
+    gap = (val[:, 1] - val[:, 0]) / np.maximum(val[:, 2] - val[:, 0], 1e-30)
+    ok = (inside.sum(1) >= 3) & (gap > 1e-5)
+    assert ok.mean() > 0.5 # the repeated points of a triple have no normal
+    err = np.linalg.norm(np.cross(n[ok], vec[ok][:, :, 0]), axis=1)
+    assert (err <= 2e-6 / gap[ok]).all(), (err * gap[ok]).max()
+
+
 def test_degenerate_normals_vs_f64(ctx, orc):
     """Points on thin noisy lines: the two smallest eigenvalues of every
     neighbourhood are close, so the FP32 pass queues them and every normal comes
