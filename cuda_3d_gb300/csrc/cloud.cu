@@ -419,6 +419,8 @@ int gca3d_destroy(gca3d_context *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream)
         cudaStreamSynchronize(ctx->stream);
+    if (ctx->spare)
+        gca3d_icp_plan_destroy(ctx->spare);
     ctx->arena.release();
     for (auto e : ctx->prof.events)
         cudaEventDestroy(e);

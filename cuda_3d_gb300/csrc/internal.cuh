@@ -69,6 +69,13 @@ struct Arena
         failed = false;
     }
     void release();
+    size_t bytes() const
+    {
+        size_t n = 0;
+        for (auto &c : chunks)
+            n += c.size;
+        return n;
+    }
     void swap(Arena &o)
     {
         chunks.swap(o.chunks);
@@ -126,6 +133,8 @@ struct gca3d_context
     int64_t launches = 0;
     std::string last_error;
     gca3d::Profiler prof;
+    // the workspace of the last one-shot registration, kept for the next (schedule.cu)
+    gca3d_icp_plan *spare = nullptr;
 };
 
 struct gca3d_cloud

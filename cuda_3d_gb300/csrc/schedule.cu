@@ -36,7 +36,10 @@ struct gca3d_icp_plan
     int P = 0;
     std::vector<gca3d_cloud *> src, tgt;
     gca3d_icp_params prm{};
+    // workspace (plan_workspace): kept when a one-shot call's plan serves the next call
+    int pair_cap = 0; // pairs that the tables hold
     Arena arena;
+    SegSrc *h_src = nullptr; // pinned: sources, then targets
     SegSrc *d_src = nullptr, *d_tgt = nullptr;
     PairState *d_state = nullptr;
     PairState *h_state = nullptr;
@@ -74,6 +77,7 @@ struct gca3d_icp_plan
     // next execute (of this or another plan) may be queued before the results are read
     cudaEvent_t states_ready = nullptr;
     bool states_pending = false;
+    cudaEvent_t states_checked = nullptr; // plain mode: an iteration's states are on the host
     int *h_err = nullptr;
 };
 
@@ -98,15 +102,6 @@ int validate_params(gca3d_context *ctx, const gca3d_icp_params *p)
         if (need_normals && !(S.normal_radius > 0.0f))
             return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: normal radius must be > 0");
     }
-    return GCA3D_OK;
-}
-
-int read_states(gca3d_icp_plan *pl)
-{
-    gca3d_context *ctx = pl->ctx;
-    GCA_CUDA(ctx, cudaMemcpyAsync(pl->h_state, pl->d_state, sizeof(PairState) * pl->P, cudaMemcpyDeviceToHost,
-                                  ctx->stream));
-    GCA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return GCA3D_OK;
 }
 
@@ -446,21 +441,29 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
                 if ((st = icp_update(ctx, bs, gicp, attr0, attr1, pl->d_state, bmap, pl->max_blocks, bmap_nn,
                                      partials, corr, prm, p.compensated != 0, loop, shape)))
                     return st;
-                if (pl->host_checks && !capturing)
+                // the next search is queued before the step is inspected on the host (the
+                // reference's control flow), which then waits for the states alone; once
+                // every pair has converged it finds no work
+                const bool check = pl->host_checks && !capturing;
+                if (check)
                 {
-                    // the reference's control flow: the step is inspected on the host
-                    if ((st = read_states(pl)))
-                        return st;
+                    GCA_CUDA(ctx, cudaMemcpyAsync(pl->h_state, pl->d_state, sizeof(PairState) * P,
+                                                  cudaMemcpyDeviceToHost, ctx->stream));
+                    GCA_CUDA(ctx, cudaEventRecord(pl->states_checked, ctx->stream));
+                }
+                if (it + 1 < S.max_iter &&
+                    (st = icp_search(ctx, bs, gicp, pl->d_state, bmap_nn, pl->max_blocks_nn, corr, cert, prm,
+                                     nullptr, nullptr, shape, false)))
+                    return st;
+                if (check)
+                {
+                    GCA_CUDA(ctx, cudaEventSynchronize(pl->states_checked));
                     bool any = false;
                     for (int k = 0; k < P; ++k)
                         any |= pl->h_state[k].active != 0;
                     if (!any)
                         break;
                 }
-                if (it + 1 < S.max_iter &&
-                    (st = icp_search(ctx, bs, gicp, pl->d_state, bmap_nn, pl->max_blocks_nn, corr, cert, prm,
-                                     nullptr, nullptr, shape, false)))
-                    return st;
             }
         }
 
@@ -558,6 +561,10 @@ int gca3d_icp_plan_destroy(gca3d_icp_plan *pl)
     cudaFree(pl->d_tgt);
     cudaFree(pl->d_state);
     cudaFree(pl->d_Tinit);
+    if (pl->h_src)
+        cudaFreeHost(pl->h_src);
+    if (pl->states_checked)
+        cudaEventDestroy(pl->states_checked);
     if (pl->h_state)
         cudaFreeHost(pl->h_state);
     if (pl->h_Tinit)
@@ -569,9 +576,57 @@ int gca3d_icp_plan_destroy(gca3d_icp_plan *pl)
 
 } // extern "C"
 
+// the tables, streams and events a plan of pl->P pairs and its scales needs: what is missing
+// is made, what is there is kept
+static int plan_workspace(gca3d_icp_plan *pl, bool capture)
+{
+    gca3d_context *ctx = pl->ctx;
+    const int P = pl->P;
+    if (pl->pair_cap < P)
+    {
+        if (cudaMallocHost(&pl->h_src, sizeof(SegSrc) * 2 * P) != cudaSuccess ||
+            cudaMalloc(&pl->d_src, sizeof(SegSrc) * P) != cudaSuccess ||
+            cudaMalloc(&pl->d_tgt, sizeof(SegSrc) * P) != cudaSuccess ||
+            cudaMalloc(&pl->d_state, sizeof(PairState) * P) != cudaSuccess ||
+            cudaMalloc(&pl->d_Tinit, sizeof(double) * 16 * P) != cudaSuccess ||
+            cudaMallocHost(&pl->h_state, sizeof(PairState) * P) != cudaSuccess ||
+            cudaMallocHost(&pl->h_err, sizeof(int)) != cudaSuccess ||
+            cudaMallocHost(&pl->h_Tinit, sizeof(double) * 16 * P) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "icp plan: allocation");
+        }
+        pl->pair_cap = P;
+    }
+    if (capture && !pl->side && cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return fail(ctx, GCA3D_ERR_CUDA, "icp plan: side stream");
+    }
+    int least_prio = 0;
+    if (cudaDeviceGetStreamPriorityRange(&least_prio, &pl->priority) != cudaSuccess)
+        pl->priority = 0;
+    auto stream = [](cudaStream_t &s) {
+        return s || cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+    };
+    auto event = [](cudaEvent_t &e) {
+        return e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    };
+    bool ok = stream(pl->prep) && stream(pl->prep_src) && event(pl->ev_fork) && event(pl->ev_fork_src) &&
+              event(pl->states_checked);
+    for (int k = 0; k < pl->prm.n_scales && ok; ++k)
+        ok = event(pl->ev_scale[k]) && event(pl->ev_grid[k]) && event(pl->ev_src[k]);
+    if (!ok)
+    {
+        cudaGetLastError();
+        return fail(ctx, GCA3D_ERR_CUDA, "icp plan: preparation stream");
+    }
+    return GCA3D_OK;
+}
+
 int gca3d::icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *const *src, gca3d_cloud *const *tgt,
                                     const gca3d_icp_params *params, bool capture, PlanPrologue prologue,
-                                    gca3d_icp_plan **out, const PlanVoxels *voxels)
+                                    gca3d_icp_plan **out, const PlanVoxels *voxels, gca3d_icp_plan *reuse)
 {
     if (!ctx || !out || P < 1 || P > kMaxSegments || !src || !tgt)
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: bad arguments (1 <= pairs <= 4096)");
@@ -586,9 +641,13 @@ int gca3d::icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *cons
         if (params->keep_target_normals && params->scales[0].voxel <= 0.0f && !tgt[k]->has_normals)
             return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: the target has no normals (estimate normals first)");
     }
-    auto *pl = new gca3d_icp_plan();
+    // (reuse: a retired plan whose workspace serves this one; the caller has taken it, and it
+    // is destroyed with this one on failure)
+    auto *pl = reuse ? reuse : new gca3d_icp_plan();
     pl->ctx = ctx;
     pl->P = P;
+    pl->src_cap = pl->tgt_cap = pl->src_max = pl->tgt_max = 0;
+    pl->max_blocks_nn = 0;
     pl->src.assign(src, src + P);
     pl->tgt.assign(tgt, tgt + P);
     pl->prm = *params;
@@ -622,57 +681,32 @@ int gca3d::icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *cons
     }
     pl->max_blocks = std::max(nb, 1);
     pl->max_blocks_nn = std::max(pl->max_blocks_nn, 1);
-    // device tables and state live outside the scratch arena
-    std::vector<SegSrc> hs(P), ht(P);
+    if ((st = plan_workspace(pl, capture)))
+    {
+        gca3d_icp_plan_destroy(pl);
+        return st;
+    }
     for (int k = 0; k < P; ++k)
     {
-        hs[k] = SegSrc{src[k]->pos, src[k]->col, nullptr, src[k]->d_count};
-        ht[k] = SegSrc{tgt[k]->pos, tgt[k]->col, tgt[k]->has_normals ? tgt[k]->nrm : nullptr, tgt[k]->d_count};
+        pl->h_src[k] = SegSrc{src[k]->pos, src[k]->col, nullptr, src[k]->d_count};
+        pl->h_src[P + k] = SegSrc{tgt[k]->pos, tgt[k]->col, tgt[k]->has_normals ? tgt[k]->nrm : nullptr, tgt[k]->d_count};
     }
-    if (cudaMalloc(&pl->d_src, sizeof(SegSrc) * P) != cudaSuccess ||
-        cudaMalloc(&pl->d_tgt, sizeof(SegSrc) * P) != cudaSuccess ||
-        cudaMalloc(&pl->d_state, sizeof(PairState) * P) != cudaSuccess ||
-        cudaMalloc(&pl->d_Tinit, sizeof(double) * 16 * P) != cudaSuccess ||
-        cudaMallocHost(&pl->h_state, sizeof(PairState) * P) != cudaSuccess ||
-        cudaMallocHost(&pl->h_err, sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&pl->h_Tinit, sizeof(double) * 16 * P) != cudaSuccess)
-    {
-        cudaGetLastError();
-        gca3d_icp_plan_destroy(pl);
-        return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "icp plan: allocation");
-    }
-    cudaMemcpy(pl->d_src, hs.data(), sizeof(SegSrc) * P, cudaMemcpyHostToDevice);
-    cudaMemcpy(pl->d_tgt, ht.data(), sizeof(SegSrc) * P, cudaMemcpyHostToDevice);
+    // (a one-shot call's copies are behind the previous call's, which it waited for)
+    cudaError_t ce = cudaMemcpyAsync(pl->d_src, pl->h_src, sizeof(SegSrc) * P, cudaMemcpyHostToDevice, ctx->stream);
+    if (ce == cudaSuccess)
+        ce = cudaMemcpyAsync(pl->d_tgt, pl->h_src + P, sizeof(SegSrc) * P, cudaMemcpyHostToDevice, ctx->stream);
     for (int k = 0; k < P; ++k)
         for (int j = 0; j < 16; ++j)
             pl->h_Tinit[16 * k + j] = (j % 5 == 0) ? 1.0 : 0.0;
-    cudaMemcpy(pl->d_Tinit, pl->h_Tinit, sizeof(double) * 16 * P, cudaMemcpyHostToDevice);
-    if (capture && cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking) != cudaSuccess)
+    if (ce == cudaSuccess && capture) // the warm-up run's; every execute copies its own
+        ce = cudaMemcpyAsync(pl->d_Tinit, pl->h_Tinit, sizeof(double) * 16 * P, cudaMemcpyHostToDevice, ctx->stream);
+    if (ce == cudaSuccess && capture)
+        ce = cudaStreamSynchronize(ctx->stream);
+    if (ce != cudaSuccess)
     {
-        cudaGetLastError();
+        st = cuda_fail(ctx, ce, "icp plan: tables");
         gca3d_icp_plan_destroy(pl);
-        return fail(ctx, GCA3D_ERR_CUDA, "icp plan: side stream");
-    }
-    int least_prio = 0;
-    if (cudaDeviceGetStreamPriorityRange(&least_prio, &pl->priority) != cudaSuccess)
-        pl->priority = 0;
-    bool events_ok = cudaStreamCreateWithFlags(&pl->prep, cudaStreamNonBlocking) == cudaSuccess &&
-                     cudaEventCreateWithFlags(&pl->ev_fork, cudaEventDisableTiming) == cudaSuccess;
-    for (int k = 0; k < params->n_scales && events_ok; ++k)
-        events_ok = cudaEventCreateWithFlags(&pl->ev_scale[k], cudaEventDisableTiming) == cudaSuccess &&
-                    cudaEventCreateWithFlags(&pl->ev_grid[k], cudaEventDisableTiming) == cudaSuccess;
-    if (events_ok)
-    {
-        events_ok = cudaStreamCreateWithFlags(&pl->prep_src, cudaStreamNonBlocking) == cudaSuccess &&
-                    cudaEventCreateWithFlags(&pl->ev_fork_src, cudaEventDisableTiming) == cudaSuccess;
-        for (int k = 0; k < params->n_scales && events_ok; ++k)
-            events_ok = cudaEventCreateWithFlags(&pl->ev_src[k], cudaEventDisableTiming) == cudaSuccess;
-    }
-    if (!events_ok)
-    {
-        cudaGetLastError();
-        gca3d_icp_plan_destroy(pl);
-        return fail(ctx, GCA3D_ERR_CUDA, "icp plan: preparation stream");
+        return st;
     }
     if (capture)
     {
@@ -819,12 +853,27 @@ int gca3d_color_icp_batched(gca3d_context *ctx, int n_pairs, gca3d_cloud *const 
 {
     if (!results)
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: results needed");
-    gca3d_icp_plan *pl = nullptr;
-    int st = icp_plan_create_internal(ctx, n_pairs, src, tgt, params, false, nullptr, &pl);
+    // the last one-shot call's workspace (scratch, tables, streams, events) when it holds
+    // enough pairs: making and freeing one took 270 us of a 64k-point alignment's 570
+    gca3d_icp_plan *spare = ctx ? ctx->spare : nullptr, *pl = nullptr;
+    if (spare && spare->pair_cap < n_pairs)
+        spare = nullptr;
+    int st = icp_plan_create_internal(ctx, n_pairs, src, tgt, params, false, nullptr, &pl, nullptr, spare);
+    if (spare && pl != spare && st == GCA3D_ERR_INVALID_VALUE)
+        return st; // refused before the workspace was touched
+    if (spare)
+        ctx->spare = nullptr; // in use, or destroyed with the failed plan
     if (st)
         return st;
     st = gca3d_icp_plan_execute(pl, T_init, results);
-    gca3d_icp_plan_destroy(pl);
+    // one is kept per context, up to 256 MB of scratch; gca3d_destroy frees it
+    if (!st && !ctx->spare && pl->arena.bytes() <= (size_t(256) << 20))
+    {
+        ctx->spare = pl;
+        pl->prologue = nullptr;
+    }
+    else
+        gca3d_icp_plan_destroy(pl);
     return st;
 }
 

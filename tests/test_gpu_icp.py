@@ -122,6 +122,38 @@ def test_batched_bit_identical_to_single(ctx, N, synth):
         assert single["fitness"] == b["fitness"]
 
 
+def test_one_shot_calls_share_a_workspace(N, synth):
+    """one context's one-shot calls reuse one workspace: sizes, pair counts and scales that
+    grow and shrink, a refused call and a call without correspondences in between give the
+    bits of a fresh context each"""
+    pairs = [synth.room_pair(seed=40 + k, n_points=n, rot_deg=2.0, trans=0.02)
+             for k, n in enumerate((4_000, 20_000, 9_000))]
+    two = [N.scale(0.1, 10, 0.2, 0.2, 0.2), N.scale(0.05, 10, 0.1, 0.1, 0.1)]
+    one = [N.scale(0.06, 15, 0.12, 0.12, 0.12)]
+    calls = [((0,), one), ((1,), two), ((0, 1, 2), two), ((2,), one), ((1, 0), one), ((0,), two)]
+
+    def run(c, which, scales):
+        s = [c.cloud_from(pairs[k].src_xyz, pairs[k].src_rgb) for k in which]
+        t = [c.cloud_from(pairs[k].tgt_xyz, pairs[k].tgt_rgb) for k in which]
+        return N.color_icp_batched(c, s, t, N.icp_params(scales))
+
+    shared = N.Context(0)
+    for k, (which, scales) in enumerate(calls):
+        got = run(shared, which, scales)
+        want = run(N.Context(0), which, scales)
+        for a, b in zip(got, want):
+            assert a["status"] == N.OK and a["scale_iterations"] == b["scale_iterations"]
+            np.testing.assert_array_equal(a["T"], b["T"])
+        if k == 1:
+            with pytest.raises(N.GcaError):
+                run(shared, (0,), [N.scale(0.1, 10, -1.0, 0.2, 0.2)])
+        if k == 3:
+            far = shared.cloud_from(pairs[0].src_xyz + 50.0, pairs[0].src_rgb)
+            tgt = shared.cloud_from(pairs[0].tgt_xyz, pairs[0].tgt_rgb)
+            r = N.color_icp(shared, far, tgt, N.icp_params(one))
+            assert r["status"] == N.ERR_NO_CORRESPONDENCES
+
+
 def test_plan_graph_replay(ctx, N, synth):
     pairs = make_batch(synth, k=4, seed=1)
     srcs = [ctx.cloud_from(p.src_xyz, p.src_rgb) for p in pairs]
