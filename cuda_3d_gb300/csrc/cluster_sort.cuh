@@ -29,16 +29,18 @@ constexpr int kClusterWarps = kClusterThreads / 32;
 constexpr int kClusterRounds = 13; // words per thread: 26 registers of the 64 there are
 constexpr int kClusterWordBits = 54; // of a word; a pass keeps its rank within the warp above them
 constexpr int64_t kClusterCap = (int64_t)kClusterBlocks * kClusterThreads * kClusterRounds; // 212,992
-constexpr int kClusterDigit = 9; // bits of the widest digit
+constexpr int kClusterDigit = 10; // bits of the widest digit: 20 bits of key take two passes, 30 three
 constexpr int kClusterBins = 1 << kClusterDigit;
+static_assert(kClusterThreads * kClusterRounds < 65536 && kClusterBins <= kClusterThreads,
+              "16-bit counts, a thread per bin");
 
-// shared memory of a block: its words, its warps' digit counts (16 bits each) and every
-// block's digit counts
+// shared memory of a block: its words, its warps' digit counts and every block's digit
+// counts (16 bits each)
 inline size_t cluster_smem(int64_t cap)
 {
     const size_t words = (size_t)((cap + kClusterBlocks - 1) / kClusterBlocks);
     return words * sizeof(uint64_t) + sizeof(uint16_t) * kClusterWarps * kClusterBins +
-           sizeof(uint32_t) * kClusterBlocks * kClusterBins;
+           sizeof(uint16_t) * kClusterBlocks * kClusterBins;
 }
 
 // where a cluster sort leaves its results; d_starts .. d_count may be null (no runs wanted)
@@ -125,7 +127,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ uint64_t s_words[];
     uint16_t *s_whist = reinterpret_cast<uint16_t *>(s_words + words); // [warp][bin]
-    uint32_t *s_count = reinterpret_cast<uint32_t *>(s_whist + kClusterWarps * kClusterBins); // [block][bin]
+    uint16_t *s_count = s_whist + kClusterWarps * kClusterBins; // [block][bin]
     __shared__ float s_bound[kClusterBlocks][6];
     __shared__ float s_red[kClusterWarps][6];
     __shared__ uint32_t s_scan[kClusterWarps];
@@ -249,7 +251,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
             for (int i = tid; i < kClusterWarps * bins / 2; i += kClusterThreads)
                 reinterpret_cast<uint32_t *>(s_whist)[i] = 0u;
             __syncthreads();
-            if (width == 9)
+            if (width == 10)
+                cluster_rank<10>(s_words, hist, e0, cnt, rounds, lo, mask);
+            else if (width == 9)
                 cluster_rank<9>(s_words, hist, e0, cnt, rounds, lo, mask);
             else if (width == 8)
                 cluster_rank<8>(s_words, hist, e0, cnt, rounds, lo, mask);
@@ -267,9 +271,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
                     s_whist[w * bins + tid] = (uint16_t)mine;
                     mine += c;
                 }
-                uint32_t *slot = s_count + rank * kClusterBins + tid;
+                uint16_t *slot = s_count + rank * kClusterBins + tid;
                 for (int b = 0; b < kClusterBlocks; ++b)
-                    *cluster.map_shared_rank(slot, b) = mine;
+                    *cluster.map_shared_rank(slot, b) = (uint16_t)mine;
             }
             const uint32_t local = block_exclusive(mine, s_scan);
             if (tid < bins)
