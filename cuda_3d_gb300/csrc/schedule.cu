@@ -59,6 +59,10 @@ struct gca3d_icp_plan
     cudaEvent_t ev_fork = nullptr;
     cudaEvent_t ev_scale[GCA3D_MAX_SCALES] = {};
     cudaEvent_t ev_grid[GCA3D_MAX_SCALES] = {}; // the scale's search grid is built (before its normals)
+    // the normals' branch of small workloads: the normals' grid, normals and gradients
+    cudaStream_t prep_nrm = nullptr;
+    cudaEvent_t ev_tgt[GCA3D_MAX_SCALES] = {}; // the scale's target cloud is there
+    cudaEvent_t ev_join = nullptr;
     // the source preparation's branch (the first scale's; every scale's in a tracker plan,
     // where the prologue makes the new frame and the target is the previous one)
     cudaStream_t prep_src = nullptr;
@@ -136,11 +140,12 @@ struct ScalePrep
 };
 
 // one scale's clouds, grids, normals, gradients and iteration scratch, enqueued on the
-// context stream (the source's on src_stream; grid_ready, if given, recorded once the
-// search grid is built); none of it depends on the pose, so it can run ahead of the
-// iterations
+// context stream (the source's on src_stream, the normals and gradients on nrm_stream;
+// tgt_ready and grid_ready, if given, recorded once the target cloud and the search grid are
+// there); none of it depends on the pose, so it can run ahead of the iterations
 static int prepare_scale(gca3d_icp_plan *pl, int si, VoxelChain &chain_src, VoxelChain &chain_tgt, ScalePrep &out,
-                         cudaStream_t src_stream, cudaEvent_t grid_ready)
+                         cudaStream_t src_stream, cudaStream_t nrm_stream, cudaEvent_t tgt_ready,
+                         cudaEvent_t grid_ready)
 {
     gca3d_context *ctx = pl->ctx;
     const gca3d_icp_params &p = pl->prm;
@@ -198,13 +203,27 @@ static int prepare_scale(gca3d_icp_plan *pl, int si, VoxelChain &chain_src, Voxe
         cell_n = std::max(cell_n, S.normal_radius);
     const bool own_nn_grid = S.max_corr < 0.9f * cell_n;
     Grid g, gnn;
-    if ((st = grid_build(ctx, bt, std::max(cell_n, own_nn_grid ? 0.0f : S.max_corr), kOriginPadF32, nullptr, g)))
-        return st;
-    if (own_nn_grid && (st = grid_build(ctx, bt, S.max_corr, kOriginPadF32, nullptr, gnn)))
+    cudaStream_t tgt_stream = ctx->stream;
+    const bool fork = nrm_stream != tgt_stream;
+    if (own_nn_grid)
+    {
+        // the two grids side by side when the normals have a branch
+        if (fork)
+        {
+            GCA_CUDA(ctx, cudaEventRecord(tgt_ready, tgt_stream));
+            GCA_CUDA(ctx, cudaStreamWaitEvent(nrm_stream, tgt_ready, 0));
+        }
+        ctx->stream = nrm_stream;
+        st = grid_build(ctx, bt, cell_n, kOriginPadF32, nullptr, g);
+        ctx->stream = tgt_stream;
+        if (st || (st = grid_build(ctx, bt, S.max_corr, kOriginPadF32, nullptr, gnn)))
+            return st;
+    }
+    else if ((st = grid_build(ctx, bt, std::max(cell_n, S.max_corr), kOriginPadF32, nullptr, g)))
         return st;
     out.gicp = own_nn_grid ? gnn : g;
     if (grid_ready) // the first correspondence search needs the grid, not the normals
-        GCA_CUDA(ctx, cudaEventRecord(grid_ready, ctx->stream));
+        GCA_CUDA(ctx, cudaEventRecord(grid_ready, tgt_stream));
     float4 *attr0 = out.attr0 = ctx->arena.get<float4>(g.cap);
     float4 *attr1 = out.attr1 = ctx->arena.get<float4>(g.cap);
     double *partials = out.partials = ctx->arena.get<double>((size_t)std::max(pl->max_blocks, 1) * kTermsPad);
@@ -217,18 +236,34 @@ static int prepare_scale(gca3d_icp_plan *pl, int si, VoxelChain &chain_src, Voxe
     float4 *grd_b = own_nn_grid ? ctx->arena.get<float4>(g.cap) : nullptr;
     if (!attr0 || !attr1 || !partials || !corr || !cert.pos || !cert.t || !bmap || !bmap_nn || (own_nn_grid && (!grd_b || (!keep && !nrm_b))))
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "icp: scratch");
+    ctx->stream = nrm_stream;
     if (own_nn_grid)
     {
-        if ((st = normals_stage(ctx, bt, g, !keep, S.normal_radius, S.max_nn, true, S.grad_radius,
-                                keep ? bt.nrm : nullptr, nullptr, nullptr, nrm_b, grd_b)))
-            return st;
-        if ((st = gather_attrs(ctx, bt, gnn, keep ? bt.nrm : nrm_b, grd_b, attr0, attr1)))
-            return st;
+        st = normals_stage(ctx, bt, g, !keep, S.normal_radius, S.max_nn, true, S.grad_radius, keep ? bt.nrm : nullptr,
+                           nullptr, nullptr, nrm_b, grd_b);
+        if (!st && fork) // the records go into the search grid's order
+        {
+            const cudaError_t e = cudaStreamWaitEvent(nrm_stream, grid_ready, 0);
+            if (e != cudaSuccess)
+                st = cuda_fail(ctx, e, "icp: preparation event");
+        }
+        if (!st)
+            st = gather_attrs(ctx, bt, gnn, keep ? bt.nrm : nrm_b, grd_b, attr0, attr1);
     }
-    else if ((st = normals_stage(ctx, bt, g, !keep, S.normal_radius, S.max_nn, true, S.grad_radius,
-                                 keep ? bt.nrm : nullptr, attr0, attr1, nullptr, nullptr)))
-        return st;
-    return GCA3D_OK;
+    else
+    {
+        if (fork)
+        {
+            const cudaError_t e = cudaStreamWaitEvent(nrm_stream, grid_ready, 0);
+            if (e != cudaSuccess)
+                st = cuda_fail(ctx, e, "icp: preparation event");
+        }
+        if (!st)
+            st = normals_stage(ctx, bt, g, !keep, S.normal_radius, S.max_nn, true, S.grad_radius,
+                               keep ? bt.nrm : nullptr, attr0, attr1, nullptr, nullptr);
+    }
+    ctx->stream = tgt_stream;
+    return st;
 }
 
 // give every kernel node of a graph the launch priority prio
@@ -276,12 +311,27 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
     const bool tracker = !serial && pl->vox_given && pl->prologue;
     cudaStream_t prep = serial ? main_stream : pl->prep;
     cudaStream_t prep_src = serial ? main_stream : pl->prep_src;
-    auto src_branch = [&](int si) { return !serial && (tracker || si == 0); };
+    // A small workload's preparation is a chain of short launches that leave the GPU idle, so
+    // it gets more branches: every scale's source beside the targets, and the normals (their
+    // grid, the walk, the gradients) beside the search grids.  Three scales, us per execute
+    // without and with them, by the points of all clouds: 0.5 M (one pair of 250k) 974, 871;
+    // 0.8 M 1357, 1241; 1.6 M 1939, 1870; 2.6 M 4835, 4822; 3.2 M 2750, 2746.  From there the
+    // launches fill the GPU and the branches get into each other's way: 6.4 M 4680, 4743;
+    // 12.8 M 8660, 8950; 64 pairs of 20k to 300k 11,670, 12,000.
+    constexpr int64_t kWidePoints = 1 << 21;
+    const bool wide = !serial && pl->src_cap + pl->tgt_cap <= kWidePoints;
+    cudaStream_t prep_nrm = wide ? pl->prep_nrm : prep;
+    auto src_branch = [&](int si) { return !serial && (tracker || wide || si == 0); };
     int st = GCA3D_OK;
     auto join = [&](int last) {
         // join the branches before giving up (a capture must end on one stream)
         if (serial)
             return;
+        if (wide && last >= 0)
+        {
+            cudaEventRecord(pl->ev_join, prep_nrm);
+            cudaStreamWaitEvent(prep, pl->ev_join, 0);
+        }
         cudaEventRecord(pl->ev_fork, prep);
         cudaStreamWaitEvent(main_stream, pl->ev_fork, 0);
         if (last >= 0)
@@ -313,6 +363,12 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
         GCA_CUDA(ctx, cudaStreamWaitEvent(prep_src, pl->ev_fork_src, 0));
         if (!tracker)
             GCA_CUDA(ctx, cudaStreamWaitEvent(prep, pl->ev_fork_src, 0));
+        if (wide)
+        {
+            // (in a tracker plan it follows the target's branch, which forked earlier)
+            GCA_CUDA(ctx, cudaEventRecord(pl->ev_join, tracker ? prep : main_stream));
+            GCA_CUDA(ctx, cudaStreamWaitEvent(prep_nrm, pl->ev_join, 0));
+        }
     }
     ScalePrep sp[GCA3D_MAX_SCALES];
     {
@@ -321,7 +377,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
         for (int si = 0; si < p.n_scales && !st; ++si)
         {
             // a finer scale's source continues the first scale's sorted state
-            if (!serial && !tracker && si == 1)
+            if (!serial && !tracker && !wide && si == 1)
             {
                 const cudaError_t e = cudaStreamWaitEvent(prep, pl->ev_src[0], 0);
                 if (e != cudaSuccess)
@@ -330,11 +386,11 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
                     break;
                 }
             }
-            st = prepare_scale(pl, si, chain_src, chain_tgt, sp[si], src_branch(si) ? prep_src : prep,
-                               serial ? nullptr : pl->ev_grid[si]);
+            st = prepare_scale(pl, si, chain_src, chain_tgt, sp[si], src_branch(si) ? prep_src : prep, prep_nrm,
+                               pl->ev_tgt[si], serial ? nullptr : pl->ev_grid[si]);
             if (!st && !serial)
             {
-                cudaError_t e = cudaEventRecord(pl->ev_scale[si], prep);
+                cudaError_t e = cudaEventRecord(pl->ev_scale[si], prep_nrm);
                 if (e == cudaSuccess && src_branch(si))
                     e = cudaEventRecord(pl->ev_src[si], prep_src);
                 if (e != cudaSuccess)
@@ -473,7 +529,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
     if (st && !serial) // join the branches before giving up
     {
         cudaStreamWaitEvent(main_stream, pl->ev_scale[p.n_scales - 1], 0);
-        cudaStreamWaitEvent(main_stream, pl->ev_src[tracker ? p.n_scales - 1 : 0], 0);
+        cudaStreamWaitEvent(main_stream, pl->ev_src[tracker || wide ? p.n_scales - 1 : 0], 0);
     }
     return st;
 }
@@ -542,6 +598,13 @@ int gca3d_icp_plan_destroy(gca3d_icp_plan *pl)
         cudaStreamDestroy(pl->prep);
     if (pl->prep_src)
         cudaStreamDestroy(pl->prep_src);
+    if (pl->prep_nrm)
+        cudaStreamDestroy(pl->prep_nrm);
+    if (pl->ev_join)
+        cudaEventDestroy(pl->ev_join);
+    for (cudaEvent_t e : pl->ev_tgt)
+        if (e)
+            cudaEventDestroy(e);
     if (pl->ev_fork_src)
         cudaEventDestroy(pl->ev_fork_src);
     for (cudaEvent_t e : pl->ev_src)
@@ -612,10 +675,11 @@ static int plan_workspace(gca3d_icp_plan *pl, bool capture)
     auto event = [](cudaEvent_t &e) {
         return e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     };
-    bool ok = stream(pl->prep) && stream(pl->prep_src) && event(pl->ev_fork) && event(pl->ev_fork_src) &&
+    bool ok = stream(pl->prep) && stream(pl->prep_src) && stream(pl->prep_nrm) && event(pl->ev_join) &&
+              event(pl->ev_fork) && event(pl->ev_fork_src) &&
               event(pl->states_checked);
     for (int k = 0; k < pl->prm.n_scales && ok; ++k)
-        ok = event(pl->ev_scale[k]) && event(pl->ev_grid[k]) && event(pl->ev_src[k]);
+        ok = event(pl->ev_scale[k]) && event(pl->ev_grid[k]) && event(pl->ev_src[k]) && event(pl->ev_tgt[k]);
     if (!ok)
     {
         cudaGetLastError();

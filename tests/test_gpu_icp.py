@@ -154,6 +154,41 @@ def test_one_shot_calls_share_a_workspace(N, synth):
             assert r["status"] == N.ERR_NO_CORRESPONDENCES
 
 
+@pytest.mark.parametrize("k,n_points", [(1, 600), (1, 6_000), (3, 6_000), (2, 530_000)])
+@pytest.mark.parametrize("mode", ["shared_grid", "two_grids", "kept_normals", "kept_two_grids", "capped"])
+@pytest.mark.parametrize("graph", [False, True])
+def test_preparation_branches_equal_serial(N, synth, k, n_points, mode, graph):
+    """the preparation on its branches (the last size is above the line up to which the normals
+    have one) gives the bits of the preparation on the context stream alone, also on a repeat"""
+    if n_points > 100_000 and (mode != "two_grids" or not graph):
+        pytest.skip("one form of the large size")
+    ctx = N.Context(0)
+    pairs = [synth.room_pair(seed=60 + j, n_points=n_points, rot_deg=2.0, trans=0.02) for j in range(k)]
+    S = [ctx.cloud_from(p.src_xyz, p.src_rgb) for p in pairs]
+    T = [ctx.cloud_from(p.tgt_xyz, p.tgt_rgb) for p in pairs]
+    kept = mode.startswith("kept")
+    corr = 0.1 if mode in ("two_grids", "kept_two_grids") else 0.3
+    kw = dict(max_nn=12) if mode == "capped" else {}
+    if kept:
+        for t in T:
+            ctx.check(ctx.L.gca3d_estimate_normals(ctx.h, t.h, 0.3, 0))
+        scales = [N.scale(0.0, 4, corr, 0.3, 0.3), N.scale(0.0, 3, corr / 2, 0.3, 0.3)]
+    else:
+        scales = [N.scale(v, 4, corr * v / 0.1, 0.3 * v / 0.1, 0.3 * v / 0.1, **kw) for v in (0.1, 0.05, 0.025)]
+    got = {}
+    for serial in (0, 1):
+        prm = N.icp_params(scales, use_graph=graph, keep_target_normals=kept,
+                           tuning=N.Tuning(0, 0, 0, 0, 0, serial))
+        plan = N.IcpPlan(ctx, S, T, prm)
+        got[serial] = [plan.execute() for _ in range(2)]
+    for reps in zip(*got[0], *got[1]):
+        for r in reps[:-1]:
+            assert r["status"] == reps[-1]["status"] and r["scale_iterations"] == reps[-1]["scale_iterations"]
+            np.testing.assert_array_equal(r["T"], reps[-1]["T"])
+    # 600 points are too sparse to register: there both end with the same status
+    assert n_points <= 600 or all(r["scale_iterations"][0] > 0 for r in got[1][0])
+
+
 def test_plan_graph_replay(ctx, N, synth):
     pairs = make_batch(synth, k=4, seed=1)
     srcs = [ctx.cloud_from(p.src_xyz, p.src_rgb) for p in pairs]
