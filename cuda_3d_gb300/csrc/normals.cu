@@ -494,9 +494,9 @@ __global__ void __launch_bounds__(256, 4) k_normals32(GridDev g, const int32_t *
 // points' moments are then finished by one lane each.  A neighbourhood beyond the shared
 // list falls back to one lane with an ordered list in local memory.
 // One thread per point with such a list is bound by its local memory: inside pass 1 it held
-// every warp with one such lane (206k points, at most 30 neighbours: 119 us for the pass,
-// @@), and where most points exceed the cap (200k points, radius of three voxels) the call
-// took 2468 us, now @@.
+// every warp with one such lane (206k points, at most 30 neighbours: 119 us for the pass; 59
+// and 13 for this one now), and where most points exceed the cap (200k points, radius of three
+// voxels) the call took 2479 us, now 760.
 constexpr int kSelCand = 256;
 constexpr int kSelWarps = 4;
 
@@ -664,14 +664,39 @@ __global__ void __launch_bounds__(32 * kSelWarps) k_normals_select(GridDev g, fl
     }
 }
 
-// pass 2: the queued near-degenerate points (a few dozen per frame), one warp per
-// point: lanes 0..8 walk one row each of the 27-cell neighbourhood and write the
-// points inside the radius to shared memory at deterministic positions (row
-// counts, then their prefix); with max_nn the max_nn nearest (distance, then
-// index) are kept by rank; the FP64 moments about the point are summed per lane
-// and across the warp in a fixed order, and lane 0 solves the eigen-problem in
-// closed form.  A neighbourhood larger than the shared list (kN64Cand points)
-// falls back to one lane walking the rows itself.
+// a warp's nine sums in every lane, each added over the lanes 16, 8, 4, 2, 1 apart as a
+// butterfly would: at each distance a lane keeps half of the values and gives the other half
+// away, so a value is added up once and not in all 32 lanes (12 FP64 additions, not 45)
+__device__ __forceinline__ void warp_sum9(double (&a)[3], double (&b)[6])
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    auto half = [&](double lo, double hi, int d) {
+        const bool up = lane & d;
+        return (up ? hi : lo) + __shfl_xor_sync(full, up ? lo : hi, d);
+    };
+    const double w0 = half(a[0], b[2], 16), w1 = half(a[1], b[3], 16), w2 = half(a[2], b[4], 16);
+    const double w3 = half(b[0], b[5], 16), w4 = half(b[1], 0.0, 16);
+    const double x0 = half(w0, w3, 8), x1 = half(w1, w4, 8), x2 = half(w2, 0.0, 8);
+    const double y0 = half(x0, x2, 4), y1 = half(x1, 0.0, 4);
+    double z = half(y0, y1, 2);
+    z += __shfl_xor_sync(full, z, 1);
+    a[0] = __shfl_sync(full, z, 0), a[1] = __shfl_sync(full, z, 2), a[2] = __shfl_sync(full, z, 4);
+    b[0] = __shfl_sync(full, z, 8), b[1] = __shfl_sync(full, z, 10), b[2] = __shfl_sync(full, z, 16);
+    b[3] = __shfl_sync(full, z, 18), b[4] = __shfl_sync(full, z, 20), b[5] = __shfl_sync(full, z, 24);
+}
+
+// pass 2: the queued near-degenerate points (a few dozen per frame, tens of thousands in a
+// batch): a warp gathers a point, lanes 0..8 walking one row each of the 27-cell neighbourhood
+// and writing the points inside the radius to shared memory at deterministic positions (row
+// counts, then their prefix); with max_nn the max_nn nearest (distance, then index) are kept
+// by rank; the FP64 moments about the point are summed per lane and across the warp in a
+// fixed order.  Up to 32 points' eigen-problems are then solved in closed form by one lane
+// each.  A neighbourhood larger than the shared list (kN64Cand points) falls back to one lane
+// walking the rows itself.
+// Bound by FP64 instructions (an SM starts one of a warp in about 19 cycles, whatever its
+// lanes do): with a warp per solve and the sums added in all lanes a scale of 64 pairs took
+// 148 us, now 75; the few points of a frame are one chain of 64-cycle operations, 34 us as before.
 constexpr int kN64Cand = 256;
 
 __global__ void __launch_bounds__(128) k_normals64(GridDev g, float rn, int max_nn, NormalOut O)
@@ -684,146 +709,167 @@ __global__ void __launch_bounds__(128) k_normals64(GridDev g, float rn, int max_
     const float rn2 = __fmul_rn(rn, rn);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
-    for (int j = blockIdx.x * 4 + warp; j < n; j += gridDim.x * 4)
+    const int warps = gridDim.x * 4;
+    const int per = min(32, max(1, (n + warps - 1) / warps)); // points per warp before they are solved
+    for (int j0 = (blockIdx.x * 4 + warp) * per; j0 < n; j0 += warps * per)
     {
-        const int s = O.degen_list[j];
-        const float4 p4 = g.spos[s];
-        const float3 p = make_float3(p4.x, p4.y, p4.z);
-        const int seg = L.bseg ? (int)(g.skey[s] >> segshift) : 0;
-        GridRows R;
-        grid_rows(g, L, seg, g.gmin[seg], p, R);
-        // the z window of this lane's row
-        int t0 = 0, e = 0;
-        if (lane < 9)
+        double M1[3] = {0.0, 0.0, 0.0}, M2[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}; // this lane's point
+        int Mk = 0;
+        for (int i = 0; i < per && j0 + i < n; ++i)
         {
-            t0 = R.r[0].x, e = R.r[0].y;
-#pragma unroll
-            for (int k = 1; k < 9; ++k)
-                if (lane == k)
-                    t0 = R.r[k].x, e = R.r[k].y;
-            int a = t0, b = e;
-            while (a < b)
+            const int s = O.degen_list[j0 + i];
+            const float4 p4 = g.spos[s];
+            const float3 p = make_float3(p4.x, p4.y, p4.z);
+            const int seg = L.bseg ? (int)(g.skey[s] >> segshift) : 0;
+            GridRows R;
+            grid_rows(g, L, seg, g.gmin[seg], p, R);
+            // the z window of this lane's row
+            int t0 = 0, e = 0;
+            if (lane < 9)
             {
-                const int m = (a + b) >> 1;
-                if (__ldg(&g.scz[m]) < R.lo)
-                    a = m + 1;
-                else
-                    b = m;
-            }
-            t0 = a;
-        }
-        auto inside = [&](int t, float &d2) {
-            const float4 q = __ldg(&g.spos[t]);
-            const int qz = __float_as_int(q.w);
-            d2 = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
-            return qz <= R.hi && d2 < rn2;
-        };
-        int cnt = 0;
-        for (int t = t0; t < e; ++t)
-        {
-            float d2;
-            if (__float_as_int(__ldg(&g.spos[t]).w) > R.hi)
-                break;
-            if (inside(t, d2))
-                ++cnt;
-        }
-        int off = cnt;
+                t0 = R.r[0].x, e = R.r[0].y;
 #pragma unroll
-        for (int d = 1; d < 16; d <<= 1)
-        {
-            const int y = __shfl_up_sync(full, off, d);
-            if (lane >= d)
-                off += y;
-        }
-        const int total = __shfl_sync(full, off, 8);
-        off -= cnt;
-        double S1[3] = {0.0, 0.0, 0.0}, S2[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        int k = 0;
-        auto acc = [&](float4 q) {
-            const double dx = (double)q.x - (double)p.x, dy = (double)q.y - (double)p.y, dz = (double)q.z - (double)p.z;
-            S1[0] += dx, S1[1] += dy, S1[2] += dz;
-            S2[0] += dx * dx, S2[1] += dx * dy, S2[2] += dx * dz;
-            S2[3] += dy * dy, S2[4] += dy * dz, S2[5] += dz * dz;
-            ++k;
-        };
-        if (total <= kN64Cand)
-        {
-            int w = off;
+                for (int k = 1; k < 9; ++k)
+                    if (lane == k)
+                        t0 = R.r[k].x, e = R.r[k].y;
+                int a = t0, b = e;
+                while (a < b)
+                {
+                    const int m = (a + b) >> 1;
+                    if (__ldg(&g.scz[m]) < R.lo)
+                        a = m + 1;
+                    else
+                        b = m;
+                }
+                t0 = a;
+            }
+            auto inside = [&](int t, float &d2) {
+                const float4 q = __ldg(&g.spos[t]);
+                const int qz = __float_as_int(q.w);
+                d2 = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
+                return qz <= R.hi && d2 < rn2;
+            };
+            int cnt = 0;
             for (int t = t0; t < e; ++t)
             {
                 float d2;
                 if (__float_as_int(__ldg(&g.spos[t]).w) > R.hi)
                     break;
                 if (inside(t, d2))
-                {
-                    s_d2[warp][w] = d2;
-                    s_t[warp][w] = t;
-                    ++w;
-                }
+                    ++cnt;
             }
-            __syncwarp();
-            const bool select = max_nn > 0 && total > max_nn;
-            for (int c = lane; c < total; c += 32)
+            int off = cnt;
+#pragma unroll
+            for (int d = 1; d < 16; d <<= 1)
             {
-                const float dc = s_d2[warp][c];
-                const int tc = s_t[warp][c];
-                bool keep = true;
-                if (select)
+                const int y = __shfl_up_sync(full, off, d);
+                if (lane >= d)
+                    off += y;
+            }
+            const int total = __shfl_sync(full, off, 8);
+            off -= cnt;
+            double S1[3] = {0.0, 0.0, 0.0}, S2[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            int k = 0;
+            auto acc = [&](float4 q) {
+                const double dx = (double)q.x - (double)p.x, dy = (double)q.y - (double)p.y, dz = (double)q.z - (double)p.z;
+                S1[0] += dx, S1[1] += dy, S1[2] += dz;
+                S2[0] += dx * dx, S2[1] += dx * dy, S2[2] += dx * dz;
+                S2[3] += dy * dy, S2[4] += dy * dz, S2[5] += dz * dz;
+                ++k;
+            };
+            if (total <= kN64Cand)
+            {
+                int w = off;
+                for (int t = t0; t < e; ++t)
                 {
-                    int rank = 0;
-                    for (int o = 0; o < total; ++o)
+                    float d2;
+                    if (__float_as_int(__ldg(&g.spos[t]).w) > R.hi)
+                        break;
+                    if (inside(t, d2))
                     {
-                        const float d2o = s_d2[warp][o];
-                        rank += d2o < dc || (d2o == dc && __ldg(&g.sidx[s_t[warp][o]]) < __ldg(&g.sidx[tc]));
+                        s_d2[warp][w] = d2;
+                        s_t[warp][w] = t;
+                        ++w;
                     }
-                    keep = rank < max_nn;
                 }
-                if (keep)
-                    acc(__ldg(&g.spos[tc]));
+                __syncwarp();
+                const bool select = max_nn > 0 && total > max_nn;
+                for (int c = lane; c < total; c += 32)
+                {
+                    const float dc = s_d2[warp][c];
+                    const int tc = s_t[warp][c];
+                    bool keep = true;
+                    if (select)
+                    {
+                        int rank = 0;
+                        for (int o = 0; o < total; ++o)
+                        {
+                            const float d2o = s_d2[warp][o];
+                            rank += d2o < dc || (d2o == dc && __ldg(&g.sidx[s_t[warp][o]]) < __ldg(&g.sidx[tc]));
+                        }
+                        keep = rank < max_nn;
+                    }
+                    if (keep)
+                        acc(__ldg(&g.spos[tc]));
+                }
+                warp_sum9(S1, S2);
+                k = __reduce_add_sync(full, k);
+                __syncwarp(); // the list is rewritten by the next point
             }
+            if (total > kN64Cand && lane == 0)
+            {
+                // a neighbourhood larger than the shared list: one lane, as the FP32 pass
+                grid_scan(g, R, [&](int t, float4 q) {
+                    if (dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z) < rn2)
+                        acc(q);
+                });
+                if (max_nn > 0 && k > max_nn)
+                {
+                    NbrEntry list[kMaxNN];
+                    S1[0] = S1[1] = S1[2] = 0.0;
+                    for (int i = 0; i < 6; ++i)
+                        S2[i] = 0.0;
+                    k = 0;
+                    const int cnt2 = select_knn(g, R, p, rn2, max_nn, list);
+                    for (int i = 0; i < cnt2; ++i)
+                        acc(g.spos[list[i].t]);
+                }
+            }
+            if (total > kN64Cand)
+            {
+                // only lane 0 has the sums
 #pragma unroll
-            for (int d = 16; d > 0; d >>= 1)
+                for (int q = 0; q < 3; ++q)
+                    S1[q] = __shfl_sync(full, S1[q], 0);
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    S2[q] = __shfl_sync(full, S2[q], 0);
+                k = __shfl_sync(full, k, 0);
+            }
+            if (lane == i)
             {
 #pragma unroll
-                for (int i = 0; i < 3; ++i)
-                    S1[i] += __shfl_xor_sync(full, S1[i], d);
+                for (int q = 0; q < 3; ++q)
+                    M1[q] = S1[q];
 #pragma unroll
-                for (int i = 0; i < 6; ++i)
-                    S2[i] += __shfl_xor_sync(full, S2[i], d);
-                k += __shfl_xor_sync(full, k, d);
-            }
-            __syncwarp(); // the list is rewritten by the next point
-        }
-        else if (lane == 0)
-        {
-            // a neighbourhood larger than the shared list: one lane, as the FP32 pass
-            grid_scan(g, R, [&](int t, float4 q) {
-                if (dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z) < rn2)
-                    acc(q);
-            });
-            if (max_nn > 0 && k > max_nn)
-            {
-                NbrEntry list[kMaxNN];
-                S1[0] = S1[1] = S1[2] = 0.0;
-                for (int i = 0; i < 6; ++i)
-                    S2[i] = 0.0;
-                k = 0;
-                const int cnt2 = select_knn(g, R, p, rn2, max_nn, list);
-                for (int i = 0; i < cnt2; ++i)
-                    acc(g.spos[list[i].t]);
+                for (int q = 0; q < 6; ++q)
+                    M2[q] = S2[q];
+                Mk = k;
             }
         }
-        if (lane == 0)
+        const int j = j0 + lane;
+        if (lane < per && j < n)
         {
-            const double kk = (double)k;
-            const double mu[3] = {S1[0] / kk, S1[1] / kk, S1[2] / kk};
+            const int s = O.degen_list[j];
+            const double kk = (double)Mk;
+            const double mu[3] = {M1[0] / kk, M1[1] / kk, M1[2] / kk};
             double C[3][3];
-            C[0][0] = S2[0] / kk - mu[0] * mu[0];
-            C[0][1] = C[1][0] = S2[1] / kk - mu[0] * mu[1];
-            C[0][2] = C[2][0] = S2[2] / kk - mu[0] * mu[2];
-            C[1][1] = S2[3] / kk - mu[1] * mu[1];
-            C[1][2] = C[2][1] = S2[4] / kk - mu[1] * mu[2];
-            C[2][2] = S2[5] / kk - mu[2] * mu[2];
+            C[0][0] = M2[0] / kk - mu[0] * mu[0];
+            C[0][1] = C[1][0] = M2[1] / kk - mu[0] * mu[1];
+            C[0][2] = C[2][0] = M2[2] / kk - mu[0] * mu[2];
+            C[1][1] = M2[3] / kk - mu[1] * mu[1];
+            C[1][2] = C[2][1] = M2[4] / kk - mu[1] * mu[2];
+            C[2][2] = M2[5] / kk - mu[2] * mu[2];
             double v[3];
             smallest_eigvec_f64(C, v);
             float3 nrm = make_float3((float)v[0], (float)v[1], (float)v[2]);

@@ -438,6 +438,34 @@ def test_degenerate_normals_vs_f64(ctx, orc):
     assert err.max() < 1e-6, np.percentile(err, [50, 99, 100])
 
 
+@pytest.mark.parametrize("lines", [1, 30, 140, 420])
+def test_degenerate_normals_many_points_vs_f64(ctx, orc, lines):
+    """as above for queues that are shorter and longer than the FP64 pass has warps (one point
+    each, several, and more than 32 each, so that a warp takes several rounds), with a queue that is
+    no multiple of them; same bound"""
+    cKDTree = pytest.importorskip("scipy.spatial").cKDTree
+    rng = np.random.default_rng(lines)
+    per = 301
+    o = rng.uniform(-1.0, 1.0, (lines, 1, 3)) * (lines / 20 + 1) ** (1 / 3)
+    d = rng.normal(size=(lines, 1, 3))
+    d /= np.linalg.norm(d, axis=2, keepdims=True)
+    t = rng.uniform(0.0, 0.5, (lines, per, 1))
+    xyz = (o + t * d + rng.normal(size=(lines, per, 3)) * 2e-4).reshape(-1, 3).astype(np.float32)
+    n = normals_gpu(ctx, xyz, 0.02)
+    ref = orc.normals_f64(xyz, 0.02, 0)
+    x64 = xyz.astype(np.float64)
+    some = rng.permutation(len(xyz))[:3000]
+    gap = np.full(len(xyz), np.nan)
+    for i, nb in zip(some, cKDTree(x64).query_ball_point(x64[some], 0.0199)):
+        if len(nb) >= 3:
+            ev = np.linalg.eigvalsh(np.cov(x64[nb].T, bias=True))
+            gap[i] = (ev[1] - ev[0]) / (ev[2] - ev[0])
+    sel = (gap > 1e-7) & (gap < 3e-4)
+    assert sel.sum() > 25
+    err = angle_err(n[sel].astype(np.float64), ref[sel])
+    assert err.max() < 1e-6, np.percentile(err, [50, 99, 100])
+
+
 def test_gradient_vs_f64(ctx, orc, room_v01):
     xyz, rgb = room_v01
     c = ctx.cloud_from(xyz, rgb)
