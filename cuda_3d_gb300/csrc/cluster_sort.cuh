@@ -10,10 +10,13 @@
 // launches, half of them passes with nothing to do, and in a pass a chain of a dozen
 // dependent memory accesses.  Here a pass of 8 bits takes 2 us plus 1 us per 1024 words of a
 // block, about half of it ranking.  Measured (GB300, whole calls, this against the launches):
-// voxel stage at 20k points 64 / 104 us, outlier removal at 180k 168 / 182, nearest
-// neighbours in 200k 245 / 251, voxel stage at 300k (with more words per thread) 161 / 136:
-// the line is drawn at 13 words per thread, 213k points.  Larger sets, and batches of
-// several, have tiles enough to fill the GPU, of which a cluster is a tenth.
+// voxel stage at 20k points 62 / 111 us, alignment of 64k 301 / 345, outlier removal at 180k
+// 136 / 157, nearest neighbours in 200k 172 / 183, normals of 206k 203 / 217.  The line is
+// drawn at 13 words per thread, 213k points: with 16 (256k, what the shared memory holds) a
+// voxel stage at 256k took 143 / 134, a 250k pair 883 / 870, and the extra registers cost the
+// 64k alignment 3 %, against 152 / 158 for neighbours in 256k.  Larger sets, and batches of
+// several, have tiles enough to fill the
+// GPU, of which a cluster is a tenth.
 #pragma once
 
 #include "sort_keys.cuh"

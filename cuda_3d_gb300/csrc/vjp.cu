@@ -30,7 +30,8 @@
 // What bounds it is the chain of launches and of dependent FP64 operations, not the points.
 // 100,000 points, K = 5 (GB300): a step adjoint in one thread was a launch of 51 us; what of
 // it does not depend on the cotangents now runs once for all steps (13 us) and the rest, a
-// few microseconds, in the point launch's last block.  The call: 904 to 680 us.  The 391
+// few microseconds, in the point launch's last block.  The call: 904 to 680 us (612 with
+// the shorter finalize and search of the forward pass).  The 391
 // block partials are still added one after the other (12 us of a point launch: an FP64
 // addition takes 64 cycles): at convergence the gradient of the start is the residue of
 // sums that cancel to their last bit, so their order is kept.

@@ -471,8 +471,8 @@ int gca3d_selfcheck_fp64(gca3d_context *ctx, int n, double out[4]);
 
 /* ---------------------------------------------------------------------------
  * bounded cross-block waits (no reference counterpart: the reference's kernels
- * never wait on one another).  The look-backs of the radix sort, the scan and the
- * frame compaction poll their predecessors' states; after `polls` unanswered
+ * never wait on one another).  The look-backs of the radix sort and the scan poll
+ * their predecessors' states; after `polls` unanswered
  * polls (64 ns sleeps between them after the first 64) a wait gives up, the
  * state counts as the end of the look-back (offsets stay inside the outputs) and
  * the call returns GCA3D_ERR_TIMEOUT.  Default 4,194,304 polls (about 0.3 s).
