@@ -988,10 +988,10 @@ __global__ void __launch_bounds__(128) k_icp_finalize(PairState *st, int P, int 
     rebuild_maps_body<128>(st, P, bmap, bmap_nn, loop);
 }
 
-IcpShape icp_shape(const gca3d_tuning &t, int P)
+IcpShape icp_shape(const gca3d_tuning &t, int P, int64_t src_cap)
 {
     IcpShape s;
-    s.nn_chunk = P == 1 ? kNNChunkSingle : kNNChunk;
+    s.nn_chunk = P == 1 || src_cap <= kNNSmallPoints ? kNNChunkSmall : kNNChunk;
     if (t.nn_item_points == 64 || t.nn_item_points == 128 || t.nn_item_points == 256 || t.nn_item_points == 512)
         s.nn_chunk = t.nn_item_points;
     if (t.nn_blocks_per_sm > 0)

@@ -422,7 +422,7 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
             int2 *corr = sp[si].corr;
             const NNCerts cert = sp[si].cert;
             int *bmap = sp[si].bmap, *bmap_nn = sp[si].bmap_nn;
-            const IcpShape shape = icp_shape(p.tuning, P);
+            const IcpShape shape = icp_shape(p.tuning, P, pl->src_cap);
             if ((st = icp_setup(ctx, pl->d_state, P, bs.seg_off, bt.seg_off, bmap, bmap_nn, si, shape.nn_chunk)))
                 return st;
             IcpScale prm;
@@ -741,8 +741,10 @@ int gca3d::icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *cons
         pl->src_max = std::max(pl->src_max, src[k]->capacity);
         pl->tgt_max = std::max(pl->tgt_max, tgt[k]->capacity);
         nb += div_up(src[k]->capacity, kIcpChunk);
-        pl->max_blocks_nn += div_up(src[k]->capacity, icp_shape(params->tuning, P).nn_chunk);
     }
+    const int nn_chunk = icp_shape(params->tuning, P, pl->src_cap).nn_chunk;
+    for (int k = 0; k < P; ++k)
+        pl->max_blocks_nn += div_up(src[k]->capacity, nn_chunk);
     pl->max_blocks = std::max(nb, 1);
     pl->max_blocks_nn = std::max(pl->max_blocks_nn, 1);
     if ((st = plan_workspace(pl, capture)))
@@ -962,7 +964,10 @@ extern "C" int gca3d_icp_autotune(gca3d_context *ctx, int n_pairs, gca3d_cloud *
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "autotune: bad arguments");
     reps = std::max(reps, 1);
     gca3d_icp_params p = *params;
-    const IcpShape s0 = icp_shape(p.tuning, n_pairs);
+    int64_t src_cap = 0;
+    for (int k = 0; k < n_pairs; ++k)
+        src_cap += src[k] ? src[k]->capacity : 0; // (a null handle is refused below)
+    const IcpShape s0 = icp_shape(p.tuning, n_pairs, src_cap);
     gca3d_tuning cur{s0.nn_chunk, s0.nn_bps, s0.acc_bps, p.tuning.voxel_resort, s0.fused ? 1 : 0,
                      p.tuning.serial_prep};
     cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -419,7 +419,7 @@ extern "C" int gca3d_color_icp_vjp(gca3d_context *ctx, gca3d_cloud *src, gca3d_c
     if ((st = grid_build(ctx, bt, p->max_corr, kOriginPadF32, nullptr, g)))
         return st;
     const int max_blocks = std::max(div_up(src->capacity, kIcpChunk), 1);
-    const int max_blocks_nn = std::max(div_up(src->capacity, kNNChunkSingle), 1);
+    const int max_blocks_nn = std::max(div_up(src->capacity, kNNChunkSmall), 1);
     float4 *attr0 = ctx->arena.get<float4>(g.cap);
     float4 *attr1 = ctx->arena.get<float4>(g.cap);
     PairState *pst = ctx->arena.get<PairState>(1);

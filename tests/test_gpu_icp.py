@@ -189,6 +189,21 @@ def test_preparation_branches_equal_serial(N, synth, k, n_points, mode, graph):
     assert n_points <= 600 or all(r["scale_iterations"][0] > 0 for r in got[1][0])
 
 
+@pytest.mark.parametrize("n_points", [(1 << 19) - 1, 1 << 19, (1 << 19) + 1])
+def test_item_size_rule_equals_every_item_size(ctx, N, synth, n_points):
+    """two pairs around the line at which the default work item of the search doubles: the poses
+    of every item size, with a last item of one point or one short of full"""
+    pairs = [synth.room_pair(seed=80 + j, n_points=n_points, rot_deg=2.0, trans=0.02) for j in range(2)]
+    S = [ctx.cloud_from(p.src_xyz, p.src_rgb) for p in pairs]
+    T = [ctx.cloud_from(p.tgt_xyz, p.tgt_rgb) for p in pairs]
+    got = [N.IcpPlan(ctx, S, T, N.icp_params([N.scale(0.05, 4, 0.06, 0.1, 0.1)], use_graph=True,
+                                             tuning=N.Tuning(item))).execute() for item in (0, 64, 128, 256, 512)]
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert a["status"] == b["status"] == N.OK and a["iterations"] == b["iterations"]
+            np.testing.assert_array_equal(a["T"], b["T"])
+
+
 def test_plan_graph_replay(ctx, N, synth):
     pairs = make_batch(synth, k=4, seed=1)
     srcs = [ctx.cloud_from(p.src_xyz, p.src_rgb) for p in pairs]
