@@ -4,7 +4,9 @@
 // blocks (16 SMs), so its whole sort runs there: every block holds a sixteenth of the words,
 // a pass ranks them warp by warp (one ballot per digit bit), the blocks exchange their digit
 // counts, and every word goes straight to its place in its destination block through
-// distributed shared memory.  Blocks meet at the cluster's hardware barrier; nothing polls.
+// distributed shared memory.  Blocks meet at the cluster's hardware barrier; nothing polls.  No
+// block touches another's shared memory before the barrier that all have started by, nor after
+// the last one.
 //
 // What bounds the alternative (sort_keys.cuh, sort_scan.cu) at these sizes is latency: ten
 // launches, half of them passes with nothing to do, and in a pass a chain of a dozen
@@ -22,6 +24,7 @@
 #include "sort_keys.cuh"
 
 #include <cooperative_groups.h>
+#include <utility>
 
 namespace gca3d
 {
@@ -128,6 +131,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
+    // another block's shared memory may be accessed once that block has started: every block
+    // arrives here and waits before its first remote write, behind its reading of the points
+    auto started = cluster.barrier_arrive();
     extern __shared__ uint64_t s_words[];
     uint16_t *s_whist = reinterpret_cast<uint16_t *>(s_words + words); // [warp][bin]
     uint16_t *s_count = s_whist + kClusterWarps * kClusterBins; // [block][bin]
@@ -168,6 +174,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
                 s_red[warp][a] = v[a];
         }
         __syncthreads();
+        cluster.barrier_wait(std::move(started)); // every block has started
         if (tid < 6)
         {
             float m = s_red[0][tid];
