@@ -488,17 +488,57 @@ __global__ void __launch_bounds__(256, 4) k_normals32(GridDev g, const int32_t *
 
 // The points with more than max_nn neighbours: the max_nn nearest (distance, then index)
 // selected, then as in pass 1.  A warp per point: its lanes read the window's candidates side
-// by side, those inside the radius go to shared memory as (distance, index) keys, a
-// candidate's rank is the number of smaller keys, and nine lanes sum the nine moments over
-// the ranks in order (the order of an ordered list, so the sums round alike).  Up to 32
-// points' moments are then finished by one lane each.  A neighbourhood beyond the shared
-// list falls back to one lane with an ordered list in local memory.
-// One thread per point with such a list is bound by its local memory: inside pass 1 it held
+// by side (the rows nearest the point first), those inside the radius go to shared memory as
+// (distance, index) keys, a candidate's rank is the number of smaller keys, and nine lanes sum
+// the nine moments over the ranks in order (the order of an ordered list, so the sums round
+// alike).  When the shared list is full its max_nn smallest keys are moved to the front and
+// no candidate farther than these is taken from then on, so a neighbourhood of any size stays with the
+// whole warp.  Up to 32 points' moments are then finished by one lane each.
+// A thread per point with an ordered list is bound by its local memory: inside pass 1 it held
 // every warp with one such lane (206k points, at most 30 neighbours: 119 us for the pass; 59
 // and 13 for this one now), and where most points exceed the cap (200k points, radius of three
-// voxels) the call took 2479 us, now 760.
+// voxels) the call took 2479 us, now 760.  One lane with that list for neighbourhoods beyond
+// the shared one was worse still: 100k points with 300 neighbours each and a cap of 30 took
+// 3530 us with a thread per point, 22,000 so, and 1720 now (600: 5140, 34,000, 2140; 3000:
+// 12,400, 96,000, 6690; 200, which fit the shared list: 2820, 1610, 1620).
 constexpr int kSelCand = 256;
+static_assert(kSelCand >= kMaxNN + 64, "a full list holds more keys than are kept, and room for 32 more after");
 constexpr int kSelWarps = 4;
+
+// the keep smallest of a warp's cnt keys to the front of the list, in order; returns the
+// largest distance among them
+__device__ __noinline__ float select_front(unsigned long long *key, int *cand, int cnt, int keep)
+{
+    constexpr int kPer = kSelCand / 32;
+    const int lane = threadIdx.x & 31;
+    unsigned long long mine[kPer];
+    int t[kPer], rank[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+    {
+        const int c = lane + 32 * i;
+        mine[i] = c < cnt ? key[c] : 0ull;
+        t[i] = c < cnt ? cand[c] : 0;
+        rank[i] = 0;
+    }
+    for (int o = 0; o < cnt; ++o)
+    {
+        const unsigned long long k = key[o];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+            rank[i] += k < mine[i];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+        if (lane + 32 * i < cnt && rank[i] < keep)
+        {
+            key[rank[i]] = mine[i];
+            cand[rank[i]] = t[i];
+        }
+    __syncwarp();
+    return __uint_as_float((unsigned)(key[keep - 1] >> 32));
+}
 
 template <bool Grad>
 __global__ void __launch_bounds__(32 * kSelWarps) k_normals_select(GridDev g, float rn, int max_nn, NormalOut O)
@@ -534,10 +574,12 @@ __global__ void __launch_bounds__(32 * kSelWarps) k_normals_select(GridDev g, fl
             int cx, cy, cz;
             grid_cell(g, L, g.gmin[seg], p, cx, cy, cz);
             const int lo = cz - 1, hi = cz + 1;
-            // lane k < 9: the part of row k in the window, to within two points at either end
+            // lane k < 9: the part of a row in the window, to within two points at either end; the
+            // point's own row, its four neighbours, the corners
             int2 r;
             load_rows<1>(g, L, seg, lo, hi, &r, [&](int, int &x, int &y) {
-                x = cx + lane / 3 - 1, y = cy + lane % 3 - 1;
+                const int k = (int)(0x862075314ull >> (4 * min(lane, 8))) & 15; // 3 (x + 1) + (y + 1)
+                x = cx + k / 3 - 1, y = cy + k % 3 - 1;
                 return lane < 9;
             });
             int len = 0;
@@ -568,6 +610,7 @@ __global__ void __launch_bounds__(32 * kSelWarps) k_normals_select(GridDev g, fl
             const int total = __shfl_sync(full, end, 8);
             __syncwarp();
             int cnt = 0;
+            float limit = INFINITY; // candidates beyond it are not among the max_nn nearest
             for (int c0 = 0; c0 < total; c0 += 32)
             {
                 const int c = c0 + lane;
@@ -584,12 +627,20 @@ __global__ void __launch_bounds__(32 * kSelWarps) k_normals_select(GridDev g, fl
                     const float4 q = __ldg(&g.spos[t]);
                     const int qz = __float_as_int(q.w);
                     d2 = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
-                    in = qz >= lo && qz <= hi && d2 < rn2;
+                    in = qz >= lo && qz <= hi && d2 < rn2 && d2 <= limit;
                 }
-                const unsigned m = __ballot_sync(full, in);
-                const int at = cnt + __popc(m & ((1u << lane) - 1u));
-                if (in && at < kSelCand)
+                unsigned m = __ballot_sync(full, in);
+                if (cnt + __popc(m) > kSelCand)
                 {
+                    __syncwarp();
+                    limit = select_front(key, cand, cnt, max_nn);
+                    cnt = max_nn;
+                    in = in && d2 <= limit;
+                    m = __ballot_sync(full, in);
+                }
+                if (in)
+                {
+                    const int at = cnt + __popc(m & ((1u << lane) - 1u));
                     key[at] = (unsigned long long)__float_as_uint(d2) << 32 | (unsigned)__ldg(&g.sidx[t]);
                     cand[at] = t;
                 }
@@ -597,47 +648,25 @@ __global__ void __launch_bounds__(32 * kSelWarps) k_normals_select(GridDev g, fl
             }
             __syncwarp();
             const int keep = min(cnt, max_nn);
+            for (int c = lane; c < cnt; c += 32)
+            {
+                const unsigned long long mine = key[c];
+                int rank = 0;
+#pragma unroll 4
+                for (int o = 0; o < cnt; ++o)
+                    rank += key[o] < mine;
+                if (rank < max_nn)
+                {
+                    const float4 q = __ldg(&g.spos[cand[c]]);
+                    off[0][rank] = q.x - p.x, off[1][rank] = q.y - p.y, off[2][rank] = q.z - p.z;
+                }
+            }
+            __syncwarp();
             float v = 0.0f;
-            if (cnt <= kSelCand)
-            {
-                for (int c = lane; c < cnt; c += 32)
-                {
-                    const unsigned long long mine = key[c];
-                    int rank = 0;
+            if (lane < 9)
 #pragma unroll 4
-                    for (int o = 0; o < cnt; ++o)
-                        rank += key[o] < mine;
-                    if (rank < max_nn)
-                    {
-                        const float4 q = __ldg(&g.spos[cand[c]]);
-                        off[0][rank] = q.x - p.x, off[1][rank] = q.y - p.y, off[2][rank] = q.z - p.z;
-                    }
-                }
-                __syncwarp();
-                if (lane < 9)
-#pragma unroll 4
-                    for (int o = 0; o < keep; ++o)
-                        v = fmaf(off[ma][o], off[mb][o], v); // times 1: the sum of an addition
-            }
-            else
-            {
-                NbrEntry list[kMaxNN];
-                GridRows R;
-                if (lane == 0)
-                {
-                    grid_rows(g, L, seg, g.gmin[seg], p, R);
-                    select_knn(g, R, p, rn2, max_nn, list);
-                    for (int o = 0; o < keep; ++o)
-                    {
-                        const float4 q = __ldg(&g.spos[list[o].t]);
-                        off[0][o] = q.x - p.x, off[1][o] = q.y - p.y, off[2][o] = q.z - p.z;
-                    }
-                }
-                __syncwarp();
-                if (lane < 9)
-                    for (int o = 0; o < keep; ++o)
-                        v = fmaf(off[ma][o], off[mb][o], v);
-            }
+                for (int o = 0; o < keep; ++o)
+                    v = fmaf(off[ma][o], off[mb][o], v); // times 1: the sum of an addition
             float sum[9];
 #pragma unroll
             for (int q = 0; q < 9; ++q)

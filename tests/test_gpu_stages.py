@@ -406,6 +406,63 @@ def test_capped_normals_vs_f64(ctx, max_nn, density):
     assert (err <= 2e-6 / gap[ok]).all(), (err * gap[ok]).max()
 
 
+@pytest.mark.parametrize("near", [225, 255, 256, 257, 289, 480, 481, 2000])
+@pytest.mark.parametrize("max_nn", [1, 3, 30, 64])
+@pytest.mark.parametrize("order", ["random", "far_first"])
+def test_capped_selection_around_its_list(ctx, near, max_nn, order):
+    """neighbourhoods (one group of points, every point with all the others in its radius)
+    around the sizes at which the selection's list of 256 keys is filled and cut back, and far
+    above; the points in random order and with the distances to the first falling.  The kept
+    set decides the normal, so it must be the FP64 normal of the max_nn nearest (FP32
+    distance, then index) within 2e-6 / relative gap of its two smallest eigenvalues, as above"""
+    rng = np.random.default_rng(near + max_nn)
+    uv = (rng.random((near, 2)) - 0.5) * 0.02
+    xyz = np.stack([uv[:, 0], uv[:, 1], 3.0 * uv[:, 0] ** 2 + 0.004 * rng.random(near)], 1).astype(np.float32)
+    if order == "far_first":
+        xyz = xyz[np.argsort(-((xyz - xyz[0]) ** 2).sum(1))]
+    radius = np.float32(0.06)
+    d2 = np.zeros((near, near), np.float32)
+    for k in range(3):
+        d = xyz[None, :, k] - xyz[:, None, k]
+        d2 += d * d
+    assert (d2 < radius * radius).all()
+    kept = np.argsort(d2, axis=1, kind="stable")[:, :max_nn]
+    n = normals_gpu(ctx, xyz, radius, max_nn).astype(np.float64)
+    if max_nn < 3:
+        assert not n.any() # fewer than three points have no normal
+        return
+    off = xyz[kept].astype(np.float64) - xyz[:, None].astype(np.float64)
+    mu = off.mean(1)
+    cov = np.einsum("nki,nkj->nij", off, off) / max_nn - mu[:, :, None] * mu[:, None, :]
+    val, vec = np.linalg.eigh(cov)
+    gap = (val[:, 1] - val[:, 0]) / np.maximum(val[:, 2] - val[:, 0], 1e-30)
+    ok = gap > 1e-5
+    assert ok.mean() > 0.5
+    err = np.linalg.norm(np.cross(n[ok], vec[ok][:, :, 0]), axis=1)
+    assert (err <= 2e-6 / gap[ok]).all(), (err * gap[ok]).max()
+
+
+def test_capped_normals_cost_grows_with_the_neighbourhood(ctx):
+    """a cap of 30 with about 200 and 400 neighbours a point, either side of the selection's
+    list: twice the candidates take a few times as long (2.2 measured), not tens of times"""
+    import time
+
+    rng = np.random.default_rng(5)
+    n = 60_000
+    c = ctx.cloud_from(np.stack([rng.random(n), rng.random(n), 0.002 * rng.random(n)], 1).astype(np.float32))
+
+    def best(near):
+        radius = float(np.sqrt(near / (np.pi * n)))
+        times = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            ctx.check(ctx.L.gca3d_estimate_normals(ctx.h, c.h, radius, 30)) # waits for its result
+            times.append(time.perf_counter() - t0)
+        return min(times)
+
+    assert best(400) < 5.0 * best(200)
+
+
 def test_degenerate_normals_vs_f64(ctx, orc):
     """Points on thin noisy lines: the two smallest eigenvalues of every
     neighbourhood are close, so the FP32 pass queues them and every normal comes
