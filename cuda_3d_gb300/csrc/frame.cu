@@ -9,7 +9,8 @@
 // device and compacts with thrust::remove_if.  Here k_frame_filter filters pixel
 // tiles staged in shared memory with their halo, decides which pixels become points and
 // writes the filtered depth, one bit per pixel and one count per row of a tile;
-// k_frame_points (one block per row) sums the counts above its row and writes the
+// k_frame_points (one block per row) adds up the counts above its row, or takes their scan
+// for a very tall frame, and writes the
 // compacted SoA points in raster order.  Same arithmetic order as the reference (unfused
 // multiply/add); the filter weights use det_expf below instead of expf, so the CPU oracle
 // reproduces every output bit.
@@ -33,6 +34,12 @@ constexpr int kTileW = 64;         // pixels of a filter tile: 64 x 4 (fixed), 6
 constexpr int kRangeFixed = 1024;  // tabulated depth differences of the fixed filter
 constexpr int kRangeAdaptive = 1536; // of the adaptive filter: past the last weight above zero
 constexpr float kNoDepth = 1e9f;   // a tap without a depth: beyond every tabulated difference
+// Up to so many additions of row counts (height x counts) k_frame_points adds up those above
+// each row itself: that is quadratic in the height, but no launch.  Above, they are scanned
+// first.  us summed / scanned: 640 x 480 (2.3 M) 37 / 45, 1920 x 1080 (35 M) 92 / 99,
+// 64 x 8192 (67 M) 55 / 60, 2048 x 2048 (134 M) 165 / 165, 64 x 16,384 (268 M) 86 / 79,
+// 64 x 65,536 414 / 221, 64 x 262,144 5370 / 803, 2048 x 8192 690 / 537.
+constexpr int64_t kSummedCounts = int64_t(1) << 27;
 constexpr int kAdaptiveSteps = 6;                                // adaptive filter: radius 0..5
 constexpr int kAdaptiveRadius = kAdaptiveSteps - 1;
 constexpr int kAdaptiveSq = 2 * kAdaptiveRadius * kAdaptiveRadius + 1; // squared offsets 0..50
@@ -285,8 +292,13 @@ __global__ void __launch_bounds__(kFrameThreads) k_frame_filter(const uint16_t *
     }
 }
 
-// the points of one image row, after those of the rows above it: the counts above (a few
-// KB, in L2) are summed by every block, which needs no wait between blocks
+// the length of the row counts, for their scan
+__global__ void k_frame_counts(int32_t *d_counts, int32_t n) { *d_counts = n; }
+
+// the points of one image row, after those of the rows above it.  Scanned: count holds the
+// counts' exclusive prefixes; otherwise the counts, and every block sums those above its row
+// (from L2), which needs no launch and no wait between blocks
+template <bool Scanned>
 __global__ void __launch_bounds__(kFrameThreads) k_frame_points(const uint8_t *__restrict__ bgr, FrameParams P,
                                                                 const float *__restrict__ zin,
                                                                 const uint32_t *__restrict__ mask,
@@ -300,12 +312,15 @@ __global__ void __launch_bounds__(kFrameThreads) k_frame_points(const uint8_t *_
     const int words = (P.w + 31) >> 5;
     const uint32_t w0 = lane < words ? mask[y * mask_pitch + lane] : 0u;
     const uint32_t w1 = lane + 32 < words ? mask[y * mask_pitch + lane + 32] : 0u;
-    int above = 0;
-    for (int i = threadIdx.x; i < y * tiles_x; i += kFrameThreads)
-        above += count[i];
-    above = __reduce_add_sync(0xffffffffu, above);
-    if (lane == 0)
-        s_sum[warp] = above;
+    if (!Scanned)
+    {
+        int above = 0;
+        for (int i = threadIdx.x; i < y * tiles_x; i += kFrameThreads)
+            above += count[i];
+        above = __reduce_add_sync(0xffffffffu, above);
+        if (lane == 0)
+            s_sum[warp] = above;
+    }
     int p0 = __popc(w0), p1 = __popc(w1);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1)
@@ -315,11 +330,16 @@ __global__ void __launch_bounds__(kFrameThreads) k_frame_points(const uint8_t *_
             p0 += a, p1 += b;
     }
     p1 += __shfl_sync(0xffffffffu, p0, 31);
-    __syncthreads();
     int base = 0;
+    if (Scanned)
+        base = count[y * tiles_x];
+    else
+    {
+        __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kFrameThreads / 32; ++k)
-        base += s_sum[k];
+        for (int k = 0; k < kFrameThreads / 32; ++k)
+            base += s_sum[k];
+    }
     if (y == P.h - 1 && threadIdx.x == 31)
         *d_count = base + p1;
     for (int i = warp; i < words; i += kFrameThreads / 32)
@@ -347,8 +367,12 @@ int frame_to_cloud(gca3d_context *ctx, const uint16_t *depth, const uint8_t *bgr
     const int tiles_x = div_up(P.w, kTileW), words = div_up(P.w, 32);
     float *z = ctx->arena.get<float>((size_t)P.w * P.h);
     uint32_t *mask = ctx->arena.get<uint32_t>((size_t)words * P.h);
-    int *count = ctx->arena.get<int>((size_t)tiles_x * P.h);
-    if (!z || !mask || !count)
+    const int64_t counts = (int64_t)tiles_x * P.h;
+    int *count = ctx->arena.get<int>(counts);
+    const bool scanned = counts * P.h > kSummedCounts;
+    int *prefix = scanned ? ctx->arena.get<int>(counts) : nullptr;
+    int *d_counts = scanned ? ctx->arena.get<int>(1) : nullptr;
+    if (!z || !mask || !count || (scanned && (!prefix || !d_counts)))
         return fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "frame_to_cloud: scratch");
     // the fixed filter's weights reach zero at a difference of 10.2 sigma (exp(-104)): the
     // table ends just past it, or at its capacity (then larger differences are evaluated)
@@ -375,8 +399,17 @@ int frame_to_cloud(gca3d_context *ctx, const uint16_t *depth, const uint8_t *bgr
     default: filter(std::integral_constant<int, 7>{}); break;
     }
     GCA_CHECK_LAUNCH(ctx);
-    k_frame_points<<<P.h, kFrameThreads, 0, ctx->stream>>>(bgr, P, z, mask, count, words, tiles_x, out->pos, out->col,
-                                                           out->d_count);
+    if (scanned)
+    {
+        k_frame_counts<<<1, 1, 0, ctx->stream>>>(d_counts, (int32_t)counts);
+        GCA_CHECK_LAUNCH(ctx);
+        const int st = exclusive_scan(ctx, count, prefix, d_counts, counts, nullptr);
+        if (st)
+            return st;
+    }
+    const auto points = scanned ? k_frame_points<true> : k_frame_points<false>;
+    points<<<P.h, kFrameThreads, 0, ctx->stream>>>(bgr, P, z, mask, scanned ? prefix : count, words, tiles_x, out->pos,
+                                                   out->col, out->d_count);
     GCA_CHECK_LAUNCH(ctx);
     GCA_PROF_END(ctx, kKidFrame);
     return GCA3D_OK;

@@ -685,6 +685,54 @@ def test_frame_tiles_and_weight_tables_vs_oracle(ctx, N, orc, w, h, mode, radius
     np.testing.assert_array_equal(d["rgb"], oc)
 
 
+@pytest.mark.parametrize("w,h", [(64, 11_585), (64, 11_586), (320, 5181), (320, 5182), (65, 20_001)])
+def test_tall_frames_vs_oracle(ctx, N, orc, w, h):
+    """both forms of the rows' offsets, around the line at which they change (2^27 for the
+    height times the row counts, of which there is one per 64 pixels of a row); most pixels
+    have no depth"""
+    rng = np.random.default_rng(w + h)
+    depth = np.where(rng.random((h, w)) < 0.3, rng.integers(1000, 1400, (h, w)), 0).astype(np.uint16)
+    depth[h // 3: h // 2] = 0
+    bgr = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+    dbuf, cbuf = ctx.alloc(depth.nbytes), ctx.alloc(bgr.nbytes)
+    dbuf.write(depth)
+    cbuf.write(bgr)
+    cloud = ctx.cloud(h * w)
+    intr = (525.0, 525.0, w / 2, h / 2)
+    di, f = N.Intrinsics(*intr), N.Filter(0, 0, 3.0, 30.0)
+    ctx.check(ctx.L.gca3d_frame_to_cloud(ctx.h, dbuf.ptr, cbuf.ptr, w, h, C.byref(di), None, None, 0.001, 0.2, 10.0,
+                                         C.byref(f), cloud.h))
+    d = cloud.download()
+    ox, oc = orc.make_point_cloud(depth, bgr, intr, mode=0, radius=0, sigma_space=3.0, sigma_depth=30.0, tmin=0.2,
+                                  tmax=10.0)
+    assert len(ox) > 0.2 * h * w
+    np.testing.assert_array_equal(d["xyz"], ox)
+    np.testing.assert_array_equal(d["rgb"], oc)
+
+
+def test_frame_cost_is_linear_in_the_height(ctx, N):
+    """a tall frame of 64 x 262,144 pixels against a wide one with as many: alike (the row
+    offsets took the tall one eight times as long when every row summed all rows above it)"""
+    import time
+
+    def best(w, h):
+        d, b = ctx.alloc(2 * w * h), ctx.alloc(3 * w * h)
+        d.write(np.full((h, w), 1500, np.uint16))
+        b.write(np.zeros((h, w, 3), np.uint8))
+        out = ctx.cloud(h * w)
+        di, f = N.Intrinsics(525.0, 525.0, w / 2, h / 2), N.Filter(2, 2, 3.0, 30.0)
+        times = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            ctx.check(ctx.L.gca3d_frame_to_cloud(ctx.h, d.ptr, b.ptr, w, h, C.byref(di), None, None, 0.001, 0.2, 10.0,
+                                                 C.byref(f), out.h))
+            ctx.sync()
+            times.append(time.perf_counter() - t0)
+        return min(times)
+
+    assert best(64, 262_144) < 4.0 * best(2048, 8192)
+
+
 # --------------------------------------------------------------------------- #
 # radius outlier removal, gather by index, AoS view
 # --------------------------------------------------------------------------- #
