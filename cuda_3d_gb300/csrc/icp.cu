@@ -330,6 +330,28 @@ struct BlockPair
     int pair, start, end;
 };
 
+// the last pair whose first item is <= w (pairs without items share theirs with the next;
+// bmap[0] is 0): 64 entries a round, so one round up to 64 pairs and two at 4096.  Its loads
+// are most of an item's latency: with 32 entries a round in order, up to 128 rounds, 4096 pairs
+// of 1000 points took 30,600 us (10 steps), now 28,500, and 64 pairs 884, 886.
+__device__ __forceinline__ int item_pair(int w, const int *bmap, int P)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int lo = 0, n = P;
+    for (;;)
+    {
+        const int step = (n + 63) >> 6;
+        const int a = lane * step, b = a + 32 * step;
+        const bool la = a < n && bmap[lo + a] <= w, lb = b < n && bmap[lo + b] <= w;
+        const int c = __popc(__ballot_sync(full, la)) + __popc(__ballot_sync(full, lb));
+        lo += (c - 1) * step;
+        if (step == 1)
+            return lo;
+        n = min(step, n - (c - 1) * step);
+    }
+}
+
 __device__ __forceinline__ void item_setup(int w, int items, const int32_t *src_off, const PairState *st,
                                            const int *bmap, int P, int chunk, float *s_T, BlockPair *s_item)
 {
@@ -337,16 +359,8 @@ __device__ __forceinline__ void item_setup(int w, int items, const int32_t *src_
     int p = -1;
     if (w < items)
     {
-        // the last pair whose first item is <= w (pairs without items share theirs with the next)
-        for (int base = 0; base < P; base += 32)
-        {
-            const bool le = base + lane < P && bmap[base + lane] <= w;
-            const int c = __popc(__ballot_sync(0xffffffffu, le));
-            p += c;
-            if (c < 32)
-                break;
-        }
-        if (p >= 0 && !st[p].active)
+        p = item_pair(w, bmap, P);
+        if (!st[p].active)
             p = -1;
     }
     if (p >= 0 && lane < 12)

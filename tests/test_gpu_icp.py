@@ -122,6 +122,28 @@ def test_batched_bit_identical_to_single(ctx, N, synth):
         assert single["fitness"] == b["fitness"]
 
 
+@pytest.mark.parametrize("k", [63, 64, 65, 129, 4095, 4096])
+def test_many_pairs_bit_identical_to_single(ctx, N, synth, k):
+    """pair counts around the widths of the item map's search, up to the largest allowed;
+    clouds are shared, and empty ones (pairs without work items) lie at the start, at the end
+    and in runs between"""
+    base = [synth.room_pair(seed=300 + j, n_points=700 + 151 * j, rot_deg=2.0, trans=0.02) for j in range(5)]
+    S = [ctx.cloud_from(p.src_xyz, p.src_rgb) for p in base] + [ctx.cloud(16)]
+    T = [ctx.cloud_from(p.tgt_xyz, p.tgt_rgb) for p in base] + [ctx.cloud(16)]
+    rng = np.random.default_rng(k)
+    which = rng.integers(0, 5, k)
+    for at in (0, 1, k // 2, k - 1):
+        which[at] = 5
+    which[k // 3: k // 3 + 35] = 5
+    prm = N.icp_params([N.scale(0.15, 4, 0.5, 0.6, 0.6)], use_graph=True)
+    single = [N.IcpPlan(ctx, [s], [t], prm).execute()[0] for s, t in zip(S, T)]
+    assert all(r["status"] == N.OK for r in single[:5]) and single[5]["status"] == N.ERR_NO_CORRESPONDENCES
+    many = N.IcpPlan(ctx, [S[j] for j in which], [T[j] for j in which], prm).execute()
+    for j, r in zip(which, many):
+        assert r["status"] == single[j]["status"] and r["iterations"] == single[j]["iterations"]
+        np.testing.assert_array_equal(r["T"], single[j]["T"])
+
+
 def test_one_shot_calls_share_a_workspace(N, synth):
     """one context's one-shot calls reuse one workspace: sizes, pair counts and scales that
     grow and shrink, a refused call and a call without correspondences in between give the
