@@ -1002,6 +1002,38 @@ __global__ void __launch_bounds__(128) k_icp_finalize(PairState *st, int P, int 
     rebuild_maps_body<128>(st, P, bmap, bmap_nn, loop);
 }
 
+// The same by one block per pair.  A cluster per pair pays where the sums are long: for a
+// single pair (whose maps it also rebuilds directly), and from about 48 partials a pair (48k
+// points; max_blocks, by capacity).  Below, its eight blocks and two barriers cost more than
+// the sums they share.  us for 30 steps, a cluster and one block: 1 pair of 1k points 874,
+// 907, of 64k 993, 1064; 2 pairs of 4k 985, 963, of 16k 1050, 1037, of 48k 1144, 1158, of 128k
+// 1700, 1750; 16 pairs of 4k 1134, 1086, of 32k 2548, 2530, of 64k 4397, 4412; 10 steps of
+// 4096 pairs of 1k 28,710, 27,630.
+constexpr int kClusterPartials = 48;
+template <bool Comp>
+__global__ void __launch_bounds__(kIcpThreads) k_icp_finalize_many(PairState *st, int P, int *bmap, int *bmap_nn,
+                                                                   const double *partials, IcpScale prm, IcpLoop loop)
+{
+    __shared__ double s_S[kTermsPad];
+    __shared__ int s_last;
+    const int pair = blockIdx.x;
+    PairState &Ps = st[pair];
+    if (Ps.active)
+    {
+        const FinalizeIn in = finalize_in(Ps);
+        finalize_sums<Comp>(Ps, partials + (size_t)bmap[pair] * kTermsPad, s_S);
+        finalize_solve(Ps, P, pair, s_S, prm, in);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        s_last = atomicAdd(loop.ticket, 1u) == (unsigned)(P - 1);
+    __syncthreads();
+    if (!s_last)
+        return;
+    rebuild_maps_body<kIcpThreads>(st, P, bmap, bmap_nn, loop);
+}
+
 IcpShape icp_shape(const gca3d_tuning &t, int P, int64_t src_cap)
 {
     IcpShape s;
@@ -1085,6 +1117,14 @@ int icp_update(gca3d_context *ctx, const Batch &src, const Grid &g, const float4
                 src.pos, src.seg_off, g.dev.spos, attr0, attr1, corr, st, bmap, bmap_nn, src.P, partials,
                 prm.sqrt_lg, prm.sqrt_lc, d_nt, ctx->d_err, prm, loop);
         GCA_CHECK_LAUNCH(ctx);
+        if (src.P > 1 && max_blocks < kClusterPartials * src.P)
+        {
+            const auto kernel = compensated ? k_icp_finalize_many<true> : k_icp_finalize_many<false>;
+            kernel<<<src.P, kIcpThreads, 0, ctx->stream>>>(st, src.P, bmap, bmap_nn, partials, prm, loop);
+            GCA_CHECK_LAUNCH(ctx);
+            GCA_PROF_END(ctx, kKidIcpIter);
+            return GCA3D_OK;
+        }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kSumGroups * src.P);
         cfg.blockDim = dim3(128);

@@ -144,6 +144,30 @@ def test_many_pairs_bit_identical_to_single(ctx, N, synth, k):
         np.testing.assert_array_equal(r["T"], single[j]["T"])
 
 
+@pytest.mark.parametrize("compensated", [True, False])
+@pytest.mark.parametrize("k", [2, 3, 300])
+def test_finalize_forms_give_the_same_poses(ctx, N, synth, k, compensated):
+    """the finalize with a cluster per pair and with a block per pair, on either side of the line
+    between them (48 blocks of 1024 points a pair, by the clouds' capacity) and far from it,
+    against one pair at a time"""
+    base = [synth.room_pair(seed=400 + j, n_points=(700, 9_001, 30_000)[j], rot_deg=2.0, trans=0.02)
+            for j in range(3)]
+    T = [ctx.cloud_from(p.tgt_xyz, p.tgt_rgb) for p in base]
+    scales = [N.scale(0.0, 4, 0.3, 0.4, 0.4), N.scale(0.05, 3, 0.2, 0.3, 0.3)]
+    prm = N.icp_params(scales, use_graph=True, compensated=compensated)
+    want = None
+    for blocks in (30, 47, 48, 49) if k < 10 else (30,):
+        S = [ctx.cloud_from(p.src_xyz, p.src_rgb, capacity=blocks * 1024) for p in base]
+        if want is None:
+            want = [N.IcpPlan(ctx, [s], [t], prm).execute()[0] for s, t in zip(S, T)]
+            assert all(r["status"] == N.OK for r in want)
+        got = N.IcpPlan(ctx, [S[j % 3] for j in range(k)], [T[j % 3] for j in range(k)], prm).execute()
+        for j, r in enumerate(got):
+            assert r["scale_iterations"] == want[j % 3]["scale_iterations"]
+            assert r["fitness"] == want[j % 3]["fitness"] and r["inlier_rmse"] == want[j % 3]["inlier_rmse"]
+            np.testing.assert_array_equal(r["T"], want[j % 3]["T"])
+
+
 def test_one_shot_calls_share_a_workspace(N, synth):
     """one context's one-shot calls reuse one workspace: sizes, pair counts and scales that
     grow and shrink, a refused call and a call without correspondences in between give the
