@@ -576,6 +576,24 @@ void fill_results(const gca3d_icp_plan *pl, gca3d_icp_result *res)
 
 } // namespace
 
+// the tables that hold pair_cap pairs
+static void free_tables(gca3d_icp_plan *pl)
+{
+    auto device = [](auto *&p) {
+        if (p)
+            cudaFree(p);
+        p = nullptr;
+    };
+    auto host = [](auto *&p) {
+        if (p)
+            cudaFreeHost(p);
+        p = nullptr;
+    };
+    device(pl->d_src), device(pl->d_tgt), device(pl->d_state), device(pl->d_Tinit);
+    host(pl->h_src), host(pl->h_state), host(pl->h_err), host(pl->h_Tinit);
+    pl->pair_cap = 0;
+}
+
 extern "C" {
 
 int gca3d_icp_plan_destroy(gca3d_icp_plan *pl)
@@ -590,8 +608,6 @@ int gca3d_icp_plan_destroy(gca3d_icp_plan *pl)
         cudaEventDestroy(pl->tinit_copied);
     if (pl->states_ready)
         cudaEventDestroy(pl->states_ready);
-    if (pl->h_err)
-        cudaFreeHost(pl->h_err);
     if (pl->side)
         cudaStreamDestroy(pl->side);
     if (pl->prep)
@@ -620,18 +636,9 @@ int gca3d_icp_plan_destroy(gca3d_icp_plan *pl)
             cudaEventDestroy(e);
     if (pl->graph)
         cudaGraphDestroy(pl->graph);
-    cudaFree(pl->d_src);
-    cudaFree(pl->d_tgt);
-    cudaFree(pl->d_state);
-    cudaFree(pl->d_Tinit);
-    if (pl->h_src)
-        cudaFreeHost(pl->h_src);
     if (pl->states_checked)
         cudaEventDestroy(pl->states_checked);
-    if (pl->h_state)
-        cudaFreeHost(pl->h_state);
-    if (pl->h_Tinit)
-        cudaFreeHost(pl->h_Tinit);
+    free_tables(pl);
     pl->arena.release();
     delete pl;
     return GCA3D_OK;
@@ -640,13 +647,14 @@ int gca3d_icp_plan_destroy(gca3d_icp_plan *pl)
 } // extern "C"
 
 // the tables, streams and events a plan of pl->P pairs and its scales needs: what is missing
-// is made, what is there is kept
+// or too small is made, what is there is kept
 static int plan_workspace(gca3d_icp_plan *pl, bool capture)
 {
     gca3d_context *ctx = pl->ctx;
     const int P = pl->P;
     if (pl->pair_cap < P)
     {
+        free_tables(pl);
         if (cudaMallocHost(&pl->h_src, sizeof(SegSrc) * 2 * P) != cudaSuccess ||
             cudaMalloc(&pl->d_src, sizeof(SegSrc) * P) != cudaSuccess ||
             cudaMalloc(&pl->d_tgt, sizeof(SegSrc) * P) != cudaSuccess ||
@@ -690,7 +698,7 @@ static int plan_workspace(gca3d_icp_plan *pl, bool capture)
 
 int gca3d::icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *const *src, gca3d_cloud *const *tgt,
                                     const gca3d_icp_params *params, bool capture, PlanPrologue prologue,
-                                    gca3d_icp_plan **out, const PlanVoxels *voxels, gca3d_icp_plan *reuse)
+                                    gca3d_icp_plan **out, const PlanVoxels *voxels, gca3d_icp_plan **reuse)
 {
     if (!ctx || !out || P < 1 || P > kMaxSegments || !src || !tgt)
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: bad arguments (1 <= pairs <= 4096)");
@@ -705,9 +713,11 @@ int gca3d::icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *cons
         if (params->keep_target_normals && params->scales[0].voxel <= 0.0f && !tgt[k]->has_normals)
             return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: the target has no normals (estimate normals first)");
     }
-    // (reuse: a retired plan whose workspace serves this one; the caller has taken it, and it
-    // is destroyed with this one on failure)
-    auto *pl = reuse ? reuse : new gca3d_icp_plan();
+    // (*reuse: a retired plan whose workspace serves this one; a call refused above leaves it, from
+    // here on it is this plan, and destroyed with it on failure)
+    gca3d_icp_plan *pl = reuse ? std::exchange(*reuse, nullptr) : nullptr;
+    if (!pl)
+        pl = new gca3d_icp_plan();
     pl->ctx = ctx;
     pl->P = P;
     pl->src_cap = pl->tgt_cap = pl->src_max = pl->tgt_max = 0;
@@ -919,21 +929,16 @@ int gca3d_color_icp_batched(gca3d_context *ctx, int n_pairs, gca3d_cloud *const 
 {
     if (!results)
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "icp: results needed");
-    // the last one-shot call's workspace (scratch, tables, streams, events) when it holds
-    // enough pairs: making and freeing one took 270 us of a 64k-point alignment's 570
-    gca3d_icp_plan *spare = ctx ? ctx->spare : nullptr, *pl = nullptr;
-    if (spare && spare->pair_cap < n_pairs)
-        spare = nullptr;
-    int st = icp_plan_create_internal(ctx, n_pairs, src, tgt, params, false, nullptr, &pl, nullptr, spare);
-    if (spare && pl != spare && st == GCA3D_ERR_INVALID_VALUE)
-        return st; // refused before the workspace was touched
-    if (spare)
-        ctx->spare = nullptr; // in use, or destroyed with the failed plan
+    // the last one-shot call's workspace (scratch, tables, streams, events) serves this one, grown
+    // where it is too small: making and freeing one took 270 us of a 64k-point alignment's 570
+    gca3d_icp_plan *pl = nullptr;
+    int st = icp_plan_create_internal(ctx, n_pairs, src, tgt, params, false, nullptr, &pl, nullptr,
+                                      ctx ? &ctx->spare : nullptr);
     if (st)
         return st;
     st = gca3d_icp_plan_execute(pl, T_init, results);
     // one is kept per context, up to 256 MB of scratch; gca3d_destroy frees it
-    if (!st && !ctx->spare && pl->arena.bytes() <= (size_t(256) << 20))
+    if (!st && pl->arena.bytes() <= (size_t(256) << 20))
     {
         ctx->spare = pl;
         pl->prologue = nullptr;

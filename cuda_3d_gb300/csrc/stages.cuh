@@ -89,7 +89,7 @@ struct PlanVoxels
 };
 int icp_plan_create_internal(gca3d_context *ctx, int P, gca3d_cloud *const *src, gca3d_cloud *const *tgt,
                              const gca3d_icp_params *params, bool capture, PlanPrologue prologue,
-                             gca3d_icp_plan **out, const PlanVoxels *voxels = nullptr, gca3d_icp_plan *reuse = nullptr);
+                             gca3d_icp_plan **out, const PlanVoxels *voxels = nullptr, gca3d_icp_plan **reuse = nullptr);
 
 // a single-segment batch view of a cloud (no copy; segment offsets from the arena, with
 // by_grid written by the batch's grid build)

@@ -200,6 +200,31 @@ def test_one_shot_calls_share_a_workspace(N, synth):
             assert r["status"] == N.ERR_NO_CORRESPONDENCES
 
 
+def test_one_shot_workspace_grows_with_the_pairs(N, synth):
+    """a call with more pairs than the kept workspace holds leaves one that holds them: calls
+    with three pairs cost the same whether the context's first call had one pair or three (they
+    took 1.5 times as long while the small workspace stayed and theirs was made and freed)"""
+    import time
+
+    pairs = [synth.room_pair(seed=500 + k, n_points=20_000, rot_deg=2.0, trans=0.02) for k in range(3)]
+    prm = N.icp_params([N.scale(0.05, 10, 0.1, 0.1, 0.1)])
+
+    def best(first):
+        c = N.Context(0)
+        S = [c.cloud_from(p.src_xyz, p.src_rgb) for p in pairs]
+        T = [c.cloud_from(p.tgt_xyz, p.tgt_rgb) for p in pairs]
+        N.color_icp_batched(c, S[:first], T[:first], prm)
+        times = []
+        for _ in range(20):
+            t0 = time.perf_counter()
+            N.color_icp_batched(c, S, T, prm) # waits for its results
+            times.append(time.perf_counter() - t0)
+        return min(times)
+
+    three = min(best(3), best(3))
+    assert min(best(1), best(1)) < 1.25 * three
+
+
 @pytest.mark.parametrize("k,n_points", [(1, 600), (1, 6_000), (3, 6_000), (2, 530_000)])
 @pytest.mark.parametrize("mode", ["shared_grid", "two_grids", "kept_normals", "kept_two_grids", "capped"])
 @pytest.mark.parametrize("graph", [False, True])
