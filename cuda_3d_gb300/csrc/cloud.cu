@@ -9,9 +9,24 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <utility>
 
 namespace gca3d
 {
+
+cudaError_t device_malloc(gca3d_context *ctx, void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx && ctx->spare)
+    {
+        cudaGetLastError();
+        gca3d_icp_plan_destroy(std::exchange(ctx->spare, nullptr));
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess)
+        cudaGetLastError(); // the status says it; the next launch's check must not find it
+    return e;
+}
 
 // ---------------------------------------------------------------------------
 // arena
@@ -39,7 +54,7 @@ void *Arena::take(size_t bytes)
     }
     Chunk c;
     c.size = std::max(bytes, size_t(64) << 20);
-    if (cudaMalloc(&c.ptr, c.size) != cudaSuccess)
+    if (device_malloc(owner, &c.ptr, c.size) != cudaSuccess)
     {
         cudaGetLastError();
         failed = true;
@@ -123,9 +138,9 @@ int ensure_attr(gca3d_context *ctx, gca3d_cloud *c, bool normals, bool grad)
 {
     size_t bytes = sizeof(float4) * (size_t)std::max<int64_t>(c->capacity, 1);
     if (normals && !c->nrm)
-        GCA_CUDA(ctx, cudaMalloc(&c->nrm, bytes));
+        GCA_CUDA(ctx, device_malloc(ctx, &c->nrm, bytes));
     if (grad && !c->grd)
-        GCA_CUDA(ctx, cudaMalloc(&c->grd, bytes));
+        GCA_CUDA(ctx, device_malloc(ctx, &c->grd, bytes));
     return GCA3D_OK;
 }
 
@@ -380,6 +395,7 @@ int gca3d_create(int device, void *stream, gca3d_context **out)
     }
     auto *ctx = new gca3d_context();
     ctx->device = device;
+    ctx->arena.owner = ctx;
     if (cudaSetDevice(device) != cudaSuccess)
     {
         delete ctx;
@@ -515,7 +531,7 @@ int gca3d_device_alloc(gca3d_context *ctx, int64_t bytes, void **ptr)
     if (!ctx || !ptr || bytes < 0)
         return fail(ctx, GCA3D_ERR_INVALID_VALUE, "device_alloc: bad arguments");
     *ptr = nullptr;
-    GCA_CUDA(ctx, cudaMalloc(ptr, (size_t)std::max<int64_t>(bytes, 1)));
+    GCA_CUDA(ctx, device_malloc(ctx, ptr, (size_t)std::max<int64_t>(bytes, 1)));
     return GCA3D_OK;
 }
 
@@ -547,8 +563,8 @@ int gca3d_cloud_create(gca3d_context *ctx, int64_t capacity, gca3d_cloud **out)
     c->capacity = capacity;
     c->device = ctx->device;
     size_t bytes = sizeof(float4) * (size_t)std::max<int64_t>(capacity, 1);
-    if (cudaMalloc(&c->pos, bytes) != cudaSuccess || cudaMalloc(&c->col, bytes) != cudaSuccess ||
-        cudaMalloc(&c->d_count, sizeof(int32_t)) != cudaSuccess)
+    if (device_malloc(ctx, &c->pos, bytes) != cudaSuccess || device_malloc(ctx, &c->col, bytes) != cudaSuccess ||
+        device_malloc(ctx, &c->d_count, sizeof(int32_t)) != cudaSuccess)
     {
         cudaGetLastError();
         gca3d_cloud_destroy(c);

@@ -59,6 +59,7 @@ struct Arena
     size_t cur = 0;
     bool frozen = false; // no growth allowed (during capture)
     bool failed = false;
+    gca3d_context *owner = nullptr; // the context whose allocations these are (not swapped)
 
     void *take(size_t bytes);
     void reset()
@@ -191,6 +192,13 @@ int ensure_attr(gca3d_context *ctx, gca3d_cloud *c, bool normals, bool grad);
 int consume_device_error(gca3d_context *ctx, const char *where);
 // the status for an error word already read back (0: GCA3D_OK)
 int device_error_status(gca3d_context *ctx, int word, const char *where);
+// cudaMalloc; where it fails for want of memory, the context's kept workspace is given back
+// and it is tried once more
+cudaError_t device_malloc(gca3d_context *ctx, void **p, size_t bytes);
+template <typename T> cudaError_t device_malloc(gca3d_context *ctx, T **p, size_t bytes)
+{
+    return device_malloc(ctx, reinterpret_cast<void **>(p), bytes);
+}
 
 // ---------------------------------------------------------------------------
 // device helpers

@@ -65,8 +65,8 @@ int gca3d_model_create(gca3d_context *ctx, const gca3d_model_params *p, gca3d_mo
     s->prm = *p;
     const int64_t n = (int64_t)p->width * p->height;
     int st = GCA3D_OK;
-    if (cudaMalloc(&s->d_depth, sizeof(uint16_t) * (size_t)n) != cudaSuccess ||
-        cudaMalloc(&s->d_bgr, 3 * (size_t)n) != cudaSuccess)
+    if (device_malloc(ctx, &s->d_depth, sizeof(uint16_t) * (size_t)n) != cudaSuccess ||
+        device_malloc(ctx, &s->d_bgr, 3 * (size_t)n) != cudaSuccess)
     {
         cudaGetLastError();
         st = fail(ctx, GCA3D_ERR_OUT_OF_MEMORY, "model: frame buffers");

@@ -656,10 +656,10 @@ static int plan_workspace(gca3d_icp_plan *pl, bool capture)
     {
         free_tables(pl);
         if (cudaMallocHost(&pl->h_src, sizeof(SegSrc) * 2 * P) != cudaSuccess ||
-            cudaMalloc(&pl->d_src, sizeof(SegSrc) * P) != cudaSuccess ||
-            cudaMalloc(&pl->d_tgt, sizeof(SegSrc) * P) != cudaSuccess ||
-            cudaMalloc(&pl->d_state, sizeof(PairState) * P) != cudaSuccess ||
-            cudaMalloc(&pl->d_Tinit, sizeof(double) * 16 * P) != cudaSuccess ||
+            device_malloc(ctx, &pl->d_src, sizeof(SegSrc) * P) != cudaSuccess ||
+            device_malloc(ctx, &pl->d_tgt, sizeof(SegSrc) * P) != cudaSuccess ||
+            device_malloc(ctx, &pl->d_state, sizeof(PairState) * P) != cudaSuccess ||
+            device_malloc(ctx, &pl->d_Tinit, sizeof(double) * 16 * P) != cudaSuccess ||
             cudaMallocHost(&pl->h_state, sizeof(PairState) * P) != cudaSuccess ||
             cudaMallocHost(&pl->h_err, sizeof(int)) != cudaSuccess ||
             cudaMallocHost(&pl->h_Tinit, sizeof(double) * 16 * P) != cudaSuccess)
@@ -937,7 +937,8 @@ int gca3d_color_icp_batched(gca3d_context *ctx, int n_pairs, gca3d_cloud *const 
     if (st)
         return st;
     st = gca3d_icp_plan_execute(pl, T_init, results);
-    // one is kept per context, up to 256 MB of scratch; gca3d_destroy frees it
+    // one is kept per context, up to 256 MB of scratch; gca3d_destroy frees it, and so does a
+    // later allocation of the context that finds no memory (device_malloc)
     if (!st && pl->arena.bytes() <= (size_t(256) << 20))
     {
         ctx->spare = pl;

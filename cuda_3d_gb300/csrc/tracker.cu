@@ -128,7 +128,8 @@ int gca3d_tracker_create(gca3d_context *ctx, const gca3d_tracker_params *p, gca3
     const int64_t n = (int64_t)p->width * p->height;
     t->depth_bytes = sizeof(uint16_t) * (size_t)n;
     t->bgr_bytes = 3 * (size_t)n;
-    if (cudaMalloc(&t->d_depth, t->depth_bytes) != cudaSuccess || cudaMalloc(&t->d_bgr, t->bgr_bytes) != cudaSuccess ||
+    if (device_malloc(ctx, &t->d_depth, t->depth_bytes) != cudaSuccess ||
+        device_malloc(ctx, &t->d_bgr, t->bgr_bytes) != cudaSuccess ||
         cudaMallocHost(&t->h_depth, t->depth_bytes) != cudaSuccess ||
         cudaMallocHost(&t->h_bgr, t->bgr_bytes) != cudaSuccess)
     {
@@ -146,16 +147,16 @@ int gca3d_tracker_create(gca3d_context *ctx, const gca3d_tracker_params *p, gca3
             return st;
         }
         const SegSrc seg{t->raw[k]->pos, t->raw[k]->col, nullptr, t->raw[k]->d_count};
-        bool ok = cudaMalloc(&t->d_seg[k], sizeof(SegSrc)) == cudaSuccess &&
+        bool ok = device_malloc(ctx, &t->d_seg[k], sizeof(SegSrc)) == cudaSuccess &&
                   cudaMemcpy(t->d_seg[k], &seg, sizeof(SegSrc), cudaMemcpyHostToDevice) == cudaSuccess;
         for (int s = 0; ok && s < p->icp.n_scales; ++s)
         {
             Batch &b = t->vox[k].src[s];
             b.P = 1;
             b.cap = b.max_seg_cap = n;
-            ok = cudaMalloc(&b.pos, sizeof(float4) * (size_t)n) == cudaSuccess &&
-                 cudaMalloc(&b.col, sizeof(float4) * (size_t)n) == cudaSuccess &&
-                 cudaMalloc(&b.seg_off, sizeof(int32_t) * 2) == cudaSuccess;
+            ok = device_malloc(ctx, &b.pos, sizeof(float4) * (size_t)n) == cudaSuccess &&
+                 device_malloc(ctx, &b.col, sizeof(float4) * (size_t)n) == cudaSuccess &&
+                 device_malloc(ctx, &b.seg_off, sizeof(int32_t) * 2) == cudaSuccess;
         }
         if (!ok)
         {

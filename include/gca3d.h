@@ -307,7 +307,10 @@ int gca3d_abs_residual(gca3d_context *ctx, gca3d_cloud *src, gca3d_cloud *tgt, c
 
 /* the colored ICP of one pair, optionally coarse to fine; T_init may be NULL.
  * The source cloud is not modified.  reference: color_icp::align
- * (src/registration/color_icp.cu:151-234) */
+ * (src/registration/color_icp.cu:151-234)
+ * The context keeps the workspace of its last one-shot registration (this call and the batched
+ * one; plans have their own) for the next one: up to 256 MB of device scratch, which
+ * gca3d_destroy gives back, or an allocation through the context that finds no memory. */
 int gca3d_color_icp(gca3d_context *ctx, gca3d_cloud *src, gca3d_cloud *tgt,
                     const gca3d_icp_params *params, const double T_init[16],
                     gca3d_icp_result *result);

@@ -157,3 +157,32 @@ def test_checked_build_runs_clean_and_matches(ctx, N, golden):
     # a caller's bad index is reported by the checked build as by the regular one
     check_bad_index(cctx, N, golden)
     cctx.close()
+
+
+def free_device_memory():
+    cu = C.CDLL("libcuda.so.1")
+    free, total = C.c_size_t(), C.c_size_t()
+    assert cu.cuMemGetInfo_v2(C.byref(free), C.byref(total)) == 0 # the thread's context: the library's
+    return free.value
+
+
+def test_failed_allocation_gives_the_kept_workspace_back(N):
+    """an allocation that the device cannot hold is refused with a status after the context's
+    kept one-shot workspace (at least one scratch chunk of 64 MB) has been given back; the
+    context goes on, with the same results"""
+    from cuda_3d_gb300 import synth
+
+    pr = synth.room_pair(seed=21, n_points=4_000, rot_deg=2.0, trans=0.02)
+    ctx = N.Context(0)
+    src, tgt = ctx.cloud_from(pr.src_xyz, pr.src_rgb), ctx.cloud_from(pr.tgt_xyz, pr.tgt_rgb)
+    prm = N.icp_params([N.scale(0.1, 10, 0.2, 0.2, 0.2)])
+    first = N.color_icp(ctx, src, tgt, prm)
+    kept = free_device_memory()
+    p = C.c_void_p()
+    assert ctx.L.gca3d_device_alloc(ctx.h, 1 << 42, C.byref(p)) == N.ERR_OUT_OF_MEMORY # 4 TB
+    assert not p.value
+    assert free_device_memory() >= kept + (64 << 20)
+    again = N.color_icp(ctx, src, tgt, prm)
+    assert again["status"] == N.OK
+    np.testing.assert_array_equal(again["T"], first["T"])
+    ctx.close()
