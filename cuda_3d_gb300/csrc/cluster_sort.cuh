@@ -242,6 +242,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
             for (int e = tid; e < cnt; e += kClusterThreads)
             {
                 const uint64_t i = s_words[e] & index_mask;
+                if (!GCA_INDEX_OK(i, n, o.d_err))
+                    continue;
                 const uint64_t k = mk.key(mk.point(0, (int)i), 0, L, origin, o.d_err);
                 s_words[e] = ((((k >> sub) >> low_bits) << ib) | i) & word_mask;
             }
@@ -300,7 +302,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
                 if (it < rounds && e0 + 32 * it < cnt)
                 {
                     const uint32_t d = (uint32_t)(k[it] >> lo) & mask;
-                    s_words[s_base[d] + hist[d] + (uint32_t)(k[it] >> kClusterWordBits)] = k[it] & word_mask;
+                    const uint32_t at = s_base[d] + hist[d] + (uint32_t)(k[it] >> kClusterWordBits);
+                    if (GCA_INDEX_OK(at, cnt, o.d_err))
+                        s_words[at] = k[it] & word_mask;
                 }
             __syncthreads();
 #pragma unroll
@@ -325,7 +329,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
                 {
                     const uint32_t at = s_base[(uint32_t)(k[it] >> lo) & mask] + (uint32_t)(e0 + 32 * it);
                     const uint32_t to = (uint32_t)(((uint64_t)at * chunk_inv) >> 40);
-                    cluster.map_shared_rank(s_words, to)[at - to * (uint32_t)chunk] = k[it];
+                    // (at < n: then to < 16 and the place in that block is below chunk)
+                    if (GCA_INDEX_OK(at, n, o.d_err))
+                        cluster.map_shared_rank(s_words, to)[at - to * (uint32_t)chunk] = k[it];
                 }
             cluster.sync();
         }
@@ -335,6 +341,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
         {
             const int i = (int)(s_words[e] & index_mask);
             o.vals[first + e] = i;
+            if (!GCA_INDEX_OK(i, n, o.d_err))
+                continue;
             s_words[e] = mk.key(mk.point(0, i), 0, L, origin, o.d_err);
         }
     __syncthreads();
@@ -393,8 +401,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster_sort(Maker mk, C
     {
         const bool st = (flags >> it) & 1u;
         const unsigned m = __ballot_sync(full, st);
-        if (st)
-            o.d_starts[run + __popc(m & lt_mask)] = first + e0 + 32 * it;
+        const uint32_t at = run + __popc(m & lt_mask);
+        if (st && GCA_INDEX_OK(at, n, o.d_err))
+            o.d_starts[at] = first + e0 + 32 * it;
         run += __popc(m);
     }
     if (rank == 0 && tid == 0)

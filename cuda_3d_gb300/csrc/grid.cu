@@ -168,7 +168,8 @@ __global__ void __launch_bounds__(kBlock) k_grid_scatter(SortBuffers sb, const i
         }
         if (L.direct)
         {
-            reinterpret_cast<int2 *>(slots)[rk] = make_int2(s, hi);
+            if (GCA_INDEX_OK(rk, 1ll << (L.total_bits - L.zs), err))
+                reinterpret_cast<int2 *>(slots)[rk] = make_int2(s, hi);
             continue;
         }
         uint32_t h = hash_u64(rk) & hmask;

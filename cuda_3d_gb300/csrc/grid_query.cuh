@@ -38,8 +38,9 @@ __device__ __forceinline__ void load_rows(const GridDev &g, const KeyLayout &L, 
         for (int j = 0; j < N; ++j)
         {
             int x, y;
-            const bool ok = row(j, x, y) && x >= 0 && x <= mx && y >= 0 && y <= my;
+            bool ok = row(j, x, y) && x >= 0 && x <= mx && y >= 0 && y <= my;
             const uint32_t i = ((((uint32_t)seg << L.bx | (uint32_t)x) << L.by) | (uint32_t)y) << runs;
+            ok = ok && GCA_INDEX_OK(i + b1, 1ll << (L.total_bits - L.zs), g.err); // b0 <= b1
             v[j] = ok ? run_load(g.slots, i + b0) : make_int2(-1, -1);
             w[j] = ok && b1 != b0 ? run_load(g.slots, i + b1) : make_int2(-1, -1);
         }

@@ -186,3 +186,28 @@ def test_failed_allocation_gives_the_kept_workspace_back(N):
     assert again["status"] == N.OK
     np.testing.assert_array_equal(again["T"], first["T"])
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [16 * 1024 + 1, 13 * 16 * 1024 + 1])
+@pytest.mark.parametrize("extent,voxel", [(2.0, 0.05), (900.0, 0.0005)])
+def test_checked_build_sorts_clean(N, n, extent, voxel):
+    """the checked build's one-launch sort and its launches (on either side of 212,992 points),
+    with keys that share a word with the index and keys that do not: no check fails, same bits
+    as the regular build; the grid's row table and hash through a search"""
+    from cuda_3d_gb300 import build
+
+    rng = np.random.default_rng(n)
+    xyz = (rng.random((n, 3)) * extent).astype(np.float32)
+    out = []
+    for lib in (build.build(), build.build(checked=True)):
+        c = N.Context(0, lib_path=lib)
+        src, dst = c.cloud_from(xyz, xyz / np.float32(extent)), c.cloud(n)
+        c.check(c.L.gca3d_voxel_downsample(c.h, src.h, voxel, dst.h))
+        idx = c.alloc(4 * n)
+        c.check(c.L.gca3d_nn_search(c.h, src.h, src.h, voxel * 2, idx.ptr))
+        c.sync() # a failed check is reported here at the latest
+        out.append((dst.download()["xyz"], idx.read(np.int32, n)))
+        del src, dst, idx
+        c.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
