@@ -8,7 +8,6 @@
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 #include <utility>
 
 namespace gca3d
@@ -306,18 +305,6 @@ __global__ void k_set_count_after_copy(const int32_t *d_nsrc, int32_t *d_ndst, i
 // ---------------------------------------------------------------------------
 // stage helpers used across files
 // ---------------------------------------------------------------------------
-// the one-launch sort's kernels are set up once per device (0.4 ms), by its first context
-static bool device_cluster_sort(int device)
-{
-    constexpr int kDevices = 64;
-    static std::once_flag once[kDevices];
-    static bool ok[kDevices];
-    if (device < 0 || device >= kDevices)
-        return false;
-    std::call_once(once[device], [device] { ok[device] = grid_cluster_enable() && voxel_cluster_enable(); });
-    return ok[device];
-}
-
 int seg_bounds(gca3d_context *ctx, const float4 *pos, const int32_t *seg_off, int P, int64_t max_seg_cap,
                int *ord)
 {
@@ -402,7 +389,7 @@ int gca3d_create(int device, void *stream, gca3d_context **out)
         return GCA3D_ERR_CUDA;
     }
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
-    ctx->cluster_sort = device_cluster_sort(device);
+    ctx->cluster_sort = grid_cluster_enable() && voxel_cluster_enable(); // asked by every context anew
     if (stream)
         ctx->stream = (cudaStream_t)stream;
     else

@@ -1,4 +1,4 @@
-"""Distributed shared memory is accessed only between cluster barriers.
+"""Thread-block clusters: distributed shared memory is accessed only between cluster barriers.
 
 A block of a cluster may be written to or read from by another one only once it has started,
 which a launch attribute does not promise and a cluster barrier does, and only until it
@@ -45,3 +45,13 @@ def test_remote_accesses_lie_between_barriers(name, kernel, body):
     barrier = [m.start() for m in BARRIER.finditer(body)]
     assert barrier and barrier[0] < access[0], f"{name}: {kernel} accesses a block that may not have started"
     assert barrier[-1] > access[-1], f"{name}: {kernel} accesses a block that may have left"
+
+
+def test_every_context_asks_for_the_one_launch_sort_itself():
+    """whether the device runs the cluster's kernels is kept in the context, not in the process:
+    one context that could not set them up must not decide for those after it"""
+    with open(os.path.join(CSRC, "cloud.cu")) as f:
+        text = f.read()
+    body = text[text.index("int gca3d_create("):text.index("int gca3d_destroy(")]
+    assert "grid_cluster_enable() && voxel_cluster_enable()" in body
+    assert "call_once" not in text and "static bool ok" not in text
