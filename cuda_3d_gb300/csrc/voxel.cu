@@ -229,6 +229,12 @@ __global__ void k_voxel_reduce(const SegSrc *src, const int32_t *in_off, SortBuf
             continue;
         float4 p = ps[g], c = cs[g];
         float sx = p.x, sy = p.y, sz = p.z, cr = c.x, cg = c.y, cb = c.z;
+        // one thread adds up a voxel in order, so a large one is a chain of loads that do not
+        // depend on the sums.  300k points in 1 / 29 / 3388 voxels: unrolled by the compiler's
+        // choice 48,270 / 6930 / 217 us, by eight 37,060 / 5400 / 196, by sixteen 36,950 / 5440 /
+        // 205, four points' loads in an array first 42,190 / 8300 / 229; with a few points to a
+        // voxel all alike.
+#pragma unroll 8
         for (int j = s + 1; j < e; ++j)
         {
             g = sv.val(j) - base;

@@ -228,6 +228,26 @@ def test_voxel_sort_sizes_and_key_widths_vs_oracle(ctx, orc, n, extent, voxel):
     np.testing.assert_array_equal(d["rgb"], oc)
 
 
+@pytest.mark.parametrize("per", [1, 2, 7, 8, 9, 10, 16, 17, 25, 1000])
+def test_voxel_sums_of_every_length(ctx, orc, per):
+    """voxels of exactly `per` points (and one fewer, every third), whose points are far apart in the cloud: the
+    sums in index order, bit for bit"""
+    rng = np.random.default_rng(per)
+    cells = np.stack(np.meshgrid(*[np.arange(4)] * 3), -1).reshape(-1, 3)
+    counts = np.where(np.arange(64) % 3 == 0, max(per - 1, 1), per)
+    xyz = np.repeat(cells, counts, 0) * 0.1 + 0.02 + 0.06 * rng.random((counts.sum(), 3))
+    xyz = np.concatenate([[[0.0, 0.0, 0.0]], xyz]).astype(np.float32) # the origin of the voxels
+    xyz[1:] = xyz[1:][rng.permutation(len(xyz) - 1)]
+    rgb = rng.random(xyz.shape).astype(np.float32)
+    src, out = ctx.cloud_from(xyz, rgb), ctx.cloud(len(xyz))
+    ctx.check(ctx.L.gca3d_voxel_downsample(ctx.h, src.h, 0.1, out.h))
+    d = out.download()
+    ox, oc, _, _ = orc.voxel_downsample(xyz, rgb, 0.1)
+    assert len(ox) == 64
+    np.testing.assert_array_equal(d["xyz"], ox)
+    np.testing.assert_array_equal(d["rgb"], oc)
+
+
 def test_voxel_empty_and_invalid(ctx, N):
     c = ctx.cloud(16)
     out = ctx.cloud(16)
