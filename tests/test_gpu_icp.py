@@ -168,6 +168,44 @@ def test_finalize_forms_give_the_same_poses(ctx, N, synth, k, compensated):
             np.testing.assert_array_equal(r["T"], want[j % 3]["T"])
 
 
+@pytest.mark.parametrize("compensated", [True, False])
+@pytest.mark.parametrize("n", [1000, 8192, 65_536, 65_537, 131_073])
+def test_finalize_sums_of_every_length(ctx, N, synth, n, compensated):
+    """the cluster's finalize and the fused one (one block's sums, in the same order) for 1, 8, 64,
+    65 and 129 partials: the same poses bit for bit"""
+    p = synth.room_pair(seed=5, n_points=n, rot_deg=2.0, trans=0.02)
+    S, T = ctx.cloud_from(p.src_xyz, p.src_rgb), ctx.cloud_from(p.tgt_xyz, p.tgt_rgb)
+    r = 12.0 / np.sqrt(n)
+    got = [N.IcpPlan(ctx, [S], [T], N.icp_params([N.scale(0.0, 5, r, r, r)], use_graph=True, compensated=compensated,
+                                                 tuning=N.Tuning(0, 0, 0, 0, fused, 0))).execute()[0] for fused in (0, 1)]
+    assert got[0]["status"] == N.OK and got[0]["iterations"] == got[1]["iterations"]
+    assert got[0]["fitness"] == got[1]["fitness"] and got[0]["inlier_rmse"] == got[1]["inlier_rmse"]
+    np.testing.assert_array_equal(got[0]["T"], got[1]["T"])
+
+
+def test_plain_sums_cost_no_more_than_compensated(ctx, N, synth):
+    """FP32 sums without compensation are the cheaper option of the two: a registration with
+    them takes at most a little longer (it took 1.26 times as long when their partials were read
+    one after the other)"""
+    import time
+
+    p = synth.room_pair(seed=3, n_points=120_000, rot_deg=8.0, trans=0.1)
+    S, T = ctx.cloud_from(p.src_xyz, p.src_rgb), ctx.cloud_from(p.tgt_xyz, p.tgt_rgb)
+
+    def best(compensated):
+        plan = N.IcpPlan(ctx, [S], [T], N.icp_params([N.scale(0.0, 20, 0.14, 0.05, 0.05)], use_graph=True, rot_eps=1e-30,
+                                                     trans_eps=0.0, compensated=compensated))
+        times = []
+        for _ in range(15):
+            t0 = time.perf_counter()
+            r = plan.execute()[0]
+            times.append(time.perf_counter() - t0)
+        assert r["iterations"] == 20
+        return min(times)
+
+    assert best(False) < 1.1 * best(True)
+
+
 def test_one_shot_calls_share_a_workspace(N, synth):
     """one context's one-shot calls reuse one workspace: sizes, pair counts and scales that
     grow and shrink, a refused call and a call without correspondences in between give the
