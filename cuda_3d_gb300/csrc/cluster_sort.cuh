@@ -1,6 +1,7 @@
 // cluster_sort.cuh -- bounds, keys and stable radix sort of one point set in one launch.
 //
-// A set of at most kClusterCap points fits in the shared memory of one cluster of 16 thread
+// A set in a buffer of at most kClusterCap points (the host knows its capacity, not its count)
+// fits in the shared memory of one cluster of 16 thread
 // blocks (16 SMs), so its whole sort runs there: every block holds a sixteenth of the words,
 // a pass ranks them warp by warp (one ballot per digit bit), the blocks exchange their digit
 // counts, and every word goes straight to its place in its destination block through
@@ -32,7 +33,8 @@ namespace gca3d
 constexpr int kClusterBlocks = 16;
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterWarps = kClusterThreads / 32;
-constexpr int kClusterRounds = 13; // words per thread: 26 registers of the 64 there are
+constexpr int kClusterRounds = 13; // words per thread: 26 registers of the 64 there are, which spill a little
+                                   // (ptxas: 124 bytes stored for grids, 144 for voxels)
 constexpr int kClusterWordBits = 54; // of a word; a pass keeps its rank within the warp above them
 constexpr int64_t kClusterCap = (int64_t)kClusterBlocks * kClusterThreads * kClusterRounds; // 212,992
 constexpr int kClusterDigit = 10; // bits of the widest digit: 20 bits of key take two passes, 30 three

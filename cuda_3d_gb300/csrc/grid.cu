@@ -6,9 +6,11 @@
 //
 // GB300 layout: points are physically reordered into cell order (float4 with the z
 // cell in .w), so a query streams contiguous memory.  Instead of a dense
-// nx*ny*nz table the grid keeps a hash of the occupied (segment, x, y) rows ->
-// [start, end) in the sorted arrays; a 27-cell neighbourhood is 9 row lookups and
-// 9 contiguous scans over z.  Cells, rows and the scan order (x, then y, then z,
+// nx*ny*nz table of cells the grid keeps [start, end) in the sorted arrays for the rows
+// (segment, x, y): a direct table of runs of a row's z cells where the key is short enough
+// for a few entries per point, a hash of the occupied rows elsewhere.  A 27-cell
+// neighbourhood is 9 rows, each one or two entries (two where its window of z cells crosses
+// a run) or a hash probe, and 9 contiguous scans over z.  Cells, rows and the scan order (x, then y, then z,
 // then ascending original index) are the reference's, so radius lists come out in
 // the reference's order for the same grid origin.  Memory is O(points), not
 // O(bounding-box volume).

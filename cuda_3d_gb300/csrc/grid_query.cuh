@@ -1,4 +1,4 @@
-// grid_query.cuh -- device-side traversal of the row-hashed uniform grid.
+// grid_query.cuh -- device-side traversal of the uniform grid through its row table.
 #pragma once
 
 #include "internal.cuh"

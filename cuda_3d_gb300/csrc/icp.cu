@@ -8,16 +8,17 @@
 // Three launches per Gauss-Newton iteration cover every pair (two with the fused
 // finalize).  A block owns a chunk of one pair's source points.  k_icp_nn transforms
 // them by the pair's current pose and finds the nearest target point inside max_corr
-// (row-hashed grid, ties to the smaller index); it keeps few registers so many warps
+// (grid with a row table, ties to the smaller index); it keeps few registers so many warps
 // hide the latency of the neighbour walk, and it skips the walk for points whose
 // certificate from an earlier search of the scale still decides the answer
 // (grid_query.cuh).  k_icp_accum builds the geometric and photometric residuals and
 // their 6-vector Jacobians in FP32 and accumulates the 21 + 6 + 1 system terms plus
 // the correspondence count and squared distances.  Accumulation is compensated FP32
 // inside the block (two-sum per thread and per shuffle level) and FP64 across warps
-// and blocks.  k_icp_finalize (one block per pair) -- or, fused, the last accumulate
+// and blocks.  k_icp_finalize (a cluster of eight blocks per pair; k_icp_finalize_many,
+// one block per pair, for several pairs of few points) -- or, fused, the last accumulate
 // block of the pair to finish (atomic ticket, no waiting) -- sums the pair's block
-// partials in FP64 in block order, solves the 6x6 system by FP64 LDL^T, maps the step
+// partials in FP64 in a fixed order, solves the 6x6 system by FP64 LDL^T, maps the step
 // to SE(3) (Euler ZYX as the reference, or the exponential), composes the pose in
 // FP64 and applies the reference's convergence test; a converged pair skips the
 // remaining launches.  The source cloud is never rewritten: the pose is applied on

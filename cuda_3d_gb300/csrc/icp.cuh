@@ -11,15 +11,14 @@ constexpr int kIcpThreads = 256;
 constexpr int kIcpChunk = 1024; // source points per accumulate work item (one partial each)
 // source points per correspondence work item by default: few points make few items of 256
 // (200k points: 800, of which 760 run at once and the rest after them), so for a single pair
-// and up to kNNSmallPoints source points in all they are halved; a large batch has items
-// enough, and pays for each.  ms per execute with 256 and with 128: frame pair -3 %, 250k pair
+// and up to kNNSmallPoints source points in all (by the clouds' capacity, which is what the host
+// knows) they are halved; a large batch has items enough, and pays for each.  ms per execute with 256 and with 128: frame pair -3 %, 250k pair
 // -6 %; 2 pairs of 200k 1.235, 1.173; 4 of them 1.870, 1.797; 16 pairs of 5k to 60k 3.78, 3.51;
 // 64 of those (1.4M points) 7.04, 7.04; 16 pairs of 200k 4.62, 4.72; 64 pairs of 20k to 300k
 // 11.41, 11.94.
 constexpr int kNNChunk = 256, kNNChunkSmall = 128;
 constexpr int64_t kNNSmallPoints = 1 << 20;
-constexpr int kNNChunkMin = 64; // the smallest item size a tuning may choose
-constexpr int kNNChunkMax = 512; // the largest
+constexpr int kNNChunkMax = 512; // the largest item size a tuning may choose
 
 // the launch shape in force (defaults filled in)
 struct IcpShape
@@ -45,7 +44,7 @@ struct PairState
     int status;
     unsigned int ticket;
     int nblocks;    // accumulate work items (kIcpChunk points) of the scale
-    int nblocks_nn; // correspondence work items (kNNChunk points) of the scale
+    int nblocks_nn; // correspondence work items (IcpShape::nn_chunk points) of the scale
     int nsrc;
     int ntgt;
     int scale;

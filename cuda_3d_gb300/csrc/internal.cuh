@@ -317,14 +317,6 @@ __device__ __forceinline__ void block_bounds_commit(float mn[3], float mx[3], in
     }
 }
 
-template <typename T> __device__ __forceinline__ T warp_sum(T v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // the wait limit of the context whose control words ctl points to (see gca3d_context)
 __device__ __forceinline__ uint32_t wait_limit(const int *ctl)
 {
@@ -339,21 +331,9 @@ __device__ __forceinline__ bool index_ok(long long i, long long n, int *err)
     return false;
 }
 
-// bounded spin read of a volatile 64-bit status word until pred holds
-__device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long *p)
-{
-    return *reinterpret_cast<const volatile unsigned long long *>(p);
-}
-
 // ---------------------------------------------------------------------------
 // batched ("segmented") point sets: P clouds back to back
 // ---------------------------------------------------------------------------
-
-// per-segment AABB as ordered ints: [seg][0..2] min, [seg][3..5] max
-struct SegBounds
-{
-    int *ord; // 6 * P
-};
 
 // parameters of one packed 64-bit cell key layout, shared by all segments
 struct KeyLayout

@@ -9,12 +9,14 @@
 // registers; no lists exist.  Moments are taken about the query point, so the
 // FP32 covariance does not cancel at metre-scale coordinates (the reference's
 // E[xx^T] - E[x]E[x]^T does).  The 3x3 eigen-problem is solved in closed form in
-// FP32; points whose two smallest eigenvalues are close (a few dozen per frame)
-// are queued and redone by a second kernel with the covariance rebuilt in FP64
-// and a closed-form FP64 eigen-solve, one warp per point (FP64 issues at a small
-// fraction of the FP32 rate here, so the work is spread over lanes, and a
-// divergent fallback inside the FP32 kernel would stall whole warps).  A third
-// kernel computes the gradients.  The gradient follows the reference's
+// FP32.  Points with more than max_nn neighbours go to a selection pass, a warp per
+// point.  Points whose two smallest eigenvalues are close (a few dozen per frame, tens
+// of thousands in a batch) are queued and redone by a further kernel with the covariance
+// rebuilt in FP64, a warp gathering a point, and a closed-form FP64 eigen-solve, a lane
+// per point (FP64 issues at a small fraction of the FP32 rate here, so the work is spread
+// over lanes, and a divergent fallback inside the FP32 kernel would stall whole warps).
+// Gradients are summed in the same walk, or by a kernel of their own where only they are
+// wanted.  The gradient follows the reference's
 // system: tangent-plane least squares, (knn - 1)^2 n n^T orthogonality term,
 // 1e-6 ridge, LDL^T solve (in the tangent/normal basis, see solve_gradient_system).
 #include "grid_query.cuh"

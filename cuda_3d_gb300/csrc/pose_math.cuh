@@ -214,11 +214,6 @@ __device__ __forceinline__ double sin_or_cos_small(double x, bool cosine)
     const double last = fma(p, -z, 0.5); // the cosine has one coefficient more
     return fma(cosine ? -z : -x * z, cosine ? last : p, cosine ? 1.0 : x);
 }
-__device__ __forceinline__ void sincos_small(double x, double &s, double &c)
-{
-    s = sin_or_cos_small(x, false);
-    c = sin_or_cos_small(x, true);
-}
 
 // the coefficients of the SO(3) / SE(3) exponential, A = sin t / t,
 // B = (1 - cos t) / t^2, C = (t - sin t) / t^3 (k = 0, 1, 2), as series in t2 = t^2 for
@@ -234,12 +229,6 @@ __device__ __forceinline__ double exp_coeff_small(double t2, int k)
     p = fma(p, -t2, pick(1.0 / 120.0, 1.0 / 720.0, 1.0 / 5040.0));
     p = fma(p, -t2, pick(1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0));
     return fma(p, -t2, pick(1.0, 0.5, 1.0 / 6.0));
-}
-__device__ __forceinline__ void exp_coeffs_small(double t2, double &A, double &B, double &C)
-{
-    A = exp_coeff_small(t2, 0);
-    B = exp_coeff_small(t2, 1);
-    C = exp_coeff_small(t2, 2);
 }
 
 // the solve over one warp (same symmetric pivots, factorisation and
@@ -359,9 +348,9 @@ __device__ inline int solve6_warp(const double *S /* 21 upper + 6 rhs */, double
 
 // pose_from_x_device over one warp: every lane returns Ti[lane] for lane < 16
 // (row-major 4x4), the same formulas with one matrix entry per lane.  The three
-// sines and cosines of the Euler map are on separate lanes (sincos_small up to
-// kSmallAngle); the exponential's coefficients are exp_coeffs_small's series up to
-// a rotation of kSmallAngle, else three divisions on separate lanes.
+// sines and cosines of the Euler map are on separate lanes (sin_or_cos_small up to
+// kSmallAngle); the exponential's coefficients too (exp_coeff_small's series up to
+// a rotation of kSmallAngle, else three divisions).
 __device__ inline double pose_from_x_warp(const double x[6], int map)
 {
     const unsigned full = 0xffffffffu;

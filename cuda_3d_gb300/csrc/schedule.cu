@@ -8,7 +8,7 @@
 // them when the scale has no voxel size), build the target grid for normals and
 // colour gradients (cell = their largest radius) and, when the correspondence
 // distance is smaller, a second, tighter target grid for the NN search; estimate
-// target normals and gradients, then launch the two ICP kernels per iteration.  Nothing on the way
+// target normals and gradients, then launch the iterations (search, accumulate, finalize).  Nothing on the way
 // synchronises with the host unless the plain mode is chosen, which, like the
 // reference, checks convergence on the host after every iteration.  A plan runs
 // the schedule once to size its scratch memory and then captures it as one CUDA
@@ -313,8 +313,9 @@ int run_schedule(gca3d_icp_plan *pl, bool capturing)
     cudaStream_t prep_src = serial ? main_stream : pl->prep_src;
     // A small workload's preparation is a chain of short launches that leave the GPU idle, so
     // it gets more branches: every scale's source beside the targets, and the normals (their
-    // grid, the walk, the gradients) beside the search grids.  Three scales, us per execute
-    // without and with them, by the points of all clouds: 0.5 M (one pair of 250k) 974, 871;
+    // grid, the walk, the gradients) beside the search grids.  The line goes by the clouds'
+    // capacity (the host does not know their counts).  Three scales, us per execute without and
+    // with them, for clouds as large as their buffers: 0.5 M (one pair of 250k) 974, 871;
     // 0.8 M 1357, 1241; 1.6 M 1939, 1870; 2.6 M 4835, 4822; 3.2 M 2750, 2746.  From there the
     // launches fill the GPU and the branches get into each other's way: 6.4 M 4680, 4743;
     // 12.8 M 8660, 8950; 64 pairs of 20k to 300k 11,670, 12,000.

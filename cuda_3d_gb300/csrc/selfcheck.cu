@@ -23,22 +23,23 @@ __global__ void k_selfcheck_fp64(int n, double *out)
         const double q = 1.0 / d;
         max_into(&out[0], fabs(rcp_nr(d) - q) / (fabs(q) * kEps));
         const double x = -kSmallAngle + 2.0 * kSmallAngle * f;
-        double s0, c0, s1, c1;
+        double s0, c0;
         sincos(x, &s0, &c0);
-        sincos_small(x, s1, c1);
-        if (s0 != 0.0)
-            max_into(&out[1], fabs(s1 - s0) / (fabs(s0) * kEps));
-        max_into(&out[2], fabs(c1 - c0) / (fabs(c0) * kEps));
+        // as the finalize calls them: neighbouring lanes for neighbouring results
+        const bool cosine = threadIdx.x & 1;
+        const double ref = cosine ? c0 : s0, got = sin_or_cos_small(x, cosine);
+        if (ref != 0.0)
+            max_into(&out[cosine ? 2 : 1], fabs(got - ref) / (fabs(ref) * kEps));
         const double t = 0.05 + (kSmallAngle - 0.05) * f, t2 = t * t;
-        double A, B, C;
-        exp_coeffs_small(t2, A, B, C);
+        const int m = threadIdx.x % 3;
+        const double coeff = exp_coeff_small(t2, m);
         double st, ct;
         sincos(t, &st, &ct);
-        const double A0 = st / t, B0 = (1.0 - ct) / t2, C0 = (t - st) / (t2 * t);
+        const double coeff0 = m == 0 ? st / t : (m == 1 ? (1.0 - ct) / t2 : (t - st) / (t2 * t));
         // the closed forms cancel: 1 - cos t and t - sin t keep about t^2 / 2 and t^2 / 6
         // of their operands, so their rounding error is within eps (4 + 8 / t^2)
         const double bound = kEps * (4.0 + 8.0 / t2);
-        max_into(&out[3], fmax(fabs(A - A0) / A0, fmax(fabs(B - B0) / B0, fabs(C - C0) / C0)) / bound);
+        max_into(&out[3], fabs(coeff - coeff0) / coeff0 / bound);
     }
 }
 

@@ -33,8 +33,8 @@
 // few microseconds, in the point launch's last block.  The call: 904 to 680 us (612 with
 // the shorter finalize and search of the forward pass).  The 391
 // block partials are still added one after the other (12 us of a point launch: an FP64
-// addition takes 64 cycles): at convergence the gradient of the start is the residue of
-// sums that cancel to their last bit, so their order is kept.
+// addition takes 64 cycles); running sums in a fixed order, as the finalize has them, would
+// shorten that chain.
 #include "icp.cuh"
 #include "pose_math.cuh"
 #include "stages.cuh"

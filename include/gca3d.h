@@ -84,8 +84,8 @@ typedef struct {
  * bit-identical for every setting.  gca3d_icp_autotune picks one for a workload. */
 typedef struct {
     int nn_item_points;      /* source points per correspondence work item: 64, 128, 256, 512
-                                (default 128 for one pair and up to 2^20 source points
-                                in all, 256 above) */
+                                (default 128 for one pair and up to 2^20 source points in
+                                all, by the clouds' capacity; 256 above) */
     int nn_blocks_per_sm;    /* correspondence grid = SMs x this (default 10), at most the items */
     int accum_blocks_per_sm; /* accumulate grid = SMs x this (default 6), at most the items */
     int voxel_resort;        /* 1: sort every scale's voxels anew; 0 (default): where the next
