@@ -15,8 +15,9 @@
 // multiply/add); the filter weights use det_expf below instead of expf, so the CPU oracle
 // reproduces every output bit.
 //
-// Measured (GB300, ncu): the adaptive 1280 x 720 frame 63 + 15 us, issue-bound (82 % of
-// the issue slots) on 11 instructions per tap; evaluating both exps per tap took 596 us.
+// Measured (GB300, ncu): the adaptive 1280 x 720 frame 62 + 15 us, issue-bound (82 % of
+// the issue slots while its SMs are busy, 53 M warp instructions); evaluating both exps per
+// tap took 596 us.
 // The fixed 5 x 5 filter at 640 x 480: 11 + 10 us against 47 us for one kernel with a block
 // per row, whose look-back chain over the rows, few warps and eight pixels of registers per
 // thread left the SMs idle.  64 x 4 tiles give that small frame 1200 blocks; the adaptive
